@@ -317,6 +317,23 @@ int lw_carve(const float* xyz, int32_t xyz_stride, const uint32_t* attr, const i
              const int32_t* n_dev, int64_t n_ub, const float* poses, int32_t every, float inv_voxel,
              float max_range, int32_t max_steps, lw_map* map, float* ray_stop, void* stream);
 
+/* Workspace of lw_carve_ws, contents undefined between calls: (ray, occupied voxel) pairs, the distinct voxels met and their
+ * planes. Pairs or voxels beyond the capacities are handled without the workspace (slower, same misses); about 16
+ * pairs and 4 voxels per ray hold an indoor frame. planes is 16-byte aligned. */
+typedef struct lw_carve_buf {
+    int64_t* pairs;   /* [pair_cap] */
+    float* planes;    /* [8 * slot_cap] */
+    int32_t* slots;   /* [slot_cap] */
+    int64_t* counts;  /* [3] */
+    int64_t pair_cap, slot_cap;
+} lw_carve_buf;
+
+/* lw_carve with a workspace: each occupied voxel the rays meet has its plane fitted once instead of once per ray (it
+ * uses the map's bcnt scratch). The same misses, bit for bit. */
+int lw_carve_ws(const float* xyz, int32_t xyz_stride, const uint32_t* attr, const int32_t* frame,
+                const int32_t* n_dev, int64_t n_ub, const float* poses, int32_t every, float inv_voxel,
+                float max_range, int32_t max_steps, lw_map* map, float* ray_stop, lw_carve_buf* cb, void* stream);
+
 /* Classify the map's voxels into the visible set (gpu.py:699-747) and compact it in slot order
  * (gpu.py:1495-1504). Writes count_dev[0]. tiles is [cap/1024 + 1] scratch. */
 int lw_map_build(const lw_map* map, const lw_view* v, int32_t min_count, float* out_xyz, uint32_t* out_attr,

@@ -307,7 +307,8 @@ template <int STRIDE>
 __global__ void k_carve_setup(const float* __restrict__ xyz, const uint32_t* __restrict__ attr,
                               const int32_t* __restrict__ frame, const int* n_dev, int64_t n_ub,
                               const float* __restrict__ poses, int every, float inv_voxel, float max_range, lw_map map,
-                              float* __restrict__ ray_stop) {
+                              float* __restrict__ ray_stop, int64_t* __restrict__ counts) {
+    if (counts && blockIdx.x == 0 && threadIdx.x < 3) counts[threadIdx.x] = 0;
     int64_t n = n_dev ? (int64_t)*n_dev : n_ub;
     if (n > n_ub) n = n_ub;
     const int mask = (int)(map.cap - 1);
@@ -329,6 +330,23 @@ __global__ void k_carve_setup(const float* __restrict__ xyz, const uint32_t* __r
         }
         ray_stop[ray] = stop;
     }
+}
+
+// Whether the ray from o along d pierces the voxel with centroid c and local plane pl (gpu.py:563-591): it crosses the
+// plane near the centroid, or, where the neighbourhood is no surface, passes close to the centroid.
+__device__ __forceinline__ bool pierces(float cx, float cy, float cz, float4 pl, float ox, float oy, float oz, float dx,
+                                        float dy, float dz, float voxel) {
+    const float rx = cx - ox, ry = cy - oy, rz = cz - oz;
+    if (pl.w > 1.5f) {
+        const float dn = dx * pl.x + dy * pl.y + dz * pl.z;
+        if (!(fabsf(dn) > 1.0e-4f)) return false;
+        const float f = (rx * pl.x + ry * pl.y + rz * pl.z) / dn;
+        const float xx = dx * f - rx, xy = dy * f - ry, xz = dz * f - rz;  // plane crossing rel. to centroid
+        return len3(xx, xy, xz) < CARVE_PIERCE_PLANE * voxel;
+    }
+    const float g = rx * dx + ry * dy + rz * dz;
+    const float qx = rx - g * dx, qy = ry - g * dy, qz = rz - g * dz;
+    return len3(qx, qy, qz) < CARVE_PIERCE_POINT * voxel;
 }
 
 // Carving, pass 2 (gpu.py:496-593): one warp per ray. Every lane steps the same DDA (identical float operations,
@@ -423,24 +441,293 @@ __global__ void __launch_bounds__(128) k_carve(const float* __restrict__ xyz, co
             if (s < 0 || __ldg(map.cnt + s) <= 0) continue;
             float cx, cy, cz;
             centroid(map, s, cx, cy, cz);
-            const float rx = cx - ox, ry = cy - oy, rz = cz - oz;
-            bool pierced = false;
             const float4 pl = local_plane_nl(vx, vy, vz, cx, cy, cz, map, mask);
-            if (pl.w > 1.5f) {
-                const float dn = dx * pl.x + dy * pl.y + dz * pl.z;
-                if (fabsf(dn) > 1.0e-4f) {
-                    const float f = (rx * pl.x + ry * pl.y + rz * pl.z) / dn;
-                    const float xx = dx * f - rx, xy = dy * f - ry, xz = dz * f - rz;  // plane crossing rel. to centroid
-                    if (len3(xx, xy, xz) < CARVE_PIERCE_PLANE * voxel) pierced = true;
-                }
-            } else {
-                const float g = rx * dx + ry * dy + rz * dz;
-                const float qx = rx - g * dx, qy = ry - g * dy, qz = rz - g * dz;
-                if (len3(qx, qy, qz) < CARVE_PIERCE_POINT * voxel) pierced = true;
-            }
+            const bool pierced = pierces(cx, cy, cz, pl, ox, oy, oz, dx, dy, dz, voxel);
             if (pierced) atomicAdd(map.miss + s, every);
         }
     }
+}
+
+// Carving with a workspace. The plane of an occupied voxel is a function of the map alone, which carving does not
+// change (only the miss counters grow), but k_carve fits it again for every ray that meets the voxel: a 27-voxel gather
+// and a float64 eigen-decomposition on the one lane that met it, with its warp waiting. Here the walk only notes
+// which occupied voxels each ray meets; each distinct one is fitted once, a thread each, and a last pass tests the
+// noted (ray, voxel) pairs. The same float operations on the same values, so the misses are k_carve's bit for bit.
+//
+// Walk: CW_PARTS lanes per ray, each walking an equal stretch of its length. The times at which a ray crosses the voxel
+// faces of one axis are a running sum that no other axis enters, and the DDA takes the three axes' crossings in
+// order of time, so a lane reaches the walk's state at its stretch by adding up each axis to there and takes from there
+// the very steps the whole walk takes. Bound by the issue of the DDA's steps and the probes' latency: for 10,000 rays of
+// about 100 steps 13.7 us, against 22 us with 8 lanes repeating the whole DDA and 16.6 us with 8 stretches (the
+// adding-up is repeated). A warp gathers its pairs in shared memory (one atomic on the pair count per warp, not
+// per round of probes: 22 us). map.bcnt, zero between calls, marks a voxel as met and then holds its place among
+// the distinct ones plus one; the last CTA of the pair pass zeroes it again.
+// For 10,000 rays the four passes take 22 + 14 + 21 + 7 us where k_carve's two took 22 + 175.
+constexpr int CW_PARTS = 4, CW_DEEP = 8, CW_THREADS = 128;
+constexpr int CW_QUEUE = 512;  // pairs a warp gathers before it writes them out
+
+__device__ __forceinline__ void key_voxel(int64_t key, int& ix, int& iy, int& iz) {
+    ix = (int)(key & KEY_MASK) - (int)KEY_BIAS;
+    iy = (int)((key >> 21) & KEY_MASK) - (int)KEY_BIAS;
+    iz = (int)((key >> 42) & KEY_MASK) - (int)KEY_BIAS;
+}
+
+// Whether a (ray, voxel) pair's voxel is pierced, with its plane fitted here (the lists were full).
+template <int STRIDE>
+__device__ __noinline__ bool carve_alone(const float* __restrict__ xyz, const uint32_t* __restrict__ attr,
+                                         const int32_t* __restrict__ frame, const float* __restrict__ poses, int64_t pair,
+                                         int every, float inv_voxel, float max_range, const lw_map& map) {
+    float ox, oy, oz, wx, wy, wz, dx, dy, dz, L;
+    carve_ray<STRIDE>(xyz, attr, frame, poses, (pair >> 32) * every, max_range, ox, oy, oz, wx, wy, wz, dx, dy, dz, L);
+    const int s = (int)(pair & 0xffffffff);
+    int ix, iy, iz;
+    key_voxel(map.keys[s], ix, iy, iz);
+    float cx, cy, cz;
+    centroid(map, s, cx, cy, cz);
+    const float4 pl = local_plane(ix, iy, iz, cx, cy, cz, map, (int)(map.cap - 1));
+    return pierces(cx, cy, cz, pl, ox, oy, oz, dx, dy, dz, 1.0f / inv_voxel);
+}
+
+template <int STRIDE>
+__global__ void __launch_bounds__(CW_THREADS) k_carve_walk(
+    const float* __restrict__ xyz, const uint32_t* __restrict__ attr, const int32_t* __restrict__ frame,
+    const int* n_dev, int64_t n_ub, const float* __restrict__ poses, int every, float inv_voxel, float max_range,
+    int max_steps, lw_map map, const float* __restrict__ ray_stop, lw_carve_buf cb) {
+    int64_t n = n_dev ? (int64_t)*n_dev : n_ub;
+    if (n > n_ub) n = n_ub;
+    const int mask = (int)(map.cap - 1);
+    const int64_t nrays = (n + every - 1) / every;
+    const int lane = threadIdx.x & 31, part = lane % CW_PARTS;
+    const unsigned below = (1u << lane) - 1u;
+    constexpr int RAYS = 32 / CW_PARTS;  // of a warp
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    __shared__ int64_t queues[CW_THREADS / 32][CW_QUEUE];
+    int64_t* queue = queues[threadIdx.x >> 5];  // the pairs this warp has met and not written out yet
+    int queued = 0;
+    // write the queued pairs out, and list the voxels that no ray had met before
+    auto flush = [&]() {
+        __syncwarp();
+        int64_t p = 0;
+        if (lane == 0 && queued > 0)
+            p = (int64_t)atomicAdd((unsigned long long*)cb.counts, (unsigned long long)queued);
+        p = __shfl_sync(0xffffffffu, p, 0);
+        for (int i0 = 0; i0 < queued; i0 += 32) {
+            bool first = false;
+            int s = 0;
+            if (i0 + lane < queued) {
+                const int64_t pair = queue[i0 + lane];
+                s = (int)(pair & 0xffffffff);
+                if (p + i0 + lane < cb.pair_cap) {
+                    cb.pairs[p + i0 + lane] = pair;
+                    first = *(volatile int*)(map.bcnt + s) == 0 && atomicExch(map.bcnt + s, 1) == 0;
+                } else if (carve_alone<STRIDE>(xyz, attr, frame, poses, pair, every, inv_voxel, max_range, map)) {
+                    atomicAdd(map.miss + s, every);
+                }
+            }
+            const unsigned fresh = __ballot_sync(0xffffffffu, first);
+            if (fresh == 0) continue;
+            int64_t q = 0;
+            if (lane == 0) q = (int64_t)atomicAdd((unsigned long long*)(cb.counts + 1), (unsigned long long)__popc(fresh));
+            q = __shfl_sync(0xffffffffu, q, 0) + __popc(fresh & below);
+            if (first) {
+                if (q < cb.slot_cap)
+                    cb.slots[q] = s;
+                else
+                    *(volatile int*)(map.bcnt + s) = 0;  // no room: the pair pass fits this voxel itself
+            }
+        }
+        __syncwarp();
+        queued = 0;
+    };
+    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * RAYS < nrays; w += nwarps) {
+        const int64_t ray = w * RAYS + lane / CW_PARTS;
+        float stop = ray < nrays ? ray_stop[ray] : 0.0f;
+        bool on = stop > 1.0f;
+        float ox = 0.f, oy = 0.f, oz = 0.f, wx, wy, wz, dx = 0.f, dy = 0.f, dz = 0.f, L;
+        if (on) carve_ray<STRIDE>(xyz, attr, frame, poses, ray * every, max_range, ox, oy, oz, wx, wy, wz, dx, dy, dz, L);
+        const float posx = ox * inv_voxel, posy = oy * inv_voxel, posz = oz * inv_voxel;
+        int ix = ifloor(posx), iy = ifloor(posy), iz = ifloor(posz);
+        int sx = 1, sy = 1, sz = 1;
+        float tmx = 1.0e30f, tmy = 1.0e30f, tmz = 1.0e30f, tdx = 1.0e30f, tdy = 1.0e30f, tdz = 1.0e30f;
+        if (dx > 1.0e-9f) {
+            tmx = ((float)(ix + 1) - posx) / dx;
+            tdx = 1.0f / dx;
+        } else if (dx < -1.0e-9f) {
+            sx = -1;
+            tmx = (posx - (float)ix) / (-dx);
+            tdx = -1.0f / dx;
+        }
+        if (dy > 1.0e-9f) {
+            tmy = ((float)(iy + 1) - posy) / dy;
+            tdy = 1.0f / dy;
+        } else if (dy < -1.0e-9f) {
+            sy = -1;
+            tmy = (posy - (float)iy) / (-dy);
+            tdy = -1.0f / dy;
+        }
+        if (dz > 1.0e-9f) {
+            tmz = ((float)(iz + 1) - posz) / dz;
+            tdz = 1.0f / dz;
+        } else if (dz < -1.0e-9f) {
+            sz = -1;
+            tmz = (posz - (float)iz) / (-dz);
+            tdz = -1.0f / dz;
+        }
+        // this lane's part of the ray: the steps that cross at [begin, stop)
+        const float begin = stop * ((float)part * (1.0f / CW_PARTS));
+        if (part + 1 < CW_PARTS) stop = stop * ((float)(part + 1) * (1.0f / CW_PARTS));
+        int step = 0;
+        while (on && step < max_steps && (tmx < begin || tmy < begin || tmz < begin)) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const bool bx = tmx < begin, by = tmy < begin, bz = tmz < begin;
+                if (bx) {
+                    tmx += tdx;
+                    ix += sx;
+                    ++step;
+                }
+                if (by) {
+                    tmy += tdy;
+                    iy += sy;
+                    ++step;
+                }
+                if (bz) {
+                    tmz += tdz;
+                    iz += sz;
+                    ++step;
+                }
+            }
+        }
+        // one step moves one of the key's fields by one
+        int64_t at = key_ijk(ix, iy, iz);
+        const int64_t kx = sx, ky = (int64_t)sy * (1LL << 21), kz = (int64_t)sz * (1LL << 42);
+        // ... unless a field could run over its 21 bits (2^20 voxels from the origin), where the carry is masked off
+        bool edge = false;
+        {
+            const int64_t reach = min((int64_t)max_steps, (int64_t)fminf(stop, 4.0e6f) + 4);
+#pragma unroll
+            for (int f = 0; f < 3; ++f) {
+                const int64_t v = (at >> (21 * f)) & KEY_MASK;
+                edge |= on && (v < reach || v > KEY_MASK - reach);
+            }
+        }
+        edge = __any_sync(0xffffffffu, edge);
+        while (true) {
+            int64_t key[CW_DEEP], got[CW_DEEP];
+            int h[CW_DEEP];
+#pragma unroll
+            for (int k = 0; k < CW_DEEP; ++k) {
+                // the next crossing; on ties z before y before x, as the comparisons x < y && x < z, y < z have it
+                const float t = fminf(tmx, fminf(tmy, tmz));
+                const bool bz = tmz == t, by = !bz && tmy == t, bx = !bz && !by;
+                on = on && step + k < max_steps && t < stop;
+                const int64_t was = at;
+                at += bx ? kx : (by ? ky : kz);
+                if (edge) {
+                    const int64_t m = KEY_MASK << (bx ? 0 : (by ? 21 : 42));
+                    at = (was & ~m) | (at & m);
+                }
+                tmx = bx ? tmx + tdx : tmx;
+                tmy = by ? tmy + tdy : tmy;
+                tmz = bz ? tmz + tdz : tmz;
+                key[k] = at;
+                h[k] = slot_hash(at) & mask;
+                got[k] = on ? __ldg(map.keys + h[k]) : EMPTY_KEY;
+            }
+            step += CW_DEEP;
+            const bool more = __any_sync(0xffffffffu, on);
+            // which of these voxels are occupied: noted as pairs, and listed when this is the first ray to meet them
+            int s[CW_DEEP];
+            bool some = false;
+#pragma unroll
+            for (int k = 0; k < CW_DEEP; ++k) {
+                s[k] = -1;
+                if (got[k] == key[k]) {
+                    s[k] = h[k];
+                } else if (got[k] != EMPTY_KEY) {
+#pragma unroll 1
+                    for (int p = 1; p < PROBES; ++p) {
+                        const int t = (h[k] + p) & mask;
+                        const int64_t kk = __ldg(map.keys + t);
+                        if (kk == key[k]) {
+                            s[k] = t;
+                            break;
+                        }
+                        if (kk == EMPTY_KEY) break;
+                    }
+                }
+                some |= s[k] >= 0;
+            }
+            if (__any_sync(0xffffffffu, some)) {
+                if (queued > CW_QUEUE - 32 * CW_DEEP) flush();
+                int cnt[CW_DEEP];
+#pragma unroll
+                for (int k = 0; k < CW_DEEP; ++k) cnt[k] = s[k] >= 0 ? __ldg(map.cnt + s[k]) : 0;
+#pragma unroll
+                for (int k = 0; k < CW_DEEP; ++k) {
+                    const unsigned hits = __ballot_sync(0xffffffffu, cnt[k] > 0);
+                    if (cnt[k] > 0) queue[queued + __popc(hits & below)] = (ray << 32) | (int64_t)s[k];
+                    queued += __popc(hits);
+                }
+            }
+            if (!more) break;
+        }
+        flush();
+    }
+}
+
+// The voxels met, a thread each: centroid in planes[2 p], local plane in planes[2 p + 1].
+__global__ void __launch_bounds__(64) k_carve_planes(lw_map map, lw_carve_buf cb) {
+    const int64_t m = min(cb.counts[1], cb.slot_cap);
+    const int mask = (int)(map.cap - 1);
+    float4* __restrict__ out = reinterpret_cast<float4*>(cb.planes);
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < m; p += (int64_t)gridDim.x * blockDim.x) {
+        const int s = cb.slots[p];
+        int ix, iy, iz;
+        key_voxel(map.keys[s], ix, iy, iz);
+        float cx, cy, cz;
+        centroid(map, s, cx, cy, cz);
+        out[2 * p] = make_float4(cx, cy, cz, 0.0f);
+        out[2 * p + 1] = local_plane(ix, iy, iz, cx, cy, cz, map, mask);
+        map.bcnt[s] = (int)p + 1;
+    }
+}
+
+// The pairs, a thread each; the last CTA out puts map.bcnt back to zero for the slots met.
+template <int STRIDE>
+__global__ void __launch_bounds__(256) k_carve_pairs(const float* __restrict__ xyz, const uint32_t* __restrict__ attr,
+                                                     const int32_t* __restrict__ frame, const float* __restrict__ poses,
+                                                     int every, float inv_voxel, float max_range, lw_map map,
+                                                     lw_carve_buf cb) {
+    __shared__ int last;
+    const int64_t np = min(cb.counts[0], cb.pair_cap);
+    const float voxel = 1.0f / inv_voxel;
+    const float4* __restrict__ planes = reinterpret_cast<const float4*>(cb.planes);
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < np; p += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t pair = cb.pairs[p];
+        const int s = (int)(pair & 0xffffffff);
+        const int q = map.bcnt[s];
+        bool hit;
+        if (q > 0) {
+            float ox, oy, oz, wx, wy, wz, dx, dy, dz, L;
+            carve_ray<STRIDE>(xyz, attr, frame, poses, (pair >> 32) * every, max_range, ox, oy, oz, wx, wy, wz, dx, dy,
+                              dz, L);
+            const float4 c = __ldg(planes + 2 * (int64_t)(q - 1));
+            hit = pierces(c.x, c.y, c.z, __ldg(planes + 2 * (int64_t)(q - 1) + 1), ox, oy, oz, dx, dy, dz, voxel);
+        } else {
+            hit = carve_alone<STRIDE>(xyz, attr, frame, poses, pair, every, inv_voxel, max_range, map);
+        }
+        if (hit) atomicAdd(map.miss + s, every);
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+        last = atomicAdd((unsigned long long*)(cb.counts + 2), 1ull) == (unsigned long long)gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    const int64_t m = min(cb.counts[1], cb.slot_cap);
+#pragma unroll 4
+    for (int64_t p = threadIdx.x; p < m; p += blockDim.x) map.bcnt[cb.slots[p]] = 0;
 }
 
 // =====================================================================================================
@@ -761,17 +1048,58 @@ int lw_carve(const float* xyz, int32_t xyz_stride, const uint32_t* attr, const i
     ProfScope prof("carve", s);
     if (xyz_stride == 4) {
         k_carve_setup<4><<<grid1, 64, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range, *map,
-                                              ray_stop);
+                                              ray_stop, nullptr);
         k_carve<4><<<grid, 128, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range, max_steps,
                                         *map, ray_stop);
     } else {
         k_carve_setup<3><<<grid1, 64, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range, *map,
-                                              ray_stop);
+                                              ray_stop, nullptr);
         k_carve<3><<<grid, 128, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range, max_steps,
                                         *map, ray_stop);
     }
     LW_LAUNCHED("lw_carve");
     count_launches(2);
+    return LW_OK;
+}
+
+int lw_carve_ws(const float* xyz, int32_t xyz_stride, const uint32_t* attr, const int32_t* frame, const int32_t* n_dev,
+                int64_t n_ub, const float* poses, int32_t every, float inv_voxel, float max_range, int32_t max_steps,
+                lw_map* map, float* ray_stop, lw_carve_buf* cb, void* stream) {
+    int r = check_map(map, "lw_carve_ws");
+    if (r != LW_OK) return r;
+    if (!xyz || !attr || !frame || !poses || !ray_stop || (xyz_stride != 3 && xyz_stride != 4))
+        return set_error(LW_EINVAL, "lw_carve_ws: bad arguments");
+    if (!cb || !cb->pairs || !cb->planes || !cb->slots || !cb->counts || cb->pair_cap < 0 || cb->slot_cap < 0 ||
+        cb->slot_cap >= 0x7FFFFFFF || ((uintptr_t)cb->planes & 15) != 0)
+        return set_error(LW_EINVAL, "lw_carve_ws: incomplete workspace");
+    if (n_ub > 0x7FFFFFFF) return set_error(LW_ECAPACITY, "lw_carve_ws: more than 2^31 - 1 points");
+    if (n_ub <= 0) return LW_OK;
+    if (every < 1) every = 1;
+    cudaStream_t s = (cudaStream_t)stream;
+    const int64_t rays = (n_ub + every - 1) / every;
+    const int sms = device_sms();
+    const int grid1 = blocks_for(rays, 64, 16 * sms);                 // a thread per ray
+    const int grid2 = blocks_for(rays * CW_PARTS, CW_THREADS, 16 * sms);
+    const int grid3 = blocks_for(rays, 64, 8 * sms);                  // a thread per distinct voxel met
+    const int grid4 = blocks_for(4 * rays, 256, 4 * sms);             // a thread per pair
+    ProfScope prof("carve", s);
+    if (xyz_stride == 4) {
+        k_carve_setup<4><<<grid1, 64, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range, *map,
+                                              ray_stop, cb->counts);
+        k_carve_walk<4><<<grid2, CW_THREADS, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range,
+                                              max_steps, *map, ray_stop, *cb);
+        k_carve_planes<<<grid3, 64, 0, s>>>(*map, *cb);
+        k_carve_pairs<4><<<grid4, 256, 0, s>>>(xyz, attr, frame, poses, every, inv_voxel, max_range, *map, *cb);
+    } else {
+        k_carve_setup<3><<<grid1, 64, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range, *map,
+                                              ray_stop, cb->counts);
+        k_carve_walk<3><<<grid2, CW_THREADS, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range,
+                                              max_steps, *map, ray_stop, *cb);
+        k_carve_planes<<<grid3, 64, 0, s>>>(*map, *cb);
+        k_carve_pairs<3><<<grid4, 256, 0, s>>>(xyz, attr, frame, poses, every, inv_voxel, max_range, *map, *cb);
+    }
+    LW_LAUNCHED("lw_carve_ws");
+    count_launches(4);
     return LW_OK;
 }
 

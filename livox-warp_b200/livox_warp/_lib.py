@@ -86,6 +86,11 @@ class Map(C.Structure):
                 ("lead", P), ("stats", P), ("cap", i64)]
 
 
+class CarveBuf(C.Structure):
+    PTRS = ("pairs", "planes", "slots", "counts")
+    _fields_ = [(n, P) for n in PTRS] + [("pair_cap", i64), ("slot_cap", i64)]
+
+
 class ClusterBuf(C.Structure):
     PTRS = ("keys", "acc", "first", "vidx", "slot_of_pt", "tiles", "node_slot", "v_xyz", "v_w", "edge_off", "edges",
             "label", "st_sum", "st_lo", "st_hi", "dense", "out_cnt", "out_cen", "out_lo", "out_hi", "m", "n_clusters",
@@ -192,6 +197,7 @@ _SIGS = {
                                      C.POINTER(FrameBuf), C.POINTER(RegMap), C.POINTER(GnScratch), P, P, P]),
     "lw_map_insert": (i32, [P, i32, P, P, P, P, i64, P, C.POINTER(View), f32, C.POINTER(Map), P, P]),
     "lw_carve": (i32, [P, i32, P, P, P, i64, P, i32, f32, f32, i32, C.POINTER(Map), P, P]),
+    "lw_carve_ws": (i32, [P, i32, P, P, P, i64, P, i32, f32, f32, i32, C.POINTER(Map), P, C.POINTER(CarveBuf), P]),
     "lw_map_build": (i32, [C.POINTER(Map), C.POINTER(View), i32, P, P, P, P, P, P, P]),
     "lw_map_clear": (i32, [C.POINTER(Map), P]),
     "lw_live_build": (i32, [P, P, P, P, i64, i64, C.POINTER(PoseTable), C.POINTER(View), C.POINTER(Map), P, P, P, P,

@@ -200,6 +200,8 @@ class Pipeline:
         self.cl_vel = torch.zeros((MAX_CLUSTERS, 3), dtype=torch.float32, device=d)
         self.cl_tid = torch.full((MAX_CLUSTERS,), -1, dtype=torch.int32, device=d)
         self._slot = torch.zeros(n, dtype=torch.int32, device=d)  # per-point scratch of the insert passes
+        self._carve_rays, self._carve_t, self._carve_buf = 0, [], None  # lw_carve_ws's workspace
+        self._carve_ws(1 << 15)  # what a frame takes, made here so that no frame waits for an allocation
         self._tiles = torch.zeros(max(m, self.cap) // 1024 + 2, dtype=torch.int32, device=d)
         self.total = torch.zeros(1, dtype=torch.int32, device=d)
 
@@ -358,9 +360,24 @@ class Pipeline:
             return
         self.flush_poses()
         sx = _as_xyz(sx, self.device)
-        _lib.call("lw_carve", _lib.ptr(sx), row_stride(sx), _lib.ptr(sa), _lib.ptr(sf), _lib.ptr(n_dev), n,
-                  _lib.ptr(self.poses), max(1, int(every)), 1.0 / max(voxel, 1e-4), float(max_range), int(max_steps),
-                  C_ref(self.map_struct), _lib.ptr(self._scratch(n)), _lib.stream_ptr())
+        every = max(1, int(every))
+        rays = (n + every - 1) // every
+        _lib.call("lw_carve_ws", _lib.ptr(sx), row_stride(sx), _lib.ptr(sa), _lib.ptr(sf), _lib.ptr(n_dev), n,
+                  _lib.ptr(self.poses), every, 1.0 / max(voxel, 1e-4), float(max_range), int(max_steps),
+                  C_ref(self.map_struct), _lib.ptr(self._scratch(n)), C_ref(self._carve_ws(rays)), _lib.stream_ptr())
+
+    def _carve_ws(self, rays: int) -> _lib.CarveBuf:
+        """lw_carve_ws's workspace for at least `rays` rays. It grows by doubling, and the smaller ones are kept: a
+        stream other than the one they were made on may still be using them."""
+        if rays > self._carve_rays:
+            r = 1 << (rays - 1).bit_length()
+            pairs, slots, d = 16 * r, min(4 * r, self.map_cap), self.device
+            t = (torch.empty(pairs, dtype=torch.int64, device=d), torch.empty((slots, 8), dtype=torch.float32, device=d),
+                 torch.empty(slots, dtype=torch.int32, device=d), torch.zeros(3, dtype=torch.int64, device=d))
+            self._carve_t.append(t)
+            self._carve_buf = _lib.CarveBuf(*(_lib.ptr(x) for x in t), pairs, slots)
+            self._carve_rays = r
+        return self._carve_buf
 
     def ingest(self, xyz, attr, t, n: int, view: View, map_on: bool, voxel: float):
         """Stage, ring and map in one call, without odometry (gpu.py:1454-1462)."""
