@@ -360,20 +360,21 @@ int lw_frame_ids(const float* t, int64_t n, float inv_dt, int32_t* out, void* st
 int lw_stage_batch(const float* xyz_host, const uint32_t* attr_host, const float* t_host, int64_t n, float* xyz_dev,
                    uint32_t* attr_dev, float* t_dev, float inv_dt, int32_t* frame_dev, void* stream);
 
-/* Buffers of the neighbourhood pass: an open-addressed voxel table of cap (a power of two) slots and the dense
- * per-voxel arrays (at most one voxel per point). */
+/* Buffers of the neighbourhood pass, contents undefined between calls: an open-addressed table of cap (a power of two)
+ * slots for the bricks of 4 x 4 x 4 voxels that the points lie in (a call clears and uses the first power of two of
+ * at least 2 n slots) and dense per-voxel arrays (at most one voxel per point), numbered brick by brick. */
 typedef struct lw_nbr_buf {
-    int64_t* keys;       /* [cap] voxel keys, -1 empty (cleared by each call) */
-    int64_t* acc;        /* [cap*4] fixed-point sums of x, y, z (LW_FIX_W units) and the point count */
-    int32_t* vidx;       /* [cap] dense index of each occupied slot */
-    int32_t* v_slot;     /* [cap] slot of each dense voxel */
-    int32_t* slot_of_pt; /* [pt_cap] voxel slot of each point, -1 when the table was full */
-    float* v_xyz;        /* [cap*3] voxel centroids, in slot order */
-    int32_t* v_w;        /* [cap] points per voxel */
-    float* v_cnt;        /* [cap] point-weighted neighbour count */
+    int64_t* keys;       /* [cap] brick keys, -1 empty */
+    int64_t* acc;        /* [cap*4] fixed-point sums of x, y, z (LW_FIX_W units) and the point count, then the means */
+    int32_t* vidx;       /* [cap] upper half of each brick's mask of occupied voxels */
+    int32_t* v_slot;     /* [cap] lower half */
+    int32_t* slot_of_pt; /* [pt_cap] voxel of each point, -1 when the table was full */
+    float* v_xyz;        /* [cap*3] not used */
+    int32_t* v_w;        /* [cap] number of each brick's first voxel */
+    float* v_cnt;        /* [cap] point-weighted neighbour count (a voxel's brick before that) */
     float* v_nrm;        /* [cap*3] unit normals */
     float* v_curv;       /* [cap] curvature */
-    int32_t* tiles;      /* [cap/1024 + 1] scan scratch */
+    int32_t* tiles;      /* [cap/1024 + 1] not used */
     int32_t* m;          /* [1] voxels */
     int64_t cap, pt_cap;
 } lw_nbr_buf;

@@ -1,0 +1,153 @@
+// Voxels gathered into bricks of 4 x 4 x 4: a hash of bricks, each with a 64-bit mask of its occupied voxels, and the
+// voxels numbered brick by brick, so that voxel `bit` of a brick is number base + popcount(mask below bit).
+//
+// Why: finding a voxel's neighbours in a hash of voxels takes one probe per offset of the neighbourhood -- 343 for a
+// reach of 3 voxels, 729 for 4, nearly all of them misses. A neighbourhood of up to 4 voxels' reach lies in 27 bricks:
+// 27 probes, shared by all voxels of a brick, then a walk over the set bits of the masks, which meets only occupied
+// voxels; and those lie next to each other in memory.
+//
+// Coordinates are the 21-bit fields of the voxel key (gpu.py:231-239), so neighbourhoods wrap where keys do.
+#pragma once
+#include "lw_common.cuh"
+
+namespace lw {
+
+constexpr int64_t BRICK_MASK = (1LL << 19) - 1;  // a 21-bit field without its two low bits
+
+struct BrickHash {
+    const int64_t* keys;
+    const uint32_t* lo;  // the mask's halves
+    const uint32_t* hi;
+    const int32_t* base;
+    int mask;
+};
+
+__device__ __forceinline__ int64_t brick_key(int64_t bx, int64_t by, int64_t bz) {
+    return (bx & BRICK_MASK) | ((by & BRICK_MASK) << 19) | ((bz & BRICK_MASK) << 38);
+}
+
+// The brick of voxel (ix, iy, iz) and the voxel's bit in it: x + 4 y + 16 z of the low coordinate bits.
+__device__ __forceinline__ int64_t brick_of(int ix, int iy, int iz, int& bit) {
+    const int64_t x = ((int64_t)ix + KEY_BIAS) & KEY_MASK, y = ((int64_t)iy + KEY_BIAS) & KEY_MASK,
+                  z = ((int64_t)iz + KEY_BIAS) & KEY_MASK;
+    bit = (int)(x & 3) | ((int)(y & 3) << 2) | ((int)(z & 3) << 4);
+    return brick_key(x >> 2, y >> 2, z >> 2);
+}
+
+// Slots a hash of at most n bricks takes: the power of two from 2 n up, at least 1024 and at most cap.
+inline int64_t brick_slots(int64_t n, int64_t cap) {
+    int64_t h = 1024;
+    while (h < 2 * n) h *= 2;
+    return h < cap ? h : cap;
+}
+
+__device__ __forceinline__ int popc64(uint64_t v) { return __popcll(v); }
+
+// The n-th set bit of a mask, from 0.
+__device__ __forceinline__ int nth_bit(uint64_t mask, int n) {
+    uint32_t h = (uint32_t)mask;
+    int bit = 0;
+    if (n >= __popc(h)) {
+        n -= __popc(h);
+        h = (uint32_t)(mask >> 32);
+        bit = 32;
+    }
+    for (int k = 0; k < n; ++k) h &= h - 1;
+    return bit + __ffs(h) - 1;
+}
+
+// The low coordinates (0..3) of the brick `o` away whose distance from l is at most R, as a 4-bit pattern (R <= 4).
+__device__ __forceinline__ unsigned brick_span(int l, int o, int R) {
+    const int lo = max(0, l - R - 4 * o), hi = min(3, l + R - 4 * o);
+    return hi < lo ? 0u : (0xFu >> (3 - hi)) & (0xFu << lo);
+}
+
+// The voxels of the brick (ox, oy, oz) away within R of bit `bit` along every axis.
+__device__ __forceinline__ uint64_t brick_window(int bit, int ox, int oy, int oz, int R) {
+    const uint64_t x = brick_span(bit & 3, ox, R) * 0x1111111111111111ull;
+    const unsigned py = brick_span((bit >> 2) & 3, oy, R), pz = brick_span(bit >> 4, oz, R);
+    const uint64_t row = ((py & 1u) * 0xFu) | ((py >> 1 & 1u) * 0xF0u) | ((py >> 2 & 1u) * 0xF00u) |
+                         ((py >> 3 & 1u) * 0xF000u);
+    const uint64_t y = row * 0x0001000100010001ull;
+    const uint64_t z = ((pz & 1u) * 0xFFFFull) | ((pz >> 1 & 1u) * 0xFFFF0000ull) |
+                       ((uint64_t)(pz >> 2 & 1u) * 0xFFFFull << 32) | ((uint64_t)(pz >> 3 & 1u) * 0xFFFFull << 48);
+    return x & y & z;
+}
+
+// The 27 bricks around each of up to BRICK_ROWS bricks, for one warp's voxels.
+constexpr int BRICK_ROWS = 4;
+struct BrickRows {
+    uint64_t mask[BRICK_ROWS][27];
+    int32_t base[BRICK_ROWS][27];
+};
+
+// For the voxels of a warp, a thread each in the order of their numbers (slot: the voxel's brick, -1 for none; every
+// lane calls), run(row) with the neighbouring bricks of the lane's own brick in rows.mask[row], rows.base[row].
+// Voxels of a brick are neighbours in number, so 32 lanes hold a few bricks; their 27-brick neighbourhoods are
+// looked up by all lanes together, BRICK_ROWS at a time.
+template <class Run>
+__device__ __forceinline__ void brick_rows(const BrickHash& bh, int slot, BrickRows& rows, const Run& run) {
+    const int lane = threadIdx.x & 31;
+    const int prev = __shfl_up_sync(0xffffffffu, slot, 1);
+    const unsigned leaders = __ballot_sync(0xffffffffu, slot >= 0 && (lane == 0 || slot != prev));
+    const int mine = __popc(leaders & (0xffffffffu >> (31 - lane))) - 1;  // my brick's place among the leaders
+    const int nrows = __popc(leaders);
+    unsigned left = leaders;
+    for (int r0 = 0; r0 < nrows; r0 += BRICK_ROWS) {
+        const int here = min(BRICK_ROWS, nrows - r0);
+        int64_t lead_key[BRICK_ROWS];
+#pragma unroll
+        for (int r = 0; r < BRICK_ROWS; ++r) {
+            const int src = left ? __ffs(left) - 1 : 0;
+            left &= left - 1;
+            const int s = __shfl_sync(0xffffffffu, slot, src);
+            lead_key[r] = r < here ? bh.keys[s] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < (BRICK_ROWS * 27 + 31) / 32; ++u) {
+            const int t = lane + 32 * u, r = t / 27, c = t - 27 * r;
+            if (r < here) {
+                int64_t k = lead_key[0];
+#pragma unroll
+                for (int q = 1; q < BRICK_ROWS; ++q) k = r == q ? lead_key[q] : k;
+                const int64_t nk = brick_key((k & BRICK_MASK) + (c % 3 - 1), (k >> 19 & BRICK_MASK) + (c / 3 % 3 - 1),
+                                             (k >> 38 & BRICK_MASK) + (c / 9 - 1));
+                const int s = find_slot(nk, bh.keys, bh.mask);
+                rows.mask[r][c] = s < 0 ? 0ull : (uint64_t)bh.lo[s] | ((uint64_t)bh.hi[s] << 32);
+                rows.base[r][c] = s < 0 ? 0 : bh.base[s];
+            }
+        }
+        __syncwarp();
+        if (slot >= 0 && mine >= r0 && mine < r0 + here) run(mine - r0);
+        __syncwarp();
+    }
+}
+
+// Number the voxels brick by brick: a CTA per 1024 brick slots takes a run of numbers for its bricks (which run depends
+// on timing, so no result may depend on a voxel's number), writes each brick's base, each voxel's brick slot
+// (voxel_slot [vcap]) and whatever init(v) sets up for voxel v < vcap.
+template <class Init>
+__device__ __forceinline__ void brick_number(const int64_t* __restrict__ keys, const uint32_t* __restrict__ lo,
+                                             const uint32_t* __restrict__ hi, int32_t* __restrict__ base, int64_t slots,
+                                             int* counter, int32_t* __restrict__ voxel_slot, int64_t vcap,
+                                             const Init& init) {
+    __shared__ int sm[33];
+    __shared__ int first;
+    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool used = s < slots && keys[s] != EMPTY_KEY;
+    const int c = used ? __popc(lo[s]) + __popc(hi[s]) : 0;
+    int tot;
+    const int r = block_excl(c, sm, &tot);
+    if (tot == 0) return;
+    if (threadIdx.x == 0) first = atomicAdd(counter, tot);
+    __syncthreads();
+    if (used) {
+        base[s] = first + r;
+        for (int k = 0; k < c; ++k)
+            if (first + r + k < vcap) voxel_slot[first + r + k] = (int)s;
+    }
+    for (int k = threadIdx.x; k < tot; k += blockDim.x)
+        if (first + k < vcap) init((int64_t)first + k);
+}
+
+}  // namespace lw

@@ -7,23 +7,28 @@
 // Determinism: the reference adds float coordinates into its voxels with float atomics and sums each voxel's
 // neighbours in the order a hash-grid query returns them, so its answers depend on thread timing. Here the voxel
 // sums are int64 fixed point (exact), the neighbours of a voxel are the voxels whose centroid lies within the radius
-// -- found by probing the 7 x 7 x 7 voxel offsets that can hold one (a centroid lies inside its voxel, so with
-// voxels radius / 3 wide no farther voxel qualifies) -- and their weighted offsets and outer products are summed as
-// int64 fixed point too; the covariance and its eigen-decomposition are float64. Every point's count, normal and
-// curvature is then independent of thread order and of where keys land in the table.
+// -- all within 3 voxels along each axis (a centroid lies inside its voxel, and voxels are radius / 3 wide), found
+// through the masks of the 27 bricks around it (lw_bricks.cuh) -- and their weighted offsets and outer products are
+// summed as int64 fixed point too; the covariance and its eigen-decomposition are float64. Every point's count,
+// normal and curvature is then independent of thread order and of where keys land in the table.
+//
+// Layout of the caller's buffers: keys, v_slot / vidx and v_w hold the bricks' keys, masks' halves and bases in the first
+// brick_slots(n) slots (so a call clears what its points can fill, not the whole table); acc holds voxel v's sums and
+// then, in its place, the record (x, y, z, weight); v_cnt holds a voxel's brick slot until its count replaces it.
 #include "lw_common.cuh"
+#include "lw_bricks.cuh"
 #include "lw_linalg.cuh"
 
 namespace lw {
 
 constexpr double NB_FIX_D = 1048576.0;         // units per metre of a neighbour offset (2^20)
 constexpr double NB_FIX_DD = 1099511627776.0;  // units per m^2 of an offset product (2^40)
-constexpr int NB_REACH = 3;                    // voxel offsets probed per axis: radius / (radius / 3)
-constexpr int NB_TILE = 1024;
+constexpr int NB_REACH = 3;                    // voxels per axis: radius / (radius / 3)
 
 struct NbArgs {
     float inv_h, r2;
     int mask, want_normals;
+    int64_t vcap;  // voxel records the buffers hold
     double sensor[3];
 };
 
@@ -34,149 +39,152 @@ __device__ __forceinline__ void nb_ld(const float* __restrict__ xyz, int64_t i, 
     z = xyz[STRIDE * i + 2];
 }
 
-// Each point claims its voxel (key of floor(w * inv_h), gpu.py:243) and adds its coordinates in fixed point.
+__global__ void k_nb_clear(lw_nbr_buf nb, int64_t slots) {
+    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < slots; s += (int64_t)gridDim.x * blockDim.x) {
+        nb.keys[s] = EMPTY_KEY;
+        nb.v_slot[s] = 0;
+        nb.vidx[s] = 0;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *nb.m = 0;
+}
+
+template <int STRIDE>
+__device__ __forceinline__ int64_t nb_brick(const float* __restrict__ xyz, int64_t i, const NbArgs& a, float& x, float& y,
+                                            float& z, int& bit) {
+    nb_ld<STRIDE>(xyz, i, x, y, z);
+    return brick_of(ifloor(x * a.inv_h), ifloor(y * a.inv_h), ifloor(z * a.inv_h), bit);  // floor(w * inv_h), gpu.py:243
+}
+
+// Each point claims its voxel's brick and marks the voxel.
 template <int STRIDE>
 __global__ void k_nb_insert(const float* __restrict__ xyz, const int* n_dev, int64_t n_ub, NbArgs a, lw_nbr_buf nb) {
     int64_t n = n_dev ? (int64_t)*n_dev : n_ub;
     if (n > n_ub) n = n_ub;
-    const float FW = (float)LW_FIX_W;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         float x, y, z;
-        nb_ld<STRIDE>(xyz, i, x, y, z);
-        const int64_t key = key_ijk(ifloor(x * a.inv_h), ifloor(y * a.inv_h), ifloor(z * a.inv_h));
+        int bit;
+        const int64_t key = nb_brick<STRIDE>(xyz, i, a, x, y, z, bit);
         bool claimed;
         const int s = claim_slot(key, nb.keys, a.mask, &claimed);
         if (s >= 0) {
-            atomic_add_i64(nb.acc + 4 * (int64_t)s + 0, to_fix(x, FW));
-            atomic_add_i64(nb.acc + 4 * (int64_t)s + 1, to_fix(y, FW));
-            atomic_add_i64(nb.acc + 4 * (int64_t)s + 2, to_fix(z, FW));
-            atomic_add_i64(nb.acc + 4 * (int64_t)s + 3, 1);
+            unsigned* half = reinterpret_cast<unsigned*>((bit & 32) ? nb.vidx : nb.v_slot) + s;
+            const unsigned b = 1u << (bit & 31);
+            if ((*(volatile unsigned*)half & b) == 0) atomicOr(half, b);
         }
         nb.slot_of_pt[i] = s;
     }
 }
 
-// Occupied slots per tile, then (one CTA) their exclusive scan; the voxels are numbered in slot order.
-__global__ void k_nb_count(lw_nbr_buf nb) {
-    const int64_t s = (int64_t)blockIdx.x * NB_TILE + threadIdx.x;
-    const int f = (s < nb.cap && nb.keys[s] != EMPTY_KEY) ? 1 : 0;
-    const int c = __syncthreads_count(f);
-    if (threadIdx.x == 0) nb.tiles[blockIdx.x] = c;
+__device__ __forceinline__ BrickHash nb_hash(const lw_nbr_buf& nb, int mask) {
+    return {nb.keys, reinterpret_cast<const uint32_t*>(nb.v_slot), reinterpret_cast<const uint32_t*>(nb.vidx), nb.v_w,
+            mask};
 }
 
-__global__ void k_nb_scan(lw_nbr_buf nb, int nt) {
-    __shared__ int sm[33];
-    __shared__ int carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int base = 0; base < nt; base += blockDim.x) {
-        const int j = base + threadIdx.x;
-        const int v = j < nt ? nb.tiles[j] : 0;
-        // exclusive prefix of the counts across the CTA: warp scan + warp totals
-        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-        int inc = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += u;
+__global__ void __launch_bounds__(1024) k_nb_number(lw_nbr_buf nb, int64_t slots, int64_t vcap) {
+    brick_number(nb.keys, reinterpret_cast<const uint32_t*>(nb.v_slot), reinterpret_cast<const uint32_t*>(nb.vidx),
+                 nb.v_w, slots, nb.m, reinterpret_cast<int32_t*>(nb.v_cnt), vcap, [&](int64_t v) {
+                     longlong2* a = reinterpret_cast<longlong2*>(nb.acc + 4 * v);
+                     a[0] = a[1] = make_longlong2(0, 0);
+                 });
+}
+
+// Each point adds its coordinates to its voxel in fixed point and keeps the voxel's number.
+template <int STRIDE>
+__global__ void k_nb_sum(const float* __restrict__ xyz, const int* n_dev, int64_t n_ub, NbArgs a, lw_nbr_buf nb) {
+    int64_t n = n_dev ? (int64_t)*n_dev : n_ub;
+    if (n > n_ub) n = n_ub;
+    const float FW = (float)LW_FIX_W;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int s = nb.slot_of_pt[i];
+        if (s < 0) continue;
+        float x, y, z;
+        int bit;
+        nb_brick<STRIDE>(xyz, i, a, x, y, z, bit);
+        const uint64_t m = (uint64_t)(uint32_t)nb.v_slot[s] | ((uint64_t)(uint32_t)nb.vidx[s] << 32);
+        const int64_t v = (int64_t)nb.v_w[s] + popc64(m & ((1ull << bit) - 1));
+        if (v < a.vcap) {
+            atomic_add_i64(nb.acc + 4 * v + 0, to_fix(x, FW));
+            atomic_add_i64(nb.acc + 4 * v + 1, to_fix(y, FW));
+            atomic_add_i64(nb.acc + 4 * v + 2, to_fix(z, FW));
+            atomic_add_i64(nb.acc + 4 * v + 3, 1);
         }
-        if (lane == 31) sm[w] = inc;
-        __syncthreads();
-        if (w == 0) {
-            const int nw = blockDim.x >> 5;
-            const int x = lane < nw ? sm[lane] : 0;
-            int xi = x;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, xi, o);
-                if (lane >= o) xi += u;
-            }
-            if (lane < nw) sm[lane] = xi - x;
-            if (lane == 31) sm[32] = xi;
-        }
-        __syncthreads();
-        if (j < nt) nb.tiles[j] = carry + sm[w] + inc - v;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += sm[32];
-        __syncthreads();
+        nb.slot_of_pt[i] = v < a.vcap ? (int)v : -1;
     }
-    if (threadIdx.x == 0) *nb.m = carry;
 }
 
-__global__ void k_nb_scatter(lw_nbr_buf nb) {
-    __shared__ int sm[33];
-    const int64_t s = (int64_t)blockIdx.x * NB_TILE + threadIdx.x;
-    const int f = (s < nb.cap && nb.keys[s] != EMPTY_KEY) ? 1 : 0;
-    int tot;
-    const int r = block_rank(f, sm, &tot);
-    if (!f) return;
-    const int j = nb.tiles[blockIdx.x] + r;
-    nb.vidx[s] = j;
-    nb.v_slot[j] = (int)s;
-    const int64_t* acc = nb.acc + 4 * s;
-    const double w = (double)acc[3];
-    // the voxel's mean, exact from the fixed-point sums (the reference divides float sums, gpu.py:823)
-    nb.v_xyz[3 * (int64_t)j + 0] = (float)((double)acc[0] / (w * LW_FIX_W));
-    nb.v_xyz[3 * (int64_t)j + 1] = (float)((double)acc[1] / (w * LW_FIX_W));
-    nb.v_xyz[3 * (int64_t)j + 2] = (float)((double)acc[2] / (w * LW_FIX_W));
-    nb.v_w[j] = (int)acc[3];
+__device__ __forceinline__ int64_t nb_voxels(const lw_nbr_buf& nb, int64_t vcap) {
+    return min((int64_t)*(const unsigned*)nb.m, vcap);
 }
 
-__device__ __forceinline__ long long warp_sum_ll(long long v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+// The voxels' means, exact from the fixed-point sums (the reference divides float sums, gpu.py:823), and weights.
+__global__ void k_nb_mean(lw_nbr_buf nb, int64_t vcap) {
+    const int64_t m = nb_voxels(nb, vcap);
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < m; v += (int64_t)gridDim.x * blockDim.x) {
+        const longlong2* acc = reinterpret_cast<const longlong2*>(nb.acc + 4 * v);
+        const longlong2 p = acc[0], q = acc[1];
+        const double w = (double)q.y;
+        const float x = (float)((double)p.x / (w * LW_FIX_W)), y = (float)((double)p.y / (w * LW_FIX_W)),
+                    z = (float)((double)q.x / (w * LW_FIX_W));
+        *reinterpret_cast<float4*>(nb.acc + 4 * v) = make_float4(x, y, z, __int_as_float((int)q.y));
+    }
 }
 
-// A warp per voxel (gpu.py:829-876): its lanes probe the 343 voxel offsets 32 at a time; every voxel whose centroid
-// lies within the radius adds its points' weight, weighted offset and weighted outer product in fixed point. Lane 0
-// forms the count, and with want_normals the covariance's smallest-eigenvalue vector turned toward the sensor and
-// the curvature (smallest eigenvalue / trace).
-__global__ void k_nb_voxel(NbArgs a, lw_nbr_buf nb) {
-    const int m = *nb.m;
+// A thread per voxel, in brick order (gpu.py:829-876): every voxel whose centroid lies within the radius adds its
+// points' weight, weighted offset and weighted outer product in fixed point; from them the count, and with want_normals
+// the covariance's smallest-eigenvalue vector turned toward the sensor and the curvature (smallest eigenvalue / trace).
+// Bound by the candidates' walk and the float64 eigen-decomposition, which a thread per voxel runs on full warps. On 0.5M
+// voxels of a scanned floor a warp per voxel probing 343 offsets, its lane 0 decomposing alone, took 3.15 ms.
+constexpr int NB_THREADS = 128;
+
+__global__ void __launch_bounds__(NB_THREADS) k_nb_voxel(NbArgs a, lw_nbr_buf nb) {
+    __shared__ BrickRows rows_s[NB_THREADS / 32];
+    const int64_t m = nb_voxels(nb, a.vcap);
     const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-    constexpr int S = 2 * NB_REACH + 1, N = S * S * S;
-    for (int j = warp; j < m; j += nwarps) {
-        const float px = nb.v_xyz[3 * (int64_t)j], py = nb.v_xyz[3 * (int64_t)j + 1], pz = nb.v_xyz[3 * (int64_t)j + 2];
-        const int64_t key = nb.keys[nb.v_slot[j]];
-        const int ix = (int)(key & KEY_MASK) - (int)KEY_BIAS;
-        const int iy = (int)((key >> 21) & KEY_MASK) - (int)KEY_BIAS;
-        const int iz = (int)((key >> 42) & KEY_MASK) - (int)KEY_BIAS;
+    BrickRows& rows = rows_s[threadIdx.x >> 5];
+    const BrickHash bh = nb_hash(nb, a.mask);
+    for (int64_t j0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); j0 < m;
+         j0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t j = j0 + lane;
+        const int slot = j < m ? __float_as_int(nb.v_cnt[j]) : -1;
+        const float4 P = j < m ? *reinterpret_cast<const float4*>(nb.acc + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
         long long W = 0, s1[3] = {0, 0, 0}, s2[6] = {0, 0, 0, 0, 0, 0};
-        for (int o0 = 0; o0 < N; o0 += 32) {
-            const int o = o0 + lane;
-            if (o >= N) continue;
-            const int dz = o % S - NB_REACH, dy = (o / S) % S - NB_REACH, dx = o / (S * S) - NB_REACH;
-            const int s = find_slot(key_ijk(ix + dx, iy + dy, iz + dz), nb.keys, a.mask);
-            if (s < 0) continue;
-            const int k = nb.vidx[s];
-            const float ex = nb.v_xyz[3 * (int64_t)k] - px, ey = nb.v_xyz[3 * (int64_t)k + 1] - py,
-                        ez = nb.v_xyz[3 * (int64_t)k + 2] - pz;
-            if (ex * ex + ey * ey + ez * ez > a.r2) continue;
-            const long long w = nb.v_w[k];
-            const float FD = (float)NB_FIX_D, FDD = (float)NB_FIX_DD;
-            W += w;
-            s1[0] += w * to_fix(ex, FD);
-            s1[1] += w * to_fix(ey, FD);
-            s1[2] += w * to_fix(ez, FD);
-            s2[0] += w * to_fix(ex * ex, FDD);
-            s2[1] += w * to_fix(ex * ey, FDD);
-            s2[2] += w * to_fix(ex * ez, FDD);
-            s2[3] += w * to_fix(ey * ey, FDD);
-            s2[4] += w * to_fix(ey * ez, FDD);
-            s2[5] += w * to_fix(ez * ez, FDD);
-        }
-        W = warp_sum_ll(W);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) s1[c] = warp_sum_ll(s1[c]);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) s2[c] = warp_sum_ll(s2[c]);
-        if (lane != 0) continue;
+        brick_rows(bh, slot, rows, [&](int row) {
+            // my place in my brick: the mask's (j - base)th set bit
+            const int bit = nth_bit(rows.mask[row][13], (int)j - rows.base[row][13]);
+#pragma unroll 1
+            for (int c = 0; c < 27; ++c) {
+                const uint64_t all = rows.mask[row][c];
+                uint64_t near = all & brick_window(bit, c % 3 - 1, c / 3 % 3 - 1, c / 9 - 1, NB_REACH);
+                const int base = rows.base[row][c];
+                while (near) {
+                    const int b = __ffsll((long long)near) - 1;
+                    near &= near - 1;
+                    const int64_t k = base + popc64(all & ((1ull << b) - 1));
+                    if (k >= m) continue;
+                    const float4 Q = *reinterpret_cast<const float4*>(nb.acc + 4 * k);
+                    const float ex = Q.x - P.x, ey = Q.y - P.y, ez = Q.z - P.z;
+                    if (ex * ex + ey * ey + ez * ez > a.r2) continue;
+                    const int w = __float_as_int(Q.w);
+                    const float FD = (float)NB_FIX_D, FDD = (float)NB_FIX_DD;
+                    W += w;
+                    // an offset of at most 4 m is below 2^22 units: 32 bits
+                    s1[0] += (long long)w * __float2int_rn(ex * FD);
+                    s1[1] += (long long)w * __float2int_rn(ey * FD);
+                    s1[2] += (long long)w * __float2int_rn(ez * FD);
+                    s2[0] += w * to_fix(ex * ex, FDD);
+                    s2[1] += w * to_fix(ex * ey, FDD);
+                    s2[2] += w * to_fix(ex * ez, FDD);
+                    s2[3] += w * to_fix(ey * ey, FDD);
+                    s2[4] += w * to_fix(ey * ez, FDD);
+                    s2[5] += w * to_fix(ez * ez, FDD);
+                }
+            }
+        });
+        if (j >= m) continue;
         nb.v_cnt[j] = (float)W;
         if (a.want_normals == 0) continue;
         // toward the sensor, in float64 from the float coordinates
-        double tx = a.sensor[0] - (double)px, ty = a.sensor[1] - (double)py, tz = a.sensor[2] - (double)pz;
+        double tx = a.sensor[0] - (double)P.x, ty = a.sensor[1] - (double)P.y, tz = a.sensor[2] - (double)P.z;
         const double tl = sqrt(tx * tx + ty * ty + tz * tz);
         if (tl > 0.0) {
             tx /= tl;
@@ -188,13 +196,17 @@ __global__ void k_nb_voxel(NbArgs a, lw_nbr_buf nb) {
                               (double)s1[2] / NB_FIX_D * inv};
         const int up[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
         double C[9], ev[3], Q[9];
+#pragma unroll
         for (int r = 0; r < 3; ++r)
+#pragma unroll
             for (int c = 0; c < 3; ++c) C[r * 3 + c] = (double)s2[up[r * 3 + c]] / NB_FIX_DD * inv - mu[r] * mu[c];
         jacobi_eig<3>(C, ev, Q);
         int kmin = 0;
         if (ev[1] < ev[kmin]) kmin = 1;
         if (ev[2] < ev[kmin]) kmin = 2;
-        double nx = Q[0 * 3 + kmin], ny = Q[1 * 3 + kmin], nz = Q[2 * 3 + kmin];
+        // selects instead of indexing keep ev and Q in registers
+        auto at = [](const double* v, int k) { return k == 0 ? v[0] : (k == 1 ? v[1] : v[2]); };
+        double nx = at(Q, kmin), ny = at(Q + 3, kmin), nz = at(Q + 6, kmin);
         const double nl = sqrt(nx * nx + ny * ny + nz * nz);
         if (nl > 0.0) {
             nx /= nl;
@@ -212,10 +224,10 @@ __global__ void k_nb_voxel(NbArgs a, lw_nbr_buf nb) {
             ny = ty;
             nz = tz;
         }
-        nb.v_nrm[3 * (int64_t)j + 0] = (float)nx;
-        nb.v_nrm[3 * (int64_t)j + 1] = (float)ny;
-        nb.v_nrm[3 * (int64_t)j + 2] = (float)nz;
-        nb.v_curv[j] = (float)(fmax(ev[kmin], 0.0) / fmax(tr, 1.0e-12));
+        nb.v_nrm[3 * j + 0] = (float)nx;
+        nb.v_nrm[3 * j + 1] = (float)ny;
+        nb.v_nrm[3 * j + 2] = (float)nz;
+        nb.v_curv[j] = (float)(fmax(at(ev, kmin), 0.0) / fmax(tr, 1.0e-12));
     }
 }
 
@@ -237,7 +249,7 @@ __global__ void k_nb_gather(const int* n_dev, int64_t n_ub, int want_normals, lw
             }
             continue;
         }
-        const int v = nb.vidx[s];
+        const int v = s;
         cnt[i] = (int)(nb.v_cnt[v] + 0.5f);
         if (want_normals) {
             nrm[3 * i] = nb.v_nrm[3 * (int64_t)v];
@@ -274,28 +286,38 @@ int lw_neighborhoods(const float* xyz, int32_t xyz_stride, const int32_t* n_dev,
     NbArgs a{};
     a.inv_h = 3.0f / radius;  // voxels a third of the radius wide (gpu.py:1539)
     a.r2 = radius * radius;
-    a.mask = (int)(nb->cap - 1);
+    const int64_t slots = brick_slots(n_ub, nb->cap);
+    a.mask = (int)(slots - 1);
     a.want_normals = want_normals ? 1 : 0;
     for (int k = 0; k < 3; ++k) a.sensor[k] = sensor ? (double)sensor[k] : 0.0;
-    LW_CUDA(cudaMemsetAsync(nb->keys, 0xFF, sizeof(int64_t) * nb->cap, s));  // EMPTY_KEY is -1
-    LW_CUDA(cudaMemsetAsync(nb->acc, 0, sizeof(int64_t) * 4 * nb->cap, s));
-    LW_CUDA(cudaMemsetAsync(nb->m, 0, sizeof(int32_t), s));
-    if (n_ub <= 0) return LW_OK;
+    lw_nbr_buf b = *nb;
+    a.vcap = b.cap;
+    if ((uintptr_t)b.acc & 8) {  // the voxel records are read 16 bytes at a time
+        b.acc += 1;
+        a.vcap -= 1;
+    }
     const int sms = device_sms();
+    if (n_ub <= 0) {
+        LW_CUDA(cudaMemsetAsync(nb->m, 0, sizeof(int32_t), s));
+        return LW_OK;
+    }
+    k_nb_clear<<<blocks_for(slots, 256, 16 * sms), 256, 0, s>>>(b, slots);
     const int grid = blocks_for(n_ub, 256, 8 * sms);
     if (xyz_stride == 4)
-        k_nb_insert<4><<<grid, 256, 0, s>>>(xyz, n_dev, n_ub, a, *nb);
+        k_nb_insert<4><<<grid, 256, 0, s>>>(xyz, n_dev, n_ub, a, b);
     else
-        k_nb_insert<3><<<grid, 256, 0, s>>>(xyz, n_dev, n_ub, a, *nb);
-    const int nt = blocks_for(nb->cap, NB_TILE);
-    k_nb_count<<<nt, NB_TILE, 0, s>>>(*nb);
-    k_nb_scan<<<1, 1024, 0, s>>>(*nb, nt);
-    k_nb_scatter<<<nt, NB_TILE, 0, s>>>(*nb);
-    // a warp per voxel: at most one voxel per point
-    k_nb_voxel<<<blocks_for(n_ub * 32, 256, 16 * sms), 256, 0, s>>>(a, *nb);
-    k_nb_gather<<<grid, 256, 0, s>>>(n_dev, n_ub, a.want_normals, *nb, out_cnt, out_nrm, out_curv);
+        k_nb_insert<3><<<grid, 256, 0, s>>>(xyz, n_dev, n_ub, a, b);
+    k_nb_number<<<blocks_for(slots, 1024), 1024, 0, s>>>(b, slots, a.vcap);
+    if (xyz_stride == 4)
+        k_nb_sum<4><<<grid, 256, 0, s>>>(xyz, n_dev, n_ub, a, b);
+    else
+        k_nb_sum<3><<<grid, 256, 0, s>>>(xyz, n_dev, n_ub, a, b);
+    // at most one voxel per point
+    k_nb_mean<<<grid, 256, 0, s>>>(b, a.vcap);
+    k_nb_voxel<<<blocks_for(n_ub, NB_THREADS, 16 * sms), NB_THREADS, 0, s>>>(a, b);
+    k_nb_gather<<<grid, 256, 0, s>>>(n_dev, n_ub, a.want_normals, b, out_cnt, out_nrm, out_curv);
     LW_LAUNCHED("lw_neighborhoods");
-    count_launches(6);
+    count_launches(7);
     return LW_OK;
 }
 
