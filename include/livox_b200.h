@@ -480,23 +480,25 @@ int lw_ground(const float* xyz, int32_t xyz_stride, const float* nrm, const int3
               float thick, int32_t min_sup, float thresh, float slope_step, int32_t use_normals, float nz_min,
               float* cell_min, int32_t* cell_sup, int32_t* out_gnd, float* out_hag, void* stream);
 
-/* Buffers of the Euclidean clustering; "between calls" values are restored by every call. */
+/* Buffers of the Euclidean clustering, contents undefined between calls. A call gathers the voxels into bricks of
+ * 4 x 4 x 4 in an open-addressed table (the first power of two of at least 2 n of its cap slots) and numbers them
+ * brick by brick. */
 typedef struct lw_cluster_buf {
-    int64_t* keys;       /* [cap] voxel keys, -1 between calls */
-    int64_t* acc;        /* [cap*4] fixed-point x, y, z sums (LW_FIX_W) and point count, 0 between calls */
-    int32_t* first;      /* [cap] lowest point index per voxel, INT32_MAX between calls */
-    int32_t* vidx;       /* [cap] node of a slot */
-    int32_t* slot_of_pt; /* [pt_cap] */
+    int64_t* keys;       /* [cap] brick keys, -1 empty */
+    int64_t* acc;        /* [cap*4] the bricks' masks of occupied voxels and first voxels */
+    int32_t* first;      /* [cap] not used */
+    int32_t* vidx;       /* [cap] not used */
+    int32_t* slot_of_pt; /* [pt_cap] voxel of a point, -1 for ground and when the table was full */
     int32_t* tiles;      /* [pt_cap/1024 + 2] */
-    int32_t* node_slot;  /* [pt_cap] slot of a node */
+    int32_t* node_slot;  /* [pt_cap] voxel of a node */
     float* v_xyz;        /* [pt_cap*3] node centroids */
     int32_t* v_w;        /* [pt_cap] node point counts */
-    int32_t* edge_off;   /* [pt_cap + 1] */
-    int32_t* edges;      /* [edge_cap] neighbour lists */
+    int32_t* edge_off;   /* [pt_cap + 1] node of a voxel */
+    int32_t* edges;      /* [edge_cap] not used (may be NULL with edge_cap 0) */
     int32_t* label;      /* [pt_cap] component of a node: its smallest node index */
-    int64_t* st_sum;     /* [pt_cap*4] per-root fixed-point sums and count, 0 between calls */
-    float* st_lo;        /* [pt_cap*3] per-root minimum corner, +1e30 between calls */
-    float* st_hi;        /* [pt_cap*3] per-root maximum corner, -1e30 between calls */
+    int64_t* st_sum;     /* [pt_cap*4] per-voxel, then per-root fixed-point sums and count */
+    float* st_lo;        /* [pt_cap*3] per-root minimum corner */
+    float* st_hi;        /* [pt_cap*3] per-root maximum corner */
     int32_t* dense;      /* [pt_cap] dense cluster id of a root, -1 */
     float* out_cnt;      /* [max_out] points per cluster */
     float* out_cen;      /* [max_out*3] centroids */
@@ -504,7 +506,7 @@ typedef struct lw_cluster_buf {
     float* out_hi;       /* [max_out*3] */
     int32_t* m;          /* [1] nodes of the last call */
     int32_t* n_clusters; /* [2] clusters kept, clusters before the max_out cap */
-    int32_t* err;        /* [1] non-zero when a buffer was too small or a bounded loop gave up */
+    int32_t* err;        /* [1] non-zero when a bounded loop gave up */
     int64_t cap, pt_cap, edge_cap;
 } lw_cluster_buf;
 

@@ -14,14 +14,6 @@ namespace lw {
 
 constexpr int64_t BRICK_MASK = (1LL << 19) - 1;  // a 21-bit field without its two low bits
 
-struct BrickHash {
-    const int64_t* keys;
-    const uint32_t* lo;  // the mask's halves
-    const uint32_t* hi;
-    const int32_t* base;
-    int mask;
-};
-
 __device__ __forceinline__ int64_t brick_key(int64_t bx, int64_t by, int64_t bz) {
     return (bx & BRICK_MASK) | ((by & BRICK_MASK) << 19) | ((bz & BRICK_MASK) << 38);
 }
@@ -85,8 +77,10 @@ struct BrickRows {
 // lane calls), run(row) with the neighbouring bricks of the lane's own brick in rows.mask[row], rows.base[row].
 // Voxels of a brick are neighbours in number, so 32 lanes hold a few bricks; their 27-brick neighbourhoods are
 // looked up by all lanes together, BRICK_ROWS at a time.
-template <class Run>
-__device__ __forceinline__ void brick_rows(const BrickHash& bh, int slot, BrickRows& rows, const Run& run) {
+// mask_of(s) is the mask of the brick in slot s of the hash (keys, base, hash_mask).
+template <class MaskOf, class Run>
+__device__ __forceinline__ void brick_rows(const int64_t* keys, const int32_t* base, int hash_mask, const MaskOf& mask_of,
+                                           int slot, BrickRows& rows, const Run& run) {
     const int lane = threadIdx.x & 31;
     const int prev = __shfl_up_sync(0xffffffffu, slot, 1);
     const unsigned leaders = __ballot_sync(0xffffffffu, slot >= 0 && (lane == 0 || slot != prev));
@@ -101,7 +95,7 @@ __device__ __forceinline__ void brick_rows(const BrickHash& bh, int slot, BrickR
             const int src = left ? __ffs(left) - 1 : 0;
             left &= left - 1;
             const int s = __shfl_sync(0xffffffffu, slot, src);
-            lead_key[r] = r < here ? bh.keys[s] : 0;
+            lead_key[r] = r < here ? keys[s] : 0;
         }
 #pragma unroll
         for (int u = 0; u < (BRICK_ROWS * 27 + 31) / 32; ++u) {
@@ -112,9 +106,9 @@ __device__ __forceinline__ void brick_rows(const BrickHash& bh, int slot, BrickR
                 for (int q = 1; q < BRICK_ROWS; ++q) k = r == q ? lead_key[q] : k;
                 const int64_t nk = brick_key((k & BRICK_MASK) + (c % 3 - 1), (k >> 19 & BRICK_MASK) + (c / 3 % 3 - 1),
                                              (k >> 38 & BRICK_MASK) + (c / 9 - 1));
-                const int s = find_slot(nk, bh.keys, bh.mask);
-                rows.mask[r][c] = s < 0 ? 0ull : (uint64_t)bh.lo[s] | ((uint64_t)bh.hi[s] << 32);
-                rows.base[r][c] = s < 0 ? 0 : bh.base[s];
+                const int s = find_slot(nk, keys, hash_mask);
+                rows.mask[r][c] = s < 0 ? 0ull : mask_of(s);
+                rows.base[r][c] = s < 0 ? 0 : base[s];
             }
         }
         __syncwarp();
@@ -126,16 +120,15 @@ __device__ __forceinline__ void brick_rows(const BrickHash& bh, int slot, BrickR
 // Number the voxels brick by brick: a CTA per 1024 brick slots takes a run of numbers for its bricks (which run depends
 // on timing, so no result may depend on a voxel's number), writes each brick's base, each voxel's brick slot
 // (voxel_slot [vcap]) and whatever init(v) sets up for voxel v < vcap.
-template <class Init>
-__device__ __forceinline__ void brick_number(const int64_t* __restrict__ keys, const uint32_t* __restrict__ lo,
-                                             const uint32_t* __restrict__ hi, int32_t* __restrict__ base, int64_t slots,
-                                             int* counter, int32_t* __restrict__ voxel_slot, int64_t vcap,
-                                             const Init& init) {
+template <class MaskOf, class Init>
+__device__ __forceinline__ void brick_number(const int64_t* __restrict__ keys, const MaskOf& mask_of,
+                                             int32_t* __restrict__ base, int64_t slots, int* counter,
+                                             int32_t* __restrict__ voxel_slot, int64_t vcap, const Init& init) {
     __shared__ int sm[33];
     __shared__ int first;
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const bool used = s < slots && keys[s] != EMPTY_KEY;
-    const int c = used ? __popc(lo[s]) + __popc(hi[s]) : 0;
+    const int c = used ? popc64(mask_of((int)s)) : 0;
     int tot;
     const int r = block_excl(c, sm, &tot);
     if (tot == 0) return;

@@ -75,14 +75,13 @@ __global__ void k_nb_insert(const float* __restrict__ xyz, const int* n_dev, int
     }
 }
 
-__device__ __forceinline__ BrickHash nb_hash(const lw_nbr_buf& nb, int mask) {
-    return {nb.keys, reinterpret_cast<const uint32_t*>(nb.v_slot), reinterpret_cast<const uint32_t*>(nb.vidx), nb.v_w,
-            mask};
+__device__ __forceinline__ uint64_t nb_mask(const lw_nbr_buf& nb, int s) {
+    return (uint64_t)(uint32_t)nb.v_slot[s] | ((uint64_t)(uint32_t)nb.vidx[s] << 32);
 }
 
 __global__ void __launch_bounds__(1024) k_nb_number(lw_nbr_buf nb, int64_t slots, int64_t vcap) {
-    brick_number(nb.keys, reinterpret_cast<const uint32_t*>(nb.v_slot), reinterpret_cast<const uint32_t*>(nb.vidx),
-                 nb.v_w, slots, nb.m, reinterpret_cast<int32_t*>(nb.v_cnt), vcap, [&](int64_t v) {
+    brick_number(nb.keys, [&](int s) { return nb_mask(nb, s); }, nb.v_w, slots, nb.m,
+                 reinterpret_cast<int32_t*>(nb.v_cnt), vcap, [&](int64_t v) {
                      longlong2* a = reinterpret_cast<longlong2*>(nb.acc + 4 * v);
                      a[0] = a[1] = make_longlong2(0, 0);
                  });
@@ -100,8 +99,7 @@ __global__ void k_nb_sum(const float* __restrict__ xyz, const int* n_dev, int64_
         float x, y, z;
         int bit;
         nb_brick<STRIDE>(xyz, i, a, x, y, z, bit);
-        const uint64_t m = (uint64_t)(uint32_t)nb.v_slot[s] | ((uint64_t)(uint32_t)nb.vidx[s] << 32);
-        const int64_t v = (int64_t)nb.v_w[s] + popc64(m & ((1ull << bit) - 1));
+        const int64_t v = (int64_t)nb.v_w[s] + popc64(nb_mask(nb, s) & ((1ull << bit) - 1));
         if (v < a.vcap) {
             atomic_add_i64(nb.acc + 4 * v + 0, to_fix(x, FW));
             atomic_add_i64(nb.acc + 4 * v + 1, to_fix(y, FW));
@@ -141,14 +139,13 @@ __global__ void __launch_bounds__(NB_THREADS) k_nb_voxel(NbArgs a, lw_nbr_buf nb
     const int64_t m = nb_voxels(nb, a.vcap);
     const int lane = threadIdx.x & 31;
     BrickRows& rows = rows_s[threadIdx.x >> 5];
-    const BrickHash bh = nb_hash(nb, a.mask);
     for (int64_t j0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); j0 < m;
          j0 += (int64_t)gridDim.x * blockDim.x) {
         const int64_t j = j0 + lane;
         const int slot = j < m ? __float_as_int(nb.v_cnt[j]) : -1;
         const float4 P = j < m ? *reinterpret_cast<const float4*>(nb.acc + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
         long long W = 0, s1[3] = {0, 0, 0}, s2[6] = {0, 0, 0, 0, 0, 0};
-        brick_rows(bh, slot, rows, [&](int row) {
+        brick_rows(nb.keys, nb.v_w, a.mask, [&](int s) { return nb_mask(nb, s); }, slot, rows, [&](int row) {
             // my place in my brick: the mask's (j - base)th set bit
             const int bit = nth_bit(rows.mask[row][13], (int)j - rows.base[row][13]);
 #pragma unroll 1

@@ -7,8 +7,8 @@ the pipeline's visible points (pipe.c_xyz[:pipe.count]).
 
 Differences, deliberate: the ground grid is cleared once and then restored by each call (no 32 MB fill per call);
 the cluster nodes are ordered by their first point, so cluster ids are the same on every run; connected
-components come from one union-find pass over a neighbour graph built from the voxel hash, so cc_iters is 1 and
-cc_converged is True unless a buffer overflowed.
+components come from one union-find pass over the voxels' neighbours, so cc_iters is 1 and cc_converged is True
+unless a bounded loop gave up.
 """
 
 from __future__ import annotations
@@ -143,7 +143,7 @@ class Perception:
             "v_xyz": torch.zeros((n, 3), dtype=torch.float32, device=d),
             "v_w": torch.zeros(n, dtype=torch.int32, device=d),
             "edge_off": torch.zeros(n + 1, dtype=torch.int32, device=d),
-            "edges": torch.zeros(max(n * edge_factor // 8, 1 << 16), dtype=torch.int32, device=d),
+            "edges": torch.zeros(1, dtype=torch.int32, device=d),  # no edge list is kept (edge_factor sizes nothing)
             "label": torch.zeros(n, dtype=torch.int32, device=d),
             "st_sum": torch.zeros((n, 4), dtype=torch.int64, device=d),
             "st_lo": torch.full((n, 3), 1.0e30, dtype=torch.float32, device=d),
