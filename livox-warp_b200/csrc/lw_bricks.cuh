@@ -8,6 +8,8 @@
 //
 // Coordinates are the 21-bit fields of the voxel key (gpu.py:231-239), so neighbourhoods wrap where keys do.
 #pragma once
+#include <type_traits>
+
 #include "lw_common.cuh"
 
 namespace lw {
@@ -66,21 +68,27 @@ __device__ __forceinline__ uint64_t brick_window(int bit, int ox, int oy, int oz
     return x & y & z;
 }
 
-// The 27 bricks around each of up to BRICK_ROWS bricks, for one warp's voxels.
-constexpr int BRICK_ROWS = 4;
+// The 27 bricks around each of up to BRICK_ROWS bricks, for one CTA's voxels.
+constexpr int BRICK_ROWS = 4, BRICK_WARPS = 4;
+constexpr int BRICK_CTA = 32 * BRICK_WARPS;  // threads of a CTA that walks neighbourhoods: 32 voxels, BRICK_WARPS threads each
 struct BrickRows {
     uint64_t mask[BRICK_ROWS][27];
     int32_t base[BRICK_ROWS][27];
 };
 
-// For the voxels of a warp, a thread each in the order of their numbers (slot: the voxel's brick, -1 for none; every
-// lane calls), run(row) with the neighbouring bricks of the lane's own brick in rows.mask[row], rows.base[row].
-// Voxels of a brick are neighbours in number, so 32 lanes hold a few bricks; their 27-brick neighbourhoods are
-// looked up by all lanes together, BRICK_ROWS at a time.
-// mask_of(s) is the mask of the brick in slot s of the hash (keys, base, hash_mask).
-template <class MaskOf, class Run>
+// For the 32 voxels of a CTA, lane l of every warp serving voxel l, in the order of their numbers (slot: the voxel's
+// brick, -1 for none; every thread calls), run(row) with the bricks around the lane's own brick in rows.mask[row],
+// rows.base[row]. Voxels of a brick are neighbours in number, so 32 of them lie in a few bricks, whose 27 neighbours are
+// looked up side by side, BRICK_ROWS bricks at a time. The warps share out the 27 bricks (warp w takes w, w + BRICK_WARPS, ...):
+// a scene's voxels alone leave too few warps in flight to hide the walk's loads.
+// mask_of(s, r, c, lead) is the mask of the brick in slot s of the hash (keys, base, hash_mask), found for rows[r][c]
+// around the brick in slot lead.
+// after(r, c): run for each of the looked-up bricks once the lanes are done with them.
+struct NoAfter {};
+template <class MaskOf, class Run, class After>
 __device__ __forceinline__ void brick_rows(const int64_t* keys, const int32_t* base, int hash_mask, const MaskOf& mask_of,
-                                           int slot, BrickRows& rows, const Run& run) {
+                                           int slot, BrickRows& rows, const Run& run, const After& after) {
+    static_assert(BRICK_ROWS * 27 <= BRICK_CTA, "one lookup per thread");
     const int lane = threadIdx.x & 31;
     const int prev = __shfl_up_sync(0xffffffffu, slot, 1);
     const unsigned leaders = __ballot_sync(0xffffffffu, slot >= 0 && (lane == 0 || slot != prev));
@@ -89,31 +97,29 @@ __device__ __forceinline__ void brick_rows(const int64_t* keys, const int32_t* b
     unsigned left = leaders;
     for (int r0 = 0; r0 < nrows; r0 += BRICK_ROWS) {
         const int here = min(BRICK_ROWS, nrows - r0);
-        int64_t lead_key[BRICK_ROWS];
+        const int r = threadIdx.x / 27, c = threadIdx.x - 27 * r;
+        int lead = 0, s = -1;
 #pragma unroll
-        for (int r = 0; r < BRICK_ROWS; ++r) {
-            const int src = left ? __ffs(left) - 1 : 0;
+        for (int q = 0; q < BRICK_ROWS; ++q) {
+            const int ls = __shfl_sync(0xffffffffu, slot, left ? __ffs(left) - 1 : 0);
             left &= left - 1;
-            const int s = __shfl_sync(0xffffffffu, slot, src);
-            lead_key[r] = r < here ? keys[s] : 0;
+            lead = q == r ? ls : lead;
         }
-#pragma unroll
-        for (int u = 0; u < (BRICK_ROWS * 27 + 31) / 32; ++u) {
-            const int t = lane + 32 * u, r = t / 27, c = t - 27 * r;
-            if (r < here) {
-                int64_t k = lead_key[0];
-#pragma unroll
-                for (int q = 1; q < BRICK_ROWS; ++q) k = r == q ? lead_key[q] : k;
-                const int64_t nk = brick_key((k & BRICK_MASK) + (c % 3 - 1), (k >> 19 & BRICK_MASK) + (c / 3 % 3 - 1),
-                                             (k >> 38 & BRICK_MASK) + (c / 9 - 1));
-                const int s = find_slot(nk, keys, hash_mask);
-                rows.mask[r][c] = s < 0 ? 0ull : mask_of(s);
-                rows.base[r][c] = s < 0 ? 0 : base[s];
-            }
+        if (r < here) {
+            const int64_t k = keys[lead];
+            const int64_t nk = brick_key((k & BRICK_MASK) + (c % 3 - 1), (k >> 19 & BRICK_MASK) + (c / 3 % 3 - 1),
+                                         (k >> 38 & BRICK_MASK) + (c / 9 - 1));
+            s = c == 13 ? lead : find_slot(nk, keys, hash_mask);
+            rows.mask[r][c] = s < 0 ? 0ull : mask_of(s, r, c, lead);
+            rows.base[r][c] = s < 0 ? 0 : base[s];
         }
-        __syncwarp();
+        __syncthreads();
         if (slot >= 0 && mine >= r0 && mine < r0 + here) run(mine - r0);
-        __syncwarp();
+        __syncthreads();
+        if constexpr (!std::is_same<After, NoAfter>::value) {
+            if (s >= 0) after(r, c);
+            __syncthreads();  // after() may read what other threads' lookups left: not before all are done with it
+        }
     }
 }
 

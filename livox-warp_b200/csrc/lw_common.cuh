@@ -166,6 +166,22 @@ __device__ __forceinline__ void atomic_add_i64(int64_t* a, int64_t v) {
 // float -> int64 fixed point, round to nearest even (llrintf on the host).
 __device__ __forceinline__ int64_t to_fix(float v, float scale) { return __float2ll_rn(v * scale); }
 
+// to_fix for sums of many terms, without the float -> int64 conversion (a quarter-rate or slower instruction; six to nine of
+// them per term bound the neighbourhood kernels). Adding 1.5 x 2^23 to a float below 2^22 in magnitude rounds it to
+// the nearest integer, ties to even as the conversion does, and leaves that integer in the low bits. A product v below
+// 2^42 is split as v = hi 2^20 + lo with hi = rint(v 2^-20) and lo exact and at most 2^19, so
+// rint(v) = hi 2^20 + rint(lo): two 32-bit integers, each from one addition.
+constexpr float RINT_MAGIC = 12582912.0f;   // 1.5 x 2^23
+constexpr int RINT_BITS = 0x4B400000;       // its bits: those of a rounded value less these are the integer
+
+__device__ __forceinline__ int rint_bits(float v) { return __float_as_int(v + RINT_MAGIC); }  // integer + RINT_BITS
+
+__device__ __forceinline__ void rint_split(float v, int& hi_bits, int& lo_bits) {
+    const float h = fmaf(v, 9.5367431640625e-07f, RINT_MAGIC);  // 2^-20
+    hi_bits = __float_as_int(h);
+    lo_bits = rint_bits(fmaf(h - RINT_MAGIC, -1048576.0f, v));
+}
+
 // ---- reductions --------------------------------------------------------------------------------------------
 // claim_slot with the compare-and-swap as the probe: one atomic round trip per probed slot, where a load first
 // costs two for a slot found empty. The same slot results (a key is in at most one slot of its probe sequence:

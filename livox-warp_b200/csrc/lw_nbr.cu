@@ -127,29 +127,28 @@ __global__ void k_nb_mean(lw_nbr_buf nb, int64_t vcap) {
     }
 }
 
-// A thread per voxel, in brick order (gpu.py:829-876): every voxel whose centroid lies within the radius adds its
-// points' weight, weighted offset and weighted outer product in fixed point; from them the count, and with want_normals
-// the covariance's smallest-eigenvalue vector turned toward the sensor and the curvature (smallest eigenvalue / trace).
-// Bound by the candidates' walk and the float64 eigen-decomposition, which a thread per voxel runs on full warps. On 0.5M
-// voxels of a scanned floor a warp per voxel probing 343 offsets, its lane 0 decomposing alone, took 3.15 ms.
-constexpr int NB_THREADS = 128;
-
-__global__ void __launch_bounds__(NB_THREADS) k_nb_voxel(NbArgs a, lw_nbr_buf nb) {
-    __shared__ BrickRows rows_s[NB_THREADS / 32];
+// The voxels in brick order (gpu.py:829-876): every voxel whose centroid lies within the radius adds its points' weight,
+// weighted offset and weighted outer product in fixed point; from them the count, and with want_normals the
+// covariance's smallest-eigenvalue vector turned toward the sensor and the curvature (smallest eigenvalue / trace).
+// Bound by the issue of the candidates' arithmetic at a third of the lanes (each lane has its own window). On 0.5M voxels of a
+// scanned floor a warp per voxel probing 343 offsets, its lane 0 decomposing alone, took 3.15 ms.
+// SMALL (a radius below 2 m, so offset products stay below 2^42 units): sums from rounded bits (rint_split) instead of
+// float -> int64 conversions.
+template <bool SMALL>
+__global__ void __launch_bounds__(BRICK_CTA) k_nb_voxel(NbArgs a, lw_nbr_buf nb) {
+    __shared__ BrickRows rows;
+    __shared__ long long part[BRICK_WARPS - 1][10][32];
     const int64_t m = nb_voxels(nb, a.vcap);
-    const int lane = threadIdx.x & 31;
-    BrickRows& rows = rows_s[threadIdx.x >> 5];
-    for (int64_t j0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); j0 < m;
-         j0 += (int64_t)gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int64_t j0 = (int64_t)blockIdx.x * 32; j0 < m; j0 += (int64_t)gridDim.x * 32) {
         const int64_t j = j0 + lane;
         const int slot = j < m ? __float_as_int(nb.v_cnt[j]) : -1;
         const float4 P = j < m ? *reinterpret_cast<const float4*>(nb.acc + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
-        long long W = 0, s1[3] = {0, 0, 0}, s2[6] = {0, 0, 0, 0, 0, 0};
-        brick_rows(nb.keys, nb.v_w, a.mask, [&](int s) { return nb_mask(nb, s); }, slot, rows, [&](int row) {
-            // my place in my brick: the mask's (j - base)th set bit
+        long long W = 0, s1[3] = {0, 0, 0}, s2[6] = {0, 0, 0, 0, 0, 0}, lo[6] = {0, 0, 0, 0, 0, 0};
+        brick_rows(nb.keys, nb.v_w, a.mask, [&](int s, int, int, int) { return nb_mask(nb, s); }, slot, rows, [&](int row) {
             const int bit = nth_bit(rows.mask[row][13], (int)j - rows.base[row][13]);
 #pragma unroll 1
-            for (int c = 0; c < 27; ++c) {
+            for (int c = warp; c < 27; c += BRICK_WARPS) {
                 const uint64_t all = rows.mask[row][c];
                 uint64_t near = all & brick_window(bit, c % 3 - 1, c / 3 % 3 - 1, c / 9 - 1, NB_REACH);
                 const int base = rows.base[row][c];
@@ -164,20 +163,57 @@ __global__ void __launch_bounds__(NB_THREADS) k_nb_voxel(NbArgs a, lw_nbr_buf nb
                     const int w = __float_as_int(Q.w);
                     const float FD = (float)NB_FIX_D, FDD = (float)NB_FIX_DD;
                     W += w;
-                    // an offset of at most 4 m is below 2^22 units: 32 bits
-                    s1[0] += (long long)w * __float2int_rn(ex * FD);
-                    s1[1] += (long long)w * __float2int_rn(ey * FD);
-                    s1[2] += (long long)w * __float2int_rn(ez * FD);
-                    s2[0] += w * to_fix(ex * ex, FDD);
-                    s2[1] += w * to_fix(ex * ey, FDD);
-                    s2[2] += w * to_fix(ex * ez, FDD);
-                    s2[3] += w * to_fix(ey * ey, FDD);
-                    s2[4] += w * to_fix(ey * ez, FDD);
-                    s2[5] += w * to_fix(ez * ez, FDD);
+                    if constexpr (SMALL) {
+                        const float fx = ex * FD, fy = ey * FD, fz = ez * FD;  // exact: FD^2 = FDD
+                        s1[0] += (long long)w * rint_bits(fx);
+                        s1[1] += (long long)w * rint_bits(fy);
+                        s1[2] += (long long)w * rint_bits(fz);
+                        const float v[6] = {fx * fx, fx * fy, fx * fz, fy * fy, fy * fz, fz * fz};
+#pragma unroll
+                        for (int t = 0; t < 6; ++t) {
+                            int h, l;
+                            rint_split(v[t], h, l);
+                            s2[t] += (long long)w * h;
+                            lo[t] += (long long)w * l;
+                        }
+                    } else {
+                        s1[0] += (long long)w * __float2int_rn(ex * FD);  // at most 4 m: 2^22 units
+                        s1[1] += (long long)w * __float2int_rn(ey * FD);
+                        s1[2] += (long long)w * __float2int_rn(ez * FD);
+                        s2[0] += w * to_fix(ex * ex, FDD);
+                        s2[1] += w * to_fix(ex * ey, FDD);
+                        s2[2] += w * to_fix(ex * ez, FDD);
+                        s2[3] += w * to_fix(ey * ey, FDD);
+                        s2[4] += w * to_fix(ey * ez, FDD);
+                        s2[5] += w * to_fix(ez * ez, FDD);
+                    }
                 }
             }
-        });
-        if (j >= m) continue;
+        }, NoAfter());
+        if constexpr (SMALL) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) s1[c] -= W * RINT_BITS;
+#pragma unroll
+            for (int c = 0; c < 6; ++c) s2[c] = ((s2[c] - W * RINT_BITS) << 20) + (lo[c] - W * RINT_BITS);
+        }
+        if (warp > 0) {
+            long long(*p)[32] = part[warp - 1];
+            p[0][lane] = W;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) p[1 + c][lane] = s1[c];
+#pragma unroll
+            for (int c = 0; c < 6; ++c) p[4 + c][lane] = s2[c];
+        }
+        __syncthreads();
+        if (warp > 0 || j >= m) continue;  // the next round's first barrier comes after this round's reads of part
+#pragma unroll
+        for (int q = 0; q < BRICK_WARPS - 1; ++q) {
+            W += part[q][0][lane];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) s1[c] += part[q][1 + c][lane];
+#pragma unroll
+            for (int c = 0; c < 6; ++c) s2[c] += part[q][4 + c][lane];
+        }
         nb.v_cnt[j] = (float)W;
         if (a.want_normals == 0) continue;
         // toward the sensor, in float64 from the float coordinates
@@ -311,7 +347,11 @@ int lw_neighborhoods(const float* xyz, int32_t xyz_stride, const int32_t* n_dev,
         k_nb_sum<3><<<grid, 256, 0, s>>>(xyz, n_dev, n_ub, a, b);
     // at most one voxel per point
     k_nb_mean<<<grid, 256, 0, s>>>(b, a.vcap);
-    k_nb_voxel<<<blocks_for(n_ub, NB_THREADS, 16 * sms), NB_THREADS, 0, s>>>(a, b);
+    const int gridv = blocks_for(n_ub, 32, 64 * sms);
+    if (radius < 1.99f)
+        k_nb_voxel<true><<<gridv, BRICK_CTA, 0, s>>>(a, b);
+    else
+        k_nb_voxel<false><<<gridv, BRICK_CTA, 0, s>>>(a, b);
     k_nb_gather<<<grid, 256, 0, s>>>(n_dev, n_ub, a.want_normals, b, out_cnt, out_nrm, out_curv);
     LW_LAUNCHED("lw_neighborhoods");
     count_launches(7);

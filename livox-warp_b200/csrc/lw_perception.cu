@@ -137,7 +137,7 @@ struct ClArgs {
     int max_out;
 };
 
-// The bricks' masks and bases, in the caller's acc: [slots] 64-bit masks, then [slots] 32-bit bases.
+// The bricks' masks and bases, in the caller's acc: [slots] 64-bit masks, [slots] 32-bit bases, [slots] common labels.
 __device__ __forceinline__ uint64_t* cl_masks(const lw_cluster_buf& cb) { return reinterpret_cast<uint64_t*>(cb.acc); }
 __device__ __forceinline__ int32_t* cl_bases(const lw_cluster_buf& cb, int64_t slots) {
     return reinterpret_cast<int32_t*>(cb.acc + slots);
@@ -250,7 +250,6 @@ __global__ void k_cl_node_scatter(const int* n_dev, int64_t n_ub, lw_cluster_buf
     const int j = base + r;
     cb.node_slot[j] = v;
     cb.edge_off[v] = j;
-    cb.label[j] = j;
     const int64_t* acc = cb.st_sum + 4 * (int64_t)v;
     double w = (double)acc[3];
     cb.v_w[j] = (int)acc[3];
@@ -262,82 +261,183 @@ __global__ void k_cl_node_scatter(const int* n_dev, int64_t n_ub, lw_cluster_buf
     }
 }
 
-constexpr int UF_SPINS = 1 << 20;
+constexpr int UF_HOPS = 1 << 20;
 
+// The root of x, or -1 after UF_HOPS hops.
 __device__ __forceinline__ int uf_find(int* parent, int x) {
-    for (int it = 0; it < UF_SPINS; ++it) {
-        int p = parent[x];
+    for (int it = 0; it < UF_HOPS; ++it) {
+        // through L2: another SM's hook must be seen, or a lost CAS would be retried on the same stale root
+        int p = __ldcg(parent + x);
         if (p == x) return x;
-        int gp = parent[p];
-        if (gp != p) atomicMin(parent + x, gp);  // path halving; never raises a parent
+        int gp = __ldcg(parent + p);
+        if (gp != p) __stcg(parent + x, gp);  // path halving: x is no root, and any ancestor will do as its parent
         x = p;
     }
-    return x;
+    return -1;
 }
 
-// Pass 6: a thread per voxel, in brick order, joins it with every neighbour numbered above it (each pair once).
-// Hooks the larger root under the smaller; a CAS that loses a race retries with the new roots.
-// On 0.3M nodes of a scanned floor counting, writing, scanning and joining edge lists took 2.0 ms.
-constexpr int CL_THREADS = 128;
+// The one label of all voxels of a brick (from k_cl_brick), -1 when they have several.
+__device__ __forceinline__ int32_t* cl_common(const lw_cluster_buf& cb, int64_t slots) {
+    return reinterpret_cast<int32_t*>(cb.acc + slots) + slots;
+}
 
-__global__ void __launch_bounds__(CL_THREADS) k_cl_join(ClArgs a, lw_cluster_buf cb) {
-    __shared__ BrickRows rows_s[CL_THREADS / 32];
+// Put nodes x and y (any nodes of their components) in one component: hooks the larger root under the smaller; a CAS that
+// loses a race (another hook won: progress) retries with the new roots.
+__device__ __forceinline__ void uf_join(const lw_cluster_buf& cb, int x, int y) {
+    for (int it = 0; it < UF_HOPS; ++it) {
+        x = uf_find(cb.label, x);
+        y = uf_find(cb.label, y);
+        if (x < 0 || y < 0) break;
+        if (x == y) return;
+        const int hi = max(x, y), lo = min(x, y);
+        if (atomicCAS(cb.label + hi, hi, lo) == hi) return;
+    }
+    atomicExch(cb.err, 1);
+}
+
+// Pass 6: the components within each brick, a warp per brick and no atomics: every voxel's links to the brick's (at most 64)
+// voxels as a bit mask, closed over the links; the label is the component's smallest node. A brick of one component, as
+// most are, gets its label as the brick's common one.
+constexpr int CL_WARPS = 4;
+
+__global__ void __launch_bounds__(32 * CL_WARPS) k_cl_brick(ClArgs a, lw_cluster_buf cb) {
+    __shared__ float4 pos_s[CL_WARPS][64];  // x, y, z, bit
+    __shared__ int node_s[CL_WARPS][64];
+    __shared__ uint64_t link_s[CL_WARPS][64];
     const int m = *cb.m;
-    const int lane = threadIdx.x & 31;
-    BrickRows& rows = rows_s[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float4* pos = pos_s[warp];
+    int* node = node_s[warp];
+    uint64_t* link = link_s[warp];
+    const int64_t nwarps = (int64_t)gridDim.x * CL_WARPS;
+    for (int64_t w = (int64_t)blockIdx.x * CL_WARPS + warp; w * 32 < m; w += nwarps) {
+        const int64_t v0 = w * 32 + lane;
+        const int slot0 = v0 < m ? cl_brick(cb)[v0] : -1;
+        // the bricks whose first voxel is among the warp's 32
+        unsigned leads = __ballot_sync(0xffffffffu, slot0 >= 0 && cl_bases(cb, a.slots)[max(slot0, 0)] == (int)v0);
+        for (; leads; leads &= leads - 1) {
+            const int src = __ffs(leads) - 1;
+            const int slot = __shfl_sync(0xffffffffu, slot0, src);
+            const int64_t base = w * 32 + src;
+            const uint64_t mask = cl_masks(cb)[slot];
+            const int n = popc64(mask);
+            for (int k = lane; k < n; k += 32) {
+                const int64_t v = base + k;
+                pos[k] = make_float4(cb.st_lo[3 * v], cb.st_lo[3 * v + 1], cb.st_lo[3 * v + 2],
+                                     __int_as_float(nth_bit(mask, k)));
+                node[k] = cb.edge_off[v];
+            }
+            __syncwarp();
+            const uint64_t full = n == 64 ? ~0ull : (1ull << n) - 1;
+            for (int k = lane; k < n; k += 32) {
+                const float4 p = pos[k];
+                const uint64_t near = brick_window(__float_as_int(p.w), 0, 0, 0, a.reach);
+                uint64_t l = 1ull << k;
+                for (int q = 0; q < n; ++q) {
+                    const float4 o = pos[q];
+                    const float ex = o.x - p.x, ey = o.y - p.y, ez = o.z - p.z;
+                    if (ex * ex + ey * ey + ez * ez <= a.connect2 && (near >> __float_as_int(o.w) & 1)) l |= 1ull << q;
+                }
+                link[k] = l;
+            }
+            __syncwarp();
+            bool whole = true;
+            for (int k = lane; k < n; k += 32) {
+                uint64_t c = link[k], done = 1ull << k;
+                while (c != full && c != done) {
+                    const int q = __ffsll((long long)(c & ~done)) - 1;
+                    done |= 1ull << q;
+                    c |= link[q];
+                }
+                whole = whole && c == full;
+                int label = NO_INDEX;
+                for (uint64_t t = c; t; t &= t - 1) label = min(label, node[__ffsll((long long)t) - 1]);
+                cb.label[node[k]] = label;
+            }
+            whole = __all_sync(0xffffffffu, whole);
+            if (lane == 0) cl_common(cb, a.slots)[slot] = whole ? cb.label[node[0]] : -1;
+            __syncwarp();
+        }
+    }
+}
+
+// Pass 7: the voxels, in brick order, joined with every neighbour of another brick numbered above theirs. Two bricks of one
+// component each need a single pair that connects: the walk notes one, and the pairs of a CTA's bricks are then joined
+// side by side, a thread each -- a join is a chain of dependent loads, and made where a lane meets its pair it holds up the
+// other 31. On 0.3M nodes of a scanned floor counting, writing, scanning and joining edge lists took 2.0 ms and
+// joining each pair when met 0.65 ms.
+__global__ void __launch_bounds__(BRICK_CTA) k_cl_join(ClArgs a, lw_cluster_buf cb) {
+    __shared__ BrickRows rows;
+    __shared__ int32_t common[BRICK_ROWS][27];
+    __shared__ int32_t met[BRICK_ROWS][27];
+    const int m = *cb.m;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int R = a.reach;
-    for (int64_t j0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); j0 < m;
-         j0 += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t j0 = (int64_t)blockIdx.x * 32; j0 < m; j0 += (int64_t)gridDim.x * 32) {
         const int64_t v = j0 + lane;
         const bool live = v < m;
         const int slot = live ? cl_brick(cb)[v] : -1;
         float px = 0.f, py = 0.f, pz = 0.f;
-        int root = 0;
+        int me = 0;
         if (live) {
             px = cb.st_lo[3 * v];
             py = cb.st_lo[3 * v + 1];
             pz = cb.st_lo[3 * v + 2];
-            root = cb.edge_off[v];
+            me = cb.edge_off[v];
         }
-        brick_rows(cb.keys, cl_bases(cb, a.slots), a.mask, [&](int s) { return cl_masks(cb)[s]; }, slot, rows, [&](int row) {
-            const int own = rows.base[row][13];
-            const int bit = nth_bit(rows.mask[row][13], (int)v - own);
+        brick_rows(
+            cb.keys, cl_bases(cb, a.slots), a.mask,
+            [&](int s, int r, int c, int lead) {
+                const int l = cl_common(cb, a.slots)[s];
+                common[r][c] = l;
+                met[r][c] = -1;
+                // numbered below, or both of one component that is the same already: nothing to join
+                if (c != 13) {
+                    if (cl_bases(cb, a.slots)[s] < cl_bases(cb, a.slots)[lead]) return (uint64_t)0;
+                    const int o = cl_common(cb, a.slots)[lead];
+                    if (l >= 0 && o >= 0 && __ldcg(cb.label + l) == __ldcg(cb.label + o)) return (uint64_t)0;
+                }
+                return cl_masks(cb)[s];
+            },
+            slot, rows,
+            [&](int row) {
+                const int bit = nth_bit(rows.mask[row][13], (int)v - rows.base[row][13]);
+                const bool own_one = common[row][13] >= 0;
 #pragma unroll 1
-            for (int c = 0; c < 27; ++c) {
-                const uint64_t all = rows.mask[row][c];
-                const int base = rows.base[row][c];
-                if (base < own || all == 0) continue;
-                uint64_t near = all & brick_window(bit, c % 3 - 1, c / 3 % 3 - 1, c / 9 - 1, R);
-                if (c == 13) near = bit < 63 ? near >> (bit + 1) << (bit + 1) : 0;
-                while (near) {
-                    const int b = __ffsll((long long)near) - 1;
-                    near &= near - 1;
-                    const int64_t k = base + popc64(all & ((1ull << b) - 1));
-                    const float ex = cb.st_lo[3 * k] - px, ey = cb.st_lo[3 * k + 1] - py, ez = cb.st_lo[3 * k + 2] - pz;
-                    if (!(ex * ex + ey * ey + ez * ez <= a.connect2)) continue;
-                    int y = cb.edge_off[k];
-                    for (int it = 0; it < UF_SPINS; ++it) {
-                        if (*(volatile int*)(cb.label + y) == root) break;  // joined already
-                        root = uf_find(cb.label, root);
-                        y = uf_find(cb.label, y);
-                        if (root == y) break;
-                        const int hi = max(root, y), lo = min(root, y);
-                        if (atomicCAS(cb.label + hi, hi, lo) == hi) {
-                            root = lo;
+                for (int c = warp; c < 27; c += BRICK_WARPS) {
+                    const uint64_t all = rows.mask[row][c];
+                    if (all == 0 || c == 13) continue;
+                    uint64_t near = all & brick_window(bit, c % 3 - 1, c / 3 % 3 - 1, c / 9 - 1, R);
+                    const int base = rows.base[row][c];
+                    const bool one = own_one && common[row][c] >= 0;
+                    while (near) {
+                        if (one && *(volatile int32_t*)&met[row][c] >= 0) break;
+                        const int b = __ffsll((long long)near) - 1;
+                        near &= near - 1;
+                        const int64_t k = base + popc64(all & ((1ull << b) - 1));
+                        const float ex = cb.st_lo[3 * k] - px, ey = cb.st_lo[3 * k + 1] - py,
+                                    ez = cb.st_lo[3 * k + 2] - pz;
+                        if (!(ex * ex + ey * ey + ez * ez <= a.connect2)) continue;
+                        if (one) {
+                            *(volatile int32_t*)&met[row][c] = 1;
                             break;
                         }
-                        if (it == UF_SPINS - 1) atomicExch(cb.err, 1);
+                        uf_join(cb, me, cb.edge_off[k]);
                     }
                 }
-            }
-        });
+            },
+            [&](int r, int c) {
+                if (met[r][c] >= 0) uf_join(cb, common[r][13], common[r][c]);
+            });
     }
 }
 
 __global__ void k_cl_uf_flatten(lw_cluster_buf cb) {
     const int m = *cb.m;
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
-        cb.label[j] = uf_find(cb.label, j);
+        const int r = uf_find(cb.label, j);
+        if (r < 0) atomicExch(cb.err, 1);
+        cb.label[j] = max(r, 0);
 #pragma unroll
         for (int d = 0; d < 3; ++d) cb.st_lo[3 * (int64_t)j + d] = cb.st_hi[3 * (int64_t)j + d] = cb.v_xyz[3 * (int64_t)j + d];
     }
@@ -547,14 +647,16 @@ int lw_cluster(const float* xyz, int32_t xyz_stride, const int32_t* gnd, int32_t
     k_cl_node_count<<<nt, CTILE, 0, s>>>(n_dev, n_ub, *cb);
     k_cl_node_scatter<<<nt, CTILE, 0, s>>>(n_dev, n_ub, *cb);
     // at most one node per point
-    k_cl_join<<<blocks_for(n_ub, CL_THREADS, 16 * sms), CL_THREADS, 0, s>>>(a, *cb);
+    const int gridj = blocks_for(n_ub, 32, 64 * sms);
+    k_cl_brick<<<blocks_for(n_ub, 32 * CL_WARPS, 64 * sms), 32 * CL_WARPS, 0, s>>>(a, *cb);
+    k_cl_join<<<gridj, BRICK_CTA, 0, s>>>(a, *cb);
     k_cl_uf_flatten<<<grid, 256, 0, s>>>(*cb);
     k_cl_stats<<<blocks_for((n_ub + CL_RUN - 1) / CL_RUN, 128, 16 * sms), 128, 0, s>>>(*cb);
     k_cl_flag<<<nt, CTILE, 0, s>>>(*cb, a);
     k_cl_compact<<<nt, CTILE, 0, s>>>(*cb, a);
     k_cl_gather<<<grid, 256, 0, s>>>(n_dev, n_ub, *cb, out_cid);
     LW_LAUNCHED("lw_cluster");
-    count_launches(12);
+    count_launches(13);
     return LW_OK;
 }
 
