@@ -83,7 +83,8 @@ struct BrickRows {
 // a scene's voxels alone leave too few warps in flight to hide the walk's loads.
 // mask_of(s, r, c, lead) is the mask of the brick in slot s of the hash (keys, base, hash_mask), found for rows[r][c]
 // around the brick in slot lead.
-// after(r, c): run for each of the looked-up bricks once the lanes are done with them.
+// after(r, c, found): called by every thread once the lanes are done with the bricks looked up, found where the thread's own
+// lookup (r, c) met a brick.
 struct NoAfter {};
 template <class MaskOf, class Run, class After>
 __device__ __forceinline__ void brick_rows(const int64_t* keys, const int32_t* base, int hash_mask, const MaskOf& mask_of,
@@ -117,7 +118,7 @@ __device__ __forceinline__ void brick_rows(const int64_t* keys, const int32_t* b
         if (slot >= 0 && mine >= r0 && mine < r0 + here) run(mine - r0);
         __syncthreads();
         if constexpr (!std::is_same<After, NoAfter>::value) {
-            if (s >= 0) after(r, c);
+            after(r, c, s >= 0);
             __syncthreads();  // after() may read what other threads' lookups left: not before all are done with it
         }
     }

@@ -263,14 +263,16 @@ __global__ void k_cl_node_scatter(const int* n_dev, int64_t n_ub, lw_cluster_buf
 
 constexpr int UF_HOPS = 1 << 20;
 
-// The root of x, or -1 after UF_HOPS hops.
+// The root of x, or -1 after UF_HOPS hops. HALVE shortens the path on the way (not while labels are being put at their
+// roots: a late shortening would put one back).
+template <bool HALVE = true>
 __device__ __forceinline__ int uf_find(int* parent, int x) {
     for (int it = 0; it < UF_HOPS; ++it) {
         // through L2: another SM's hook must be seen, or a lost CAS would be retried on the same stale root
         int p = __ldcg(parent + x);
         if (p == x) return x;
         int gp = __ldcg(parent + p);
-        if (gp != p) __stcg(parent + x, gp);  // path halving: x is no root, and any ancestor will do as its parent
+        if (HALVE && gp != p) __stcg(parent + x, gp);  // x is no root, and any ancestor will do as its parent
         x = p;
     }
     return -1;
@@ -370,6 +372,7 @@ __global__ void __launch_bounds__(BRICK_CTA) k_cl_join(ClArgs a, lw_cluster_buf 
     __shared__ BrickRows rows;
     __shared__ int32_t common[BRICK_ROWS][27];
     __shared__ int32_t met[BRICK_ROWS][27];
+    __shared__ int32_t low[BRICK_ROWS];
     const int m = *cb.m;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int R = a.reach;
@@ -426,8 +429,26 @@ __global__ void __launch_bounds__(BRICK_CTA) k_cl_join(ClArgs a, lw_cluster_buf 
                     }
                 }
             },
-            [&](int r, int c) {
-                if (met[r][c] >= 0) uf_join(cb, common[r][13], common[r][c]);
+            [&](int r, int c, bool found) {
+                // a brick's own root and those of the bricks it met all go under the smallest, each hook on a word of its own;
+                // where another CTA hooked one of them meanwhile all go round again (the smallest must not be lost sight of)
+                const bool in = found && common[r][13] >= 0 && (c == 13 || met[r][c] >= 0);
+                int x = in ? common[r][c] : 0;
+                for (int it = 0; it < UF_HOPS; ++it) {
+                    if (threadIdx.x < BRICK_ROWS) low[threadIdx.x] = NO_INDEX;
+                    __syncthreads();
+                    if (in) {
+                        x = uf_find(cb.label, x);
+                        if (x >= 0)
+                            atomicMin(&low[r], x);
+                        else
+                            atomicExch(cb.err, 1);
+                    }
+                    __syncthreads();
+                    const bool open = in && x >= 0 && x != low[r] && atomicCAS(cb.label + x, x, low[r]) != x;
+                    if (x < 0) x = 0;
+                    if (!__syncthreads_or(open)) break;
+                }
             });
     }
 }
@@ -435,7 +456,7 @@ __global__ void __launch_bounds__(BRICK_CTA) k_cl_join(ClArgs a, lw_cluster_buf 
 __global__ void k_cl_uf_flatten(lw_cluster_buf cb) {
     const int m = *cb.m;
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
-        const int r = uf_find(cb.label, j);
+        const int r = uf_find<false>(cb.label, j);
         if (r < 0) atomicExch(cb.err, 1);
         cb.label[j] = max(r, 0);
 #pragma unroll
