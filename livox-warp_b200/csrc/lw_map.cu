@@ -770,15 +770,18 @@ __device__ int settled_near(int ix, int iy, int iz, const lw_view& v, const lw_m
     return 0;
 }
 
-__device__ __forceinline__ bool classify_flag_key(const lw_map& map, int64_t s, int64_t key, const lw_view& v,
-                                                  int min_count, float& wx, float& wy, float& wz) {
-    if (key == EMPTY_KEY) return false;
+// Whether slot s is drawn (gpu.py:699-747). The centroid (three float64 divides and a 32-byte read) is formed only for the
+// crop box, which is off in most views.
+__device__ __forceinline__ bool classify_flag(const lw_map& map, int64_t s, const lw_view& v, int min_count) {
     int c = map.cnt[s];
-    if (c < min_count) return false;
-    float last = map.last[s];
-    if (v.persist > 0.0f && v.now - last > v.persist) return false;
-    if (v.carve_on != 0 && ghost(c, map.miss[s], last, v) != 0) return false;
-    if (c <= 0) return false;
+    if (c < min_count || c <= 0) return false;
+    if (v.persist > 0.0f || v.carve_on != 0) {
+        float last = map.last[s];
+        if (v.persist > 0.0f && v.now - last > v.persist) return false;
+        if (v.carve_on != 0 && ghost(c, map.miss[s], last, v) != 0) return false;
+    }
+    if (v.crop_on == 0) return true;
+    float wx, wy, wz;
     centroid(map, (int)s, wx, wy, wz);
     return in_crop(wx, wy, wz, v) != 0;
 }
@@ -812,8 +815,7 @@ __global__ void __launch_bounds__(CL_THREADS) k_classify_count(lw_map map, lw_vi
     int c = 0;
 #pragma unroll
     for (int u = 0; u < CL_PER; ++u) {
-        float wx, wy, wz;
-        if (k[u] != EMPTY_KEY && classify_flag_key(map, s0 + u, k[u], v, min_count, wx, wy, wz)) ++c;
+        if (k[u] != EMPTY_KEY && classify_flag(map, s0 + u, v, min_count)) ++c;
     }
     int tot;
     block_excl(c, sm, &tot);
@@ -868,38 +870,39 @@ __global__ void __launch_bounds__(CL_THREADS) k_classify_scatter(lw_map map, lw_
                                                                  uint32_t* __restrict__ out_attr,
                                                                  float* __restrict__ out_t, int* __restrict__ out_dyn) {
     __shared__ int sm[33];
-    const int64_t s0 = (int64_t)blockIdx.x * CL_TILE + (int64_t)threadIdx.x * CL_PER;
+    __shared__ uint16_t drawn[CL_TILE];  // the tile's drawn slots, in order
+    const int64_t t0 = (int64_t)blockIdx.x * CL_TILE, s0 = t0 + (int64_t)threadIdx.x * CL_PER;
     int64_t k[CL_PER];
     load_keys(map, s0, k);
-    float wx[CL_PER], wy[CL_PER], wz[CL_PER];
     unsigned flags = 0;
 #pragma unroll
     for (int u = 0; u < CL_PER; ++u)
-        if (k[u] != EMPTY_KEY && classify_flag_key(map, s0 + u, k[u], v, min_count, wx[u], wy[u], wz[u]))
-            flags |= 1u << u;
+        if (k[u] != EMPTY_KEY && classify_flag(map, s0 + u, v, min_count)) flags |= 1u << u;
     int tot;
-    int j = tiles[blockIdx.x] + block_excl(__popc(flags), sm, &tot);
-#pragma unroll
-    for (int u = 0; u < CL_PER; ++u) {
-        if (!((flags >> u) & 1u)) continue;
-        const int64_t s = s0 + u;
+    int at = block_excl(__popc(flags), sm, &tot);
+    for (unsigned f = flags; f; f &= f - 1) drawn[at++] = (uint16_t)(threadIdx.x * CL_PER + __ffs(f) - 1);
+    __syncthreads();
+    const int first = tiles[blockIdx.x];
+    // a drawn slot per thread: with the slots' own threads forming them, one lane in eight works at a usual load
+    for (int i = threadIdx.x; i < tot; i += CL_THREADS) {
+        const int64_t s = t0 + drawn[i], j = (int64_t)first + i;
+        float wx, wy, wz;
+        centroid(map, (int)s, wx, wy, wz);
         int c = map.cnt[s];
         int n = c < LW_MAP_CAP ? c : LW_MAP_CAP;
         int refl = (int)((double)map.acc[4 * s + 3] / (double)n + 0.5);
         if (refl > 255) refl = 255;
-        out_xyz[3 * (int64_t)j + 0] = wx[u];
-        out_xyz[3 * (int64_t)j + 1] = wy[u];
-        out_xyz[3 * (int64_t)j + 2] = wz[u];
+        out_xyz[3 * j + 0] = wx;
+        out_xyz[3 * j + 1] = wy;
+        out_xyz[3 * j + 2] = wz;
         out_attr[j] = (uint32_t)refl;  // mean reflectivity only: tag, return and device mean nothing for a voxel
         out_t[j] = map.last[s];
         int dyn = 0;
         if (transient(c, map.miss[s], v) != 0)
             dyn = 1;
-        else if (settled_near(ifloor(wx[u] * v.inv_voxel), ifloor(wy[u] * v.inv_voxel), ifloor(wz[u] * v.inv_voxel), v,
-                              map) == 0)
+        else if (settled_near(ifloor(wx * v.inv_voxel), ifloor(wy * v.inv_voxel), ifloor(wz * v.inv_voxel), v, map) == 0)
             dyn = 1;
         out_dyn[j] = dyn;
-        ++j;
     }
 }
 
