@@ -130,12 +130,11 @@ __global__ void k_nb_mean(lw_nbr_buf nb, int64_t vcap) {
 // The voxels in brick order (gpu.py:829-876): every voxel whose centroid lies within the radius adds its points' weight,
 // weighted offset and weighted outer product in fixed point; from them the count, and with want_normals the
 // covariance's smallest-eigenvalue vector turned toward the sensor and the curvature (smallest eigenvalue / trace).
-// Bound by the issue of the candidates' arithmetic at a third of the lanes (each lane has its own window). On 0.5M voxels of a
-// scanned floor a warp per voxel probing 343 offsets, its lane 0 decomposing alone, took 3.15 ms.
-// SMALL (a radius below 2 m, so offset products stay below 2^42 units): sums from rounded bits (rint_split) instead of
-// float -> int64 conversions.
-template <bool SMALL>
-__global__ void __launch_bounds__(BRICK_CTA) k_nb_voxel(NbArgs a, lw_nbr_buf nb) {
+// Bound by latency and issue of the candidates' walk at a third of the lanes (each lane has its own window), so by the
+// warps in flight: 64 registers (8 CTAs per SM) 0.54 ms on 0.5M voxels of a scanned floor, 92 registers 0.66 ms; queueing a
+// lane's candidates and working the queues off on full warps was slower (0.72 ms), as were sums without float -> int64
+// conversions, which take more registers. A warp per voxel probing 343 offsets, its lane 0 decomposing alone, took 3.15 ms.
+__global__ void __launch_bounds__(BRICK_CTA, 8) k_nb_voxel(NbArgs a, lw_nbr_buf nb) {
     __shared__ BrickRows rows;
     __shared__ long long part[BRICK_WARPS - 1][10][32];
     const int64_t m = nb_voxels(nb, a.vcap);
@@ -144,7 +143,7 @@ __global__ void __launch_bounds__(BRICK_CTA) k_nb_voxel(NbArgs a, lw_nbr_buf nb)
         const int64_t j = j0 + lane;
         const int slot = j < m ? __float_as_int(nb.v_cnt[j]) : -1;
         const float4 P = j < m ? *reinterpret_cast<const float4*>(nb.acc + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
-        long long W = 0, s1[3] = {0, 0, 0}, s2[6] = {0, 0, 0, 0, 0, 0}, lo[6] = {0, 0, 0, 0, 0, 0};
+        long long W = 0, s1[3] = {0, 0, 0}, s2[6] = {0, 0, 0, 0, 0, 0};
         brick_rows(nb.keys, nb.v_w, a.mask, [&](int s, int, int, int) { return nb_mask(nb, s); }, slot, rows, [&](int row) {
             const int bit = nth_bit(rows.mask[row][13], (int)j - rows.base[row][13]);
 #pragma unroll 1
@@ -163,39 +162,18 @@ __global__ void __launch_bounds__(BRICK_CTA) k_nb_voxel(NbArgs a, lw_nbr_buf nb)
                     const int w = __float_as_int(Q.w);
                     const float FD = (float)NB_FIX_D, FDD = (float)NB_FIX_DD;
                     W += w;
-                    if constexpr (SMALL) {
-                        const float fx = ex * FD, fy = ey * FD, fz = ez * FD;  // exact: FD^2 = FDD
-                        s1[0] += (long long)w * rint_bits(fx);
-                        s1[1] += (long long)w * rint_bits(fy);
-                        s1[2] += (long long)w * rint_bits(fz);
-                        const float v[6] = {fx * fx, fx * fy, fx * fz, fy * fy, fy * fz, fz * fz};
-#pragma unroll
-                        for (int t = 0; t < 6; ++t) {
-                            int h, l;
-                            rint_split(v[t], h, l);
-                            s2[t] += (long long)w * h;
-                            lo[t] += (long long)w * l;
-                        }
-                    } else {
-                        s1[0] += (long long)w * __float2int_rn(ex * FD);  // at most 4 m: 2^22 units
-                        s1[1] += (long long)w * __float2int_rn(ey * FD);
-                        s1[2] += (long long)w * __float2int_rn(ez * FD);
-                        s2[0] += w * to_fix(ex * ex, FDD);
-                        s2[1] += w * to_fix(ex * ey, FDD);
-                        s2[2] += w * to_fix(ex * ez, FDD);
-                        s2[3] += w * to_fix(ey * ey, FDD);
-                        s2[4] += w * to_fix(ey * ez, FDD);
-                        s2[5] += w * to_fix(ez * ez, FDD);
-                    }
+                    s1[0] += (long long)w * __float2int_rn(ex * FD);  // at most 4 m: 2^22 units
+                    s1[1] += (long long)w * __float2int_rn(ey * FD);
+                    s1[2] += (long long)w * __float2int_rn(ez * FD);
+                    s2[0] += w * to_fix(ex * ex, FDD);
+                    s2[1] += w * to_fix(ex * ey, FDD);
+                    s2[2] += w * to_fix(ex * ez, FDD);
+                    s2[3] += w * to_fix(ey * ey, FDD);
+                    s2[4] += w * to_fix(ey * ez, FDD);
+                    s2[5] += w * to_fix(ez * ez, FDD);
                 }
             }
         }, NoAfter());
-        if constexpr (SMALL) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) s1[c] -= W * RINT_BITS;
-#pragma unroll
-            for (int c = 0; c < 6; ++c) s2[c] = ((s2[c] - W * RINT_BITS) << 20) + (lo[c] - W * RINT_BITS);
-        }
         if (warp > 0) {
             long long(*p)[32] = part[warp - 1];
             p[0][lane] = W;
@@ -347,11 +325,7 @@ int lw_neighborhoods(const float* xyz, int32_t xyz_stride, const int32_t* n_dev,
         k_nb_sum<3><<<grid, 256, 0, s>>>(xyz, n_dev, n_ub, a, b);
     // at most one voxel per point
     k_nb_mean<<<grid, 256, 0, s>>>(b, a.vcap);
-    const int gridv = blocks_for(n_ub, 32, 64 * sms);
-    if (radius < 1.99f)
-        k_nb_voxel<true><<<gridv, BRICK_CTA, 0, s>>>(a, b);
-    else
-        k_nb_voxel<false><<<gridv, BRICK_CTA, 0, s>>>(a, b);
+    k_nb_voxel<<<blocks_for(n_ub, 32, 64 * sms), BRICK_CTA, 0, s>>>(a, b);
     k_nb_gather<<<grid, 256, 0, s>>>(n_dev, n_ub, a.want_normals, b, out_cnt, out_nrm, out_curv);
     LW_LAUNCHED("lw_neighborhoods");
     count_launches(7);
