@@ -652,16 +652,16 @@ int lw_net_forward(const lw_initnet* net, const float* sets, int32_t n, float* p
 
 /* Scratch of the backward pass for up to n_cap samples (sizes in floats unless stated). */
 typedef struct lw_net_scratch {
-    float* dz3;       /* [2n*256] */
-    uint16_t* h2g;    /* [2n*256*128] bf16: layer-2 activations of each channel's argmax point */
-    float* d2t;       /* [128][2n*256] */
-    float* h1t;       /* [65][2n*256]: layer-1 activations, then a row of ones */
-    float* d1t;       /* [64][2n*256] */
-    float* xt;        /* [4][2n*256]: the scaled inputs, then a row of ones */
+    float* dz3;       /* [2n*256] gradient of each channel's argmax point */
+    uint16_t* h2g;    /* [2n*256*128] bf16: layer-2 activations of each set's distinct argmax points */
+    float* d2t;       /* [128][2n*256] CTAs' sums of the layer-1 and layer-2 gradients */
+    float* h1t;       /* [65][2n*256] not used */
+    float* d1t;       /* [64][2n*256] not used */
+    float* xt;        /* [4][2n*256] place of each channel's point among its set's (int32) */
     float* dzh;       /* [n][128] */
     float* dout;      /* [n][6] */
     float* dpool;     /* [2n][256] */
-    float* part;      /* [64 * 8448] split-K partials */
+    float* part;      /* [64 * 8448] not used */
     float* loss;      /* [n] per-sample loss */
     int32_t n_cap;
     int32_t pad_;

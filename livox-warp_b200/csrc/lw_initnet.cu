@@ -2,7 +2,7 @@
 // points, 512 -> 128 -> 6) on sm_100a. It has no counterpart in the reference, whose odometry predicts the next
 // pose with constant velocity (odom.py:591-592); that prediction stays the network's input frame and fallback.
 //
-// Forward: one CTA of 128 threads per point set, eight 128-point tiles in turn. Layer 1 (K = 3) runs on the CUDA
+// Forward: persistent CTAs of two groups of 128 threads, a point set per group at a time, eight 128-point tiles in turn. Layer 1 (K = 3) runs on the CUDA
 // cores; layers 2 and 3 are tcgen05.mma (kind::f16, bf16 operands from shared memory in the canonical K-major
 // layout without swizzle, float32 accumulators in TMEM). Layer 2 puts the points on M (D = H1 W2^T, one TMEM
 // lane per point), so each thread converts its own point's 128 channels back to bf16 for layer 3. Layer 3 puts
@@ -28,11 +28,12 @@ constexpr long long NET_SPINS = 1LL << 24;
 // forward shared memory (bytes)
 constexpr uint32_t SM_W2 = 0;                       // [128 out][64 in] bf16, canonical K-major
 constexpr uint32_t SM_W3 = SM_W2 + C2 * C1 * 2;     // [256 out][128 in]
-constexpr uint32_t SM_H1 = SM_W3 + C3 * C2 * 2;     // [128 points][64]
-constexpr uint32_t SM_H2 = SM_H1 + NET_T * C1 * 2;  // [128 points][128]
-constexpr uint32_t SM_PAR = SM_H2 + NET_T * C2 * 2; // W1 [192], b1 [64], b2 [128], b3 [256] float
+constexpr int NET_G = 2;                             // groups of NET_T threads, each with its own H1, H2 and TMEM columns
+constexpr uint32_t SM_H1 = SM_W3 + C3 * C2 * 2;     // per group [128 points][64]
+constexpr uint32_t SM_H2 = SM_H1 + NET_G * NET_T * C1 * 2;  // per group [128 points][128]
+constexpr uint32_t SM_PAR = SM_H2 + NET_G * NET_T * C2 * 2; // W1 [192], b1 [64], b2 [128], b3 [256] float
 constexpr uint32_t SM_TOTAL = SM_PAR + (192 + 64 + 128 + 256) * 4;
-constexpr uint32_t TMEM_COLS = 256;
+constexpr uint32_t TMEM_COLS = 256;  // per group
 
 __device__ __forceinline__ float bf(uint16_t v) { return __uint_as_float((uint32_t)v << 16); }
 __device__ __forceinline__ uint16_t to_bf(float x) {
@@ -116,22 +117,39 @@ __device__ __forceinline__ void load_canonical(const uint16_t* __restrict__ g, u
     }
 }
 
-__global__ void __launch_bounds__(NET_T, 1)
-    k_net_mlp(const uint16_t* __restrict__ w, float in_scale, const float4* __restrict__ sets,
+// Barriers of one group of NET_T threads (named barrier 1 + group).
+__device__ __forceinline__ void group_sync(int group) {
+    asm volatile("barrier.cta.sync %0, %1;" ::"r"(1 + group), "r"(NET_T) : "memory");
+}
+__device__ __forceinline__ bool group_or(int group, bool v) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\tbarrier.cta.red.or.pred q, %1, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(r)
+        : "r"(1 + group), "r"(NET_T), "r"((uint32_t)v)
+        : "memory");
+    return r != 0;
+}
+
+// Bound by the chain of a tile -- layer 1, MMA, epilogue, MMA, epilogue -- on few warps: one group alone leaves the SM idle in
+// every step of it, a second group fills in (its weights are the CTA's, 80 KB of shared memory). Batch 256: 182 us with one
+// group per CTA and a CTA per set.
+__global__ void __launch_bounds__(NET_G * NET_T, 1)
+    k_net_mlp(const uint16_t* __restrict__ w, float in_scale, const float4* __restrict__ sets, int n_sets,
               float* __restrict__ pooled, int32_t* __restrict__ argmax, int32_t* err) {
     extern __shared__ __align__(128) uint8_t sm[];
-    __shared__ __align__(8) uint64_t bar;
+    __shared__ __align__(8) uint64_t bars[NET_G];
     __shared__ uint32_t tmem_slot;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int set = blockIdx.x;
-    const uint32_t bar_a = smem_u32(&bar);
+    const int group = threadIdx.x / NET_T, tid = threadIdx.x % NET_T, warp = tid >> 5;
+    const uint32_t bar_a = smem_u32(&bars[group]);
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_a) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) {
+    if (threadIdx.x < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                     "r"(TMEM_COLS)
+                     "r"(NET_G * TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -143,150 +161,150 @@ __global__ void __launch_bounds__(NET_T, 1)
     float* sb1 = par + 192;
     float* sb2 = par + 256;
     float* sb3 = par + 384;
-    for (int i = tid; i < 192; i += NET_T) sW1[i] = bf(w[LW_NET_OFF_W1 + i]);
-    for (int i = tid; i < C1; i += NET_T) sb1[i] = bf(w[LW_NET_OFF_B1 + i]);
-    for (int i = tid; i < C2; i += NET_T) sb2[i] = bf(w[LW_NET_OFF_B2 + i]);
-    for (int i = tid; i < C3; i += NET_T) sb3[i] = bf(w[LW_NET_OFF_B3 + i]);
+    for (int i = threadIdx.x; i < 192; i += NET_G * NET_T) sW1[i] = bf(w[LW_NET_OFF_W1 + i]);
+    for (int i = threadIdx.x; i < C1; i += NET_G * NET_T) sb1[i] = bf(w[LW_NET_OFF_B1 + i]);
+    for (int i = threadIdx.x; i < C2; i += NET_G * NET_T) sb2[i] = bf(w[LW_NET_OFF_B2 + i]);
+    for (int i = threadIdx.x; i < C3; i += NET_G * NET_T) sb3[i] = bf(w[LW_NET_OFF_B3 + i]);
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tbase = tmem_slot;
+    const uint32_t tbase = tmem_slot + group * TMEM_COLS;
     const uint32_t lane_base = tbase + ((uint32_t)(warp * 32) << 16);
+    uint8_t* h1 = sm + SM_H1 + group * NET_T * C1 * 2;
+    uint8_t* h2 = sm + SM_H2 + group * NET_T * C2 * 2;
     const uint32_t s_w2 = smem_u32(sm + SM_W2), s_w3 = smem_u32(sm + SM_W3);
-    const uint32_t s_h1 = smem_u32(sm + SM_H1), s_h2 = smem_u32(sm + SM_H2);
-    float mx0 = -1.0f, mx1 = -1.0f;
-    int ag0 = -1, ag1 = -1;
+    const uint32_t s_h1 = smem_u32(h1), s_h2 = smem_u32(h2);
     uint32_t phase = 0;
-    int failed = 0;
-    const float4* pts = sets + (size_t)set * NP;
-    for (int tile = 0; tile < NP / NET_T && !failed; ++tile) {
-        // layer 1 on the CUDA cores: this thread's point, 64 channels, bf16 into H1's row
-        {
-            float4 p = __ldg(pts + tile * NET_T + tid);
-            const float x = p.x * in_scale, y = p.y * in_scale, z = p.z * in_scale;
+    bool failed = false;  // a wait ran out: this group's remaining sets read as zero
+    for (int set = blockIdx.x + group * gridDim.x; set < n_sets; set += NET_G * gridDim.x) {
+        float mx0 = -1.0f, mx1 = -1.0f;
+        int ag0 = -1, ag1 = -1;
+        const float4* pts = sets + (size_t)set * NP;
+        for (int tile = 0; tile < NP / NET_T && !failed; ++tile) {
+            // layer 1 on the CUDA cores: this thread's point, 64 channels, bf16 into H1's row
+            {
+                float4 p = __ldg(pts + tile * NET_T + tid);
+                const float x = p.x * in_scale, y = p.y * in_scale, z = p.z * in_scale;
 #pragma unroll
-            for (int c8 = 0; c8 < C1 / 8; ++c8) {
-                uint32_t pk[4];
+                for (int c8 = 0; c8 < C1 / 8; ++c8) {
+                    uint32_t pk[4];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    float h[2];
+                    for (int q = 0; q < 4; ++q) {
+                        float h[2];
 #pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const int j = c8 * 8 + q * 2 + e;
-                        float a = sb1[j];
-                        a = fmaf(sW1[3 * j + 0], x, a);
-                        a = fmaf(sW1[3 * j + 1], y, a);
-                        a = fmaf(sW1[3 * j + 2], z, a);
-                        h[e] = fmaxf(a, 0.0f);
+                        for (int e = 0; e < 2; ++e) {
+                            const int j = c8 * 8 + q * 2 + e;
+                            float a = sb1[j];
+                            a = fmaf(sW1[3 * j + 0], x, a);
+                            a = fmaf(sW1[3 * j + 1], y, a);
+                            a = fmaf(sW1[3 * j + 2], z, a);
+                            h[e] = fmaxf(a, 0.0f);
+                        }
+                        pk[q] = (uint32_t)to_bf(h[0]) | ((uint32_t)to_bf(h[1]) << 16);
                     }
-                    pk[q] = (uint32_t)to_bf(h[0]) | ((uint32_t)to_bf(h[1]) << 16);
+                    *reinterpret_cast<uint4*>(h1 + kofs(tid, c8 * 8, C1)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                 }
-                *reinterpret_cast<uint4*>(sm + SM_H1 + kofs(tid, c8 * 8, C1)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
             }
-        }
-        fence_async_smem();
-        __syncthreads();
-        // layer 2: D[point][out] = H1 W2^T, TMEM columns 0..127
-        if (tid == 0) {
-            tc_fence_after();
+            fence_async_smem();
+            group_sync(group);
+            // layer 2: D[point][out] = H1 W2^T, TMEM columns 0..127
+            if (tid == 0) {
+                tc_fence_after();
 #pragma unroll
-            for (int s = 0; s < C1 / 16; ++s)
-                umma(tbase, umma_desc(s_h1 + s * 256, 128, (C1 / 8) * 128), umma_desc(s_w2 + s * 256, 128, (C1 / 8) * 128),
-                     umma_idesc(C2), s > 0);
-            umma_commit(bar_a);
-        }
-        if (!mbar_wait(bar_a, phase)) failed = 1;
-        phase ^= 1;
-        if (__syncthreads_or(failed)) {
-            failed = 1;
-            break;
-        }
-        tc_fence_after();
-        // epilogue 2: this thread's point (TMEM lane), 128 channels + bias, ReLU, bf16 into H2's row
-#pragma unroll 1
-        for (int c = 0; c < C2 / 32; ++c) {
-            float v[32];
-            tmem_ld32(lane_base + c * 32, v);
-#pragma unroll
-            for (int c8 = 0; c8 < 4; ++c8) {
-                uint32_t pk[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int j0 = c * 32 + c8 * 8 + q * 2;
-                    const float h0 = fmaxf(v[c8 * 8 + q * 2] + sb2[j0], 0.0f);
-                    const float h1 = fmaxf(v[c8 * 8 + q * 2 + 1] + sb2[j0 + 1], 0.0f);
-                    pk[q] = (uint32_t)to_bf(h0) | ((uint32_t)to_bf(h1) << 16);
-                }
-                *reinterpret_cast<uint4*>(sm + SM_H2 + kofs(tid, c * 32 + c8 * 8, C2)) =
-                    make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                for (int s = 0; s < C1 / 16; ++s)
+                    umma(tbase, umma_desc(s_h1 + s * 256, 128, (C1 / 8) * 128),
+                         umma_desc(s_w2 + s * 256, 128, (C1 / 8) * 128), umma_idesc(C2), s > 0);
+                umma_commit(bar_a);
             }
-        }
-        fence_async_smem();
-        tc_fence_before();
-        __syncthreads();
-        // layer 3: D[channel][point] = W3 H2^T, two halves of 128 channels in TMEM columns 0..255
-        if (tid == 0) {
+            failed = group_or(group, !mbar_wait(bar_a, phase));
+            phase ^= 1;
+            if (failed) break;
             tc_fence_after();
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int s = 0; s < C2 / 16; ++s)
-                    umma(tbase + h * 128, umma_desc(s_w3 + h * 16 * (C2 / 8) * 128 + s * 256, 128, (C2 / 8) * 128),
-                         umma_desc(s_h2 + s * 256, 128, (C2 / 8) * 128), umma_idesc(NET_T), s > 0);
-            umma_commit(bar_a);
-        }
-        if (!mbar_wait(bar_a, phase)) failed = 1;
-        phase ^= 1;
-        if (__syncthreads_or(failed)) {
-            failed = 1;
-            break;
-        }
-        tc_fence_after();
-        // epilogue 3: this thread's channel (TMEM lane) over the tile's points: bias, ReLU, running max
+            // epilogue 2: this thread's point (TMEM lane), 128 channels + bias, ReLU, bf16 into H2's row
 #pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-            const float b = sb3[h * 128 + tid];
-            float m = h ? mx1 : mx0;
-            int ag = h ? ag1 : ag0;
-#pragma unroll 1
-            for (int c = 0; c < NET_T / 32; ++c) {
+            for (int c = 0; c < C2 / 32; ++c) {
                 float v[32];
-                tmem_ld32(lane_base + h * 128 + c * 32, v);
+                tmem_ld32(lane_base + c * 32, v);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const float zz = fmaxf(v[i] + b, 0.0f);
-                    if (zz > m) {
-                        m = zz;
-                        ag = tile * NET_T + c * 32 + i;
+                for (int c8 = 0; c8 < 4; ++c8) {
+                    uint32_t pk[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int j0 = c * 32 + c8 * 8 + q * 2;
+                        const float a0 = fmaxf(v[c8 * 8 + q * 2] + sb2[j0], 0.0f);
+                        const float a1 = fmaxf(v[c8 * 8 + q * 2 + 1] + sb2[j0 + 1], 0.0f);
+                        pk[q] = (uint32_t)to_bf(a0) | ((uint32_t)to_bf(a1) << 16);
                     }
+                    *reinterpret_cast<uint4*>(h2 + kofs(tid, c * 32 + c8 * 8, C2)) =
+                        make_uint4(pk[0], pk[1], pk[2], pk[3]);
                 }
             }
-            if (h) {
-                mx1 = m;
-                ag1 = ag;
-            } else {
-                mx0 = m;
-                ag0 = ag;
+            fence_async_smem();
+            tc_fence_before();
+            group_sync(group);
+            // layer 3: D[channel][point] = W3 H2^T, two halves of 128 channels in TMEM columns 0..255
+            if (tid == 0) {
+                tc_fence_after();
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int s = 0; s < C2 / 16; ++s)
+                        umma(tbase + h * 128, umma_desc(s_w3 + h * 16 * (C2 / 8) * 128 + s * 256, 128, (C2 / 8) * 128),
+                             umma_desc(s_h2 + s * 256, 128, (C2 / 8) * 128), umma_idesc(NET_T), s > 0);
+                umma_commit(bar_a);
             }
+            failed = group_or(group, !mbar_wait(bar_a, phase));
+            phase ^= 1;
+            if (failed) break;
+            tc_fence_after();
+            // epilogue 3: this thread's channel (TMEM lane) over the tile's points: bias, ReLU, running max
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                const float b = sb3[h * 128 + tid];
+                float m = h ? mx1 : mx0;
+                int ag = h ? ag1 : ag0;
+#pragma unroll 1
+                for (int c = 0; c < NET_T / 32; ++c) {
+                    float v[32];
+                    tmem_ld32(lane_base + h * 128 + c * 32, v);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        const float zz = fmaxf(v[i] + b, 0.0f);
+                        if (zz > m) {
+                            m = zz;
+                            ag = tile * NET_T + c * 32 + i;
+                        }
+                    }
+                }
+                if (h) {
+                    mx1 = m;
+                    ag1 = ag;
+                } else {
+                    mx0 = m;
+                    ag0 = ag;
+                }
+            }
+            tc_fence_before();
+            group_sync(group);
         }
-        tc_fence_before();
-        __syncthreads();
+        if (failed) {
+            if (tid == 0) atomicExch(err, 1);
+            mx0 = mx1 = 0.0f;
+            ag0 = ag1 = -1;
+        }
+        pooled[(size_t)set * C3 + tid] = mx0;
+        pooled[(size_t)set * C3 + 128 + tid] = mx1;
+        argmax[(size_t)set * C3 + tid] = ag0;
+        argmax[(size_t)set * C3 + 128 + tid] = ag1;
     }
-    if (failed) {
-        if (tid == 0) atomicExch(err, 1);
-        mx0 = mx1 = 0.0f;
-        ag0 = ag1 = -1;
-    }
-    pooled[(size_t)set * C3 + tid] = mx0;
-    pooled[(size_t)set * C3 + 128 + tid] = mx1;
-    argmax[(size_t)set * C3 + tid] = ag0;
-    argmax[(size_t)set * C3 + 128 + tid] = ag1;
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) {
+    if (threadIdx.x < 32) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot),
+                     "r"(NET_G * TMEM_COLS)
+                     : "memory");
     }
 }
 
@@ -300,8 +318,18 @@ __global__ void __launch_bounds__(CH) k_net_head(const uint16_t* __restrict__ w,
     for (int k = j; k < 2 * C3; k += CH) x[k] = bfr(pooled[(size_t)s * 2 * C3 + k]);
     __syncthreads();
     float a = bf(w[LW_NET_OFF_BH1 + j]);
-    const uint16_t* row = w + LW_NET_OFF_WH1 + (size_t)j * 2 * C3;
-    for (int k = 0; k < 2 * C3; ++k) a = fmaf(bf(row[k]), x[k], a);
+    // 8 weights a load (a thread's row is 1 KB from its neighbour's: 2-byte loads took 75 us at batch 256)
+    const uint4* row = reinterpret_cast<const uint4*>(w + LW_NET_OFF_WH1 + (size_t)j * 2 * C3);
+#pragma unroll 8
+    for (int k8 = 0; k8 < 2 * C3 / 8; ++k8) {
+        const uint4 q = __ldg(row + k8);
+        const uint32_t u[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            a = fmaf(__uint_as_float(u[e] << 16), x[8 * k8 + 2 * e], a);
+            a = fmaf(__uint_as_float(u[e] & 0xffff0000u), x[8 * k8 + 2 * e + 1], a);
+        }
+    }
     const float h = bfr(fmaxf(a, 0.0f));
     hs[j] = h;
     hid[(size_t)s * CH + j] = h;
@@ -353,130 +381,278 @@ __global__ void __launch_bounds__(CH) k_net_head_bwd(const uint16_t* __restrict_
     }
 }
 
-// One (set, channel): the channel's argmax point gets d(pooled); recompute its layer-1/2 activations and write the
-// rows the weight-gradient reductions read (K index = set * 256 + channel).
-__global__ void __launch_bounds__(C3) k_net_pt_bwd(const uint16_t* __restrict__ w, float in_scale,
-                                                   const float4* __restrict__ sets, const float* __restrict__ pooled,
-                                                   const int32_t* __restrict__ argmax, int n_sets, lw_net_scratch scr) {
-    const int set = blockIdx.x, c = threadIdx.x;
-    const int64_t K = (int64_t)n_sets * C3;
-    const int64_t kk = (int64_t)set * C3 + c;
-    const int p = argmax[kk];
-    const float v = pooled[kk];
-    const float g = (p >= 0 && p < NP && v > 0.0f) ? scr.dpool[kk] : 0.0f;
-    scr.dz3[kk] = g;
-    uint16_t* h2row = scr.h2g + kk * C2;
-    if (g == 0.0f) {
-        for (int j = 0; j < C2; ++j) {
-            h2row[j] = 0;
-            scr.d2t[j * K + kk] = 0.0f;
-        }
-        for (int i = 0; i < C1; ++i) {
-            scr.h1t[i * K + kk] = 0.0f;
-            scr.d1t[i * K + kk] = 0.0f;
-        }
-        scr.h1t[C1 * K + kk] = 0.0f;
-        for (int d = 0; d < 4; ++d) scr.xt[d * K + kk] = 0.0f;
-        return;
-    }
-    const float4 q = __ldg(sets + (size_t)set * NP + p);
-    const float x = q.x * in_scale, y = q.y * in_scale, z = q.z * in_scale;
-    float h1[C1];
-    bool a1[C1];
-#pragma unroll
-    for (int j = 0; j < C1; ++j) {
-        float a = bf(w[LW_NET_OFF_B1 + j]);
-        a = fmaf(bf(w[LW_NET_OFF_W1 + 3 * j + 0]), x, a);
-        a = fmaf(bf(w[LW_NET_OFF_W1 + 3 * j + 1]), y, a);
-        a = fmaf(bf(w[LW_NET_OFF_W1 + 3 * j + 2]), z, a);
-        a1[j] = a > 0.0f;
-        h1[j] = bfr(fmaxf(a, 0.0f));
-        scr.h1t[j * K + kk] = h1[j];
-    }
-    scr.h1t[C1 * K + kk] = 1.0f;
-    scr.xt[0 * K + kk] = x;
-    scr.xt[1 * K + kk] = y;
-    scr.xt[2 * K + kk] = z;
-    scr.xt[3 * K + kk] = 1.0f;
-    float d1[C1];
-#pragma unroll
-    for (int i = 0; i < C1; ++i) d1[i] = 0.0f;
-    const uint16_t* w3row = w + LW_NET_OFF_W3 + (size_t)c * C2;
-    for (int j = 0; j < C2; ++j) {
-        const uint16_t* w2row = w + LW_NET_OFF_W2 + (size_t)j * C1;
-        float a = bf(w[LW_NET_OFF_B2 + j]);
-#pragma unroll
-        for (int i = 0; i < C1; ++i) a = fmaf(bf(w2row[i]), h1[i], a);
-        h2row[j] = to_bf(fmaxf(a, 0.0f));
-        const float d2 = a > 0.0f ? g * bf(w3row[j]) : 0.0f;
-        scr.d2t[j * K + kk] = d2;
-        if (d2 != 0.0f) {
-#pragma unroll
-            for (int i = 0; i < C1; ++i) d1[i] = fmaf(d2, bf(w2row[i]), d1[i]);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < C1; ++i) scr.d1t[i * K + kk] = a1[i] ? d1[i] : 0.0f;
-}
+// Through the max, gradient reaches one point per channel, and the channels of a set share few points: a set's distinct
+// argmax points are gathered (at most 256, typically 60-120), their layer-1 and layer-2 activations recomputed, the
+// channels' gradients summed per point before they go through layer 2 (linear up to the points' own ReLU masks), and the weight
+// gradients of layers 1 and 2 summed in registers over all sets of a CTA -- nothing per (set, channel) but the row of
+// layer 2's output that dW3 needs goes through memory. Bound by the float32 FMAs of three [points x 128 x 64]
+// products per set (8 x 4 and 4 x 4 register tiles). At batch 256 a thread per (set, channel) that wrote every factor
+// out, and dot products over them, took 0.57 + 1.32 ms.
+constexpr int PB_T = 256, PB_P = 64;       // threads; points per tile
+constexpr int PB_W = C1 + 4, PB_D = C2 + 4;  // padded rows of W2 [128][64], H1 [64][64] and D2 [64][128]
+constexpr int PB_PART = C2 * C1 + C2 + 4 * C1;  // a CTA's sums: dW2, db2, (dW1 | db1)
 
-// Split-K partials of C[r][q] = sum_k A[r][k] B[q][k] (rows of length K): chunk `blockIdx.x` of kc columns.
-constexpr int DOT_KC = 32;
-__global__ void __launch_bounds__(256) k_dot_rows(const float* __restrict__ A, int R, const float* __restrict__ B,
-                                                  int Q, int64_t K, int64_t chunk, float* __restrict__ part) {
-    __shared__ float sa[128][DOT_KC + 1];
-    __shared__ float sb[65][DOT_KC + 1];
-    const int t = threadIdx.x;
-    const int64_t k0 = (int64_t)blockIdx.x * chunk, k1 = min(K, k0 + chunk);
-    const int RQ = R * Q;
-    float acc[33];
+struct PtSmem {
+    float w2[C2][PB_W];
+    float h1[PB_P][PB_W];    // by point
+    float h1t[C1][PB_P + 4];  // by channel
+    union {
+        float d2[PB_P][PB_D];
+        int owner[NP];         // lowest channel of a point, while a set's points are listed
+        float red[16][4 * C1];  // at the end
+    };
+    float4 x[PB_P];
+    uint64_t pos[PB_P];  // which layer-1 pre-activations are positive
+    float w1[4 * C1];     // x y z weights and bias per channel
+    float b2[C2];
+    float g[C3];          // gradient per channel
+    int point[C3];        // a channel's argmax point, -1 without gradient
+    int place[C3];        // a channel's point's place among the distinct ones
+    int chan[C3];         // channels by place
+    int first[C3 + 1];    // where a place's channels start
+    int pts[C3];          // point of a place
+    int scan[33];
+};
+static_assert(sizeof(PtSmem) <= 113 * 1024, "two CTAs per SM");
+
+__global__ void __launch_bounds__(PB_T, 2)
+    k_net_pt_bwd(const uint16_t* __restrict__ w, float in_scale, const float4* __restrict__ sets,
+                 const float* __restrict__ pooled, const int32_t* __restrict__ argmax, int n_sets, lw_net_scratch scr,
+                 int32_t* __restrict__ place_out, float* __restrict__ part) {
+    extern __shared__ __align__(16) uint8_t raw[];
+    PtSmem& sm = *reinterpret_cast<PtSmem*>(raw);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    for (int e = t; e < C2 * C1; e += PB_T) sm.w2[e / C1][e % C1] = bf(w[LW_NET_OFF_W2 + e]);
+    for (int e = t; e < 3 * C1; e += PB_T) sm.w1[(e / 3) * 4 + e % 3] = bf(w[LW_NET_OFF_W1 + e]);
+    for (int e = t; e < C1; e += PB_T) sm.w1[e * 4 + 3] = bf(w[LW_NET_OFF_B1 + e]);
+    for (int e = t; e < C2; e += PB_T) sm.b2[e] = bf(w[LW_NET_OFF_B2 + e]);
+    // sums of the CTA: dW2 rows 8 jg .., columns 4 ig ..; db2 of row t; dW1 | db1 of columns 4 ig .. over the points 4 pg ..
+    const int jg = t / 16, ig = t % 16, pg = t / 16;
+    float dw2[8][4], dw1[4][4], db2 = 0.0f;
 #pragma unroll
-    for (int u = 0; u < 33; ++u) acc[u] = 0.0f;
-    for (int64_t kb = k0; kb < k1; kb += DOT_KC) {
-        const int kn = (int)min((int64_t)DOT_KC, k1 - kb);
-        for (int e = t; e < R * DOT_KC; e += 256) {
-            const int r = e / DOT_KC, kx = e % DOT_KC;
-            sa[r][kx] = kx < kn ? A[(int64_t)r * K + kb + kx] : 0.0f;
-        }
-        for (int e = t; e < Q * DOT_KC; e += 256) {
-            const int qq = e / DOT_KC, kx = e % DOT_KC;
-            sb[qq][kx] = kx < kn ? B[(int64_t)qq * K + kb + kx] : 0.0f;
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dw2[r][q] = 0.0f;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dw1[r][q] = 0.0f;
+    for (int set = blockIdx.x; set < n_sets; set += gridDim.x) {
+        for (int e = t; e < NP; e += PB_T) sm.owner[e] = C3;
+        __syncthreads();
+        // the distinct points, in the order of their lowest channel, and the channels by point
+        {
+            const int64_t kk = (int64_t)set * C3 + t;
+            const int p = argmax[kk];
+            const float v = pooled[kk];
+            const float g = (p >= 0 && p < NP && v > 0.0f) ? scr.dpool[kk] : 0.0f;
+            scr.dz3[kk] = g;
+            sm.g[t] = g;
+            sm.point[t] = g != 0.0f ? p : -1;
+            if (g != 0.0f) atomicMin(&sm.owner[p], t);
+            sm.first[t] = 0;
+            if (t == 0) sm.first[C3] = 0;
         }
         __syncthreads();
+        const int my = sm.point[t];
+        const bool lead = my >= 0 && sm.owner[my] == t;
+        int n_pts;
+        const int rank = block_rank(lead ? 1 : 0, sm.scan, &n_pts);
+        if (lead) {
+            sm.place[t] = rank;
+            sm.pts[rank] = my;
+        }
+        __syncthreads();
+        const int place = my >= 0 ? sm.place[sm.owner[my]] : -1;
+        place_out[(int64_t)set * C3 + t] = place;
+        if (place >= 0) atomicAdd(&sm.first[place], 1);
+        __syncthreads();
+        const int count = sm.first[t];
+        int total;
+        const int start = block_excl(count, sm.scan, &total);
+        sm.first[t] = start;
+        if (t == 0) sm.first[C3] = total;
+        __syncthreads();
+        if (place >= 0) {
+            // channels of a point in ascending order: my rank among the point's channels
+            int r = 0;
+            const int lead_c = sm.owner[my];
+            for (int c = lead_c; c < t; ++c) r += sm.point[c] == my;
+            sm.chan[sm.first[place] + r] = t;
+        }
+        for (int p0 = 0; p0 < n_pts; p0 += PB_P) {
+            const int np = min(PB_P, n_pts - p0);
+            __syncthreads();  // the tile's buffers are free
+            // layer 1: thread (point, 16 channels)
+            {
+                const int p = t / 4, c0 = (t % 4) * 16;
+                float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (p < np) q = __ldg(sets + (size_t)set * NP + sm.pts[p0 + p]);
+                const float x = q.x * in_scale, y = q.y * in_scale, z = q.z * in_scale;
+                unsigned pos = 0;
 #pragma unroll
-        for (int u = 0; u < 33; ++u) {
-            const int o = t + 256 * u;
-            if (o < RQ) {
-                const int r = o / Q, qq = o % Q;
-                float a = acc[u];
-#pragma unroll 8
-                for (int kx = 0; kx < DOT_KC; ++kx) a = fmaf(sa[r][kx], sb[qq][kx], a);
-                acc[u] = a;
+                for (int i = 0; i < 16; ++i) {
+                    const float4 w1 = *reinterpret_cast<const float4*>(&sm.w1[4 * (c0 + i)]);
+                    float a = w1.w;
+                    a = fmaf(w1.x, x, a);
+                    a = fmaf(w1.y, y, a);
+                    a = fmaf(w1.z, z, a);
+                    const float h = p < np ? bfr(fmaxf(a, 0.0f)) : 0.0f;
+                    if (a > 0.0f) pos |= 1u << i;
+                    sm.h1[p][c0 + i] = h;
+                    sm.h1t[c0 + i][p] = h;
+                }
+                reinterpret_cast<uint16_t*>(&sm.pos[p])[t % 4] = (uint16_t)pos;
+                if (t % 4 == 0) sm.x[p] = p < np ? make_float4(x, y, z, 1.0f) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            __syncthreads();
+            // layer 2 of points 8 warp .., channels lane + 32 q (the sum in the order of the forward recomputation: bias, then i)
+            {
+                float a[8][4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float b = sm.b2[lane + 32 * q];
+#pragma unroll
+                    for (int r = 0; r < 8; ++r) a[r][q] = b;
+                }
+#pragma unroll 2
+                for (int k = 0; k < C1; k += 4) {
+                    float wv[4][4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        *reinterpret_cast<float4*>(wv[q]) = *reinterpret_cast<const float4*>(&sm.w2[lane + 32 * q][k]);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        float h[8];
+                        *reinterpret_cast<float4*>(h) = *reinterpret_cast<const float4*>(&sm.h1t[k + e][8 * warp]);
+                        *reinterpret_cast<float4*>(h + 4) = *reinterpret_cast<const float4*>(&sm.h1t[k + e][8 * warp + 4]);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+#pragma unroll
+                            for (int r = 0; r < 8; ++r) a[r][q] = fmaf(wv[q][e], h[r], a[r][q]);
+                    }
+                }
+                // the row for dW3, and the gradient at layer 2: the point's channels' g W3, masked
+#pragma unroll 1
+                for (int r = 0; r < 8; ++r) {
+                    const int p = 8 * warp + r;
+                    float d[4] = {0.f, 0.f, 0.f, 0.f};
+                    float ar[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        ar[q] = a[0][q];
+#pragma unroll
+                        for (int s = 1; s < 8; ++s) ar[q] = r == s ? a[s][q] : ar[q];
+                    }
+                    if (p < np) {
+                        uint16_t* row = scr.h2g + ((int64_t)set * C3 + p0 + p) * C2;
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) row[lane + 32 * q] = to_bf(fmaxf(ar[q], 0.0f));
+                        const int k1 = sm.first[p0 + p + 1];
+                        for (int k = sm.first[p0 + p]; k < k1; ++k) {
+                            const int c = sm.chan[k];
+                            const float g = sm.g[c];
+                            const uint16_t* w3 = w + LW_NET_OFF_W3 + (size_t)c * C2 + lane;
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) d[q] = fmaf(g, bf(__ldg(w3 + 32 * q)), d[q]);
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) sm.d2[p][lane + 32 * q] = ar[q] > 0.0f ? d[q] : 0.0f;
+                }
+            }
+            __syncthreads();
+            // dW2 += D2^T H1, db2
+#pragma unroll 2
+            for (int p = 0; p < np; ++p) {
+                float d[8], h[4];
+                *reinterpret_cast<float4*>(d) = *reinterpret_cast<const float4*>(&sm.d2[p][8 * jg]);
+                *reinterpret_cast<float4*>(d + 4) = *reinterpret_cast<const float4*>(&sm.d2[p][8 * jg + 4]);
+                *reinterpret_cast<float4*>(h) = *reinterpret_cast<const float4*>(&sm.h1[p][4 * ig]);
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) dw2[r][q] = fmaf(d[r], h[q], dw2[r][q]);
+            }
+            if (t < C2)
+                for (int p = 0; p < np; ++p) db2 += sm.d2[p][t];
+            // D1 = D2 W2 under layer 1's mask, then dW1 | db1 += D1^T [x y z 1]
+            if (4 * pg < np) {
+                float a[4][4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) a[r][q] = 0.0f;
+#pragma unroll 2
+                for (int j = 0; j < C2; j += 4) {
+                    float d[4][4], wv[4][4];
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        *reinterpret_cast<float4*>(d[r]) = *reinterpret_cast<const float4*>(&sm.d2[4 * pg + r][j]);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        *reinterpret_cast<float4*>(wv[e]) = *reinterpret_cast<const float4*>(&sm.w2[j + e][4 * ig]);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+#pragma unroll
+                        for (int r = 0; r < 4; ++r)
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) a[r][q] = fmaf(d[r][e], wv[e][q], a[r][q]);
+                }
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const float4 x = sm.x[4 * pg + r];  // zero beyond the tile's points
+                    const unsigned pos = (unsigned)(sm.pos[4 * pg + r] >> (4 * ig)) & 15u;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float d = (pos >> q & 1u) ? a[r][q] : 0.0f;
+                        dw1[q][0] = fmaf(d, x.x, dw1[q][0]);
+                        dw1[q][1] = fmaf(d, x.y, dw1[q][1]);
+                        dw1[q][2] = fmaf(d, x.z, dw1[q][2]);
+                        dw1[q][3] = fmaf(d, x.w, dw1[q][3]);
+                    }
+                }
             }
         }
-        __syncthreads();
+        __syncthreads();  // the lists are free for the next set
     }
+    float* out = part + (int64_t)blockIdx.x * PB_PART;
 #pragma unroll
-    for (int u = 0; u < 33; ++u) {
-        const int o = t + 256 * u;
-        if (o < RQ) part[(int64_t)blockIdx.x * RQ + o] = acc[u];
-    }
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) out[(8 * jg + r) * C1 + 4 * ig + q] = dw2[r][q];
+    if (t < C2) out[C2 * C1 + t] = db2;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int d = 0; d < 4; ++d) sm.red[pg][(4 * ig + q) * 4 + d] = dw1[q][d];
+    __syncthreads();
+    float s = 0.0f;
+    for (int k = 0; k < 16; ++k) s += sm.red[k][t];
+    out[C2 * C1 + C2 + t] = s;
 }
 
-// out[o] = sum over splits of part[split][o], in split order; scattered into the gradient by `map`.
-// mode 0: dW2|db2 from C[128][65]; mode 1: dW1|db1 from C[64][4]
-__global__ void k_dot_reduce(const float* __restrict__ part, int splits, int RQ, int mode, float* __restrict__ grad) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= RQ) return;
+// The CTAs' sums into the gradient of layers 1 and 2: 8 lanes per element, each a fixed share of the CTAs in order.
+__global__ void k_net_pt_sum(const float* __restrict__ part, int parts, float* __restrict__ grad) {
+    __shared__ float sm[8][33];
+    const int e = blockIdx.x * 32 + (threadIdx.x & 31), share = threadIdx.x >> 5;
     float s = 0.0f;
-    for (int k = 0; k < splits; ++k) s += part[(int64_t)k * RQ + o];
-    if (mode == 0) {
-        const int j = o / 65, i = o % 65;
-        if (i < 64)
-            grad[LW_NET_OFF_W2 + j * 64 + i] = s;
-        else
-            grad[LW_NET_OFF_B2 + j] = s;
+    if (e < PB_PART) {
+#pragma unroll 8
+        for (int k = share; k < parts; k += 8) s += part[(int64_t)k * PB_PART + e];
+    }
+    sm[share][threadIdx.x & 31] = s;
+    __syncthreads();
+    if (share != 0 || e >= PB_PART) return;
+    s = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s += sm[k][threadIdx.x];
+    if (e < C2 * C1) {
+        grad[LW_NET_OFF_W2 + e] = s;
+    } else if (e < C2 * C1 + C2) {
+        grad[LW_NET_OFF_B2 + e - C2 * C1] = s;
     } else {
-        const int i = o / 4, d = o % 4;
+        const int q = e - C2 * C1 - C2, i = q / 4, d = q % 4;
         if (d < 3)
             grad[LW_NET_OFF_W1 + i * 3 + d] = s;
         else
@@ -484,21 +660,37 @@ __global__ void k_dot_reduce(const float* __restrict__ part, int splits, int RQ,
     }
 }
 
-// dW3[c][k] = sum_set dz3[set][c] h2g[set][c][k], db3[c] = sum_set dz3[set][c]
-__global__ void k_net_dw3(const lw_net_scratch scr, int n_sets, float* __restrict__ grad) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= C3 * (C2 + 1)) return;
-    const int c = o / (C2 + 1), k = o % (C2 + 1);
-    float s = 0.0f;
-    for (int set = 0; set < n_sets; ++set) {
+// dW3[c][k] = sum_set dz3[set][c] h2[point of (set, c)][k], db3[c] = sum_set dz3[set][c]: a CTA per channel, the sets in
+// DW3_G shares, a row's 128 values side by side (a thread per (c, k) over all sets: 0.33 ms at batch 256).
+constexpr int DW3_G = 8;
+__global__ void __launch_bounds__(C2 * DW3_G) k_net_dw3(const lw_net_scratch scr, const int32_t* __restrict__ place,
+                                                        int n_sets, float* __restrict__ grad) {
+    __shared__ float sum[DW3_G][C2], bias[DW3_G];
+    const int c = blockIdx.x, k = threadIdx.x % C2, share = threadIdx.x / C2;
+    float s = 0.0f, sb = 0.0f;
+#pragma unroll 4
+    for (int set = share; set < n_sets; set += DW3_G) {
         const int64_t kk = (int64_t)set * C3 + c;
         const float g = scr.dz3[kk];
-        if (g != 0.0f) s = fmaf(g, k < C2 ? bf(scr.h2g[kk * C2 + k]) : 1.0f, s);
+        const int p = max(place[kk], 0);
+        const float h = g != 0.0f ? bf(scr.h2g[((int64_t)set * C3 + p) * C2 + k]) : 0.0f;
+        s = fmaf(g, h, s);
+        sb += g;
     }
-    if (k < C2)
-        grad[LW_NET_OFF_W3 + c * C2 + k] = s;
-    else
-        grad[LW_NET_OFF_B3 + c] = s;
+    sum[share][k] = s;
+    if (k == 0) bias[share] = sb;
+    __syncthreads();
+    if (share != 0) return;
+    s = 0.0f;
+#pragma unroll
+    for (int q = 0; q < DW3_G; ++q) s += sum[q][k];
+    grad[LW_NET_OFF_W3 + c * C2 + k] = s;
+    if (k == 0) {
+        sb = 0.0f;
+#pragma unroll
+        for (int q = 0; q < DW3_G; ++q) sb += bias[q];
+        grad[LW_NET_OFF_B3 + c] = sb;
+    }
 }
 
 // the head's weights: dWh1[j][k] = sum_s dzh[s][j] bf16(pooled)[s][k], dbh1, dWh2[o][j] = sum_s dout[s][o] hid[s][j],
@@ -751,8 +943,9 @@ int net_forward_launch(const lw_initnet& net, const float* sets, int n, float* p
         LW_CUDA(cudaFuncSetAttribute(k_net_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_TOTAL));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    k_net_mlp<<<2 * n, NET_T, SM_TOTAL, s>>>(net.w, net.in_scale, reinterpret_cast<const float4*>(sets), pooled,
-                                             argmax, err);
+    const int ctas = 2 * n < device_sms() ? 2 * n : device_sms();  // one per SM; a second group's sets from there on
+    k_net_mlp<<<ctas, NET_G * NET_T, SM_TOTAL, s>>>(net.w, net.in_scale, reinterpret_cast<const float4*>(sets), 2 * n,
+                                                    pooled, argmax, err);
     k_net_head<<<n, CH, 0, s>>>(net.w, net.out_scale, pooled, hid, step);
     LW_LAUNCHED("lw_net_forward");
     count_launches(2);
@@ -830,21 +1023,24 @@ int lw_net_backward(const lw_initnet* net, const float* sets, int32_t n, const f
     cudaStream_t s = (cudaStream_t)stream;
     ProfScope prof("net_backward", s);
     const int n_sets = 2 * n;
-    const int64_t K = (int64_t)n_sets * C3;
     k_net_head_bwd<<<n, CH, 0, s>>>(net->w, net->out_scale, hid, step, target, w_loss, n, *scr);
-    k_net_pt_bwd<<<n_sets, C3, 0, s>>>(net->w, net->in_scale, reinterpret_cast<const float4*>(sets), pooled, argmax,
-                                       n_sets, *scr);
-    const int splits = 64;
-    const int64_t chunk = ((K + splits - 1) / splits + DOT_KC - 1) / DOT_KC * DOT_KC;
-    const int used = (int)((K + chunk - 1) / chunk);
-    k_dot_rows<<<used, 256, 0, s>>>(scr->d2t, C2, scr->h1t, C1 + 1, K, chunk, scr->part);
-    k_dot_reduce<<<blocks_for(C2 * (C1 + 1), 256), 256, 0, s>>>(scr->part, used, C2 * (C1 + 1), 0, net->grad);
-    k_dot_rows<<<used, 256, 0, s>>>(scr->d1t, C1, scr->xt, 4, K, chunk, scr->part);  // after the reduce above
-    k_dot_reduce<<<1, 256, 0, s>>>(scr->part, used, C1 * 4, 1, net->grad);
-    k_net_dw3<<<blocks_for(C3 * (C2 + 1), 256), 256, 0, s>>>(*scr, n_sets, net->grad);
+    static bool attr_set[64] = {};
+    int dev = 0;
+    LW_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !attr_set[dev]) {
+        LW_CUDA(cudaFuncSetAttribute(k_net_pt_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PtSmem)));
+        if (dev >= 0 && dev < 64) attr_set[dev] = true;
+    }
+    // d2t holds the CTAs' sums (at most one CTA per set, 32768 floats of d2t per set), xt the channels' places
+    const int ctas = n_sets < 2 * device_sms() ? n_sets : 2 * device_sms();
+    int32_t* place = reinterpret_cast<int32_t*>(scr->xt);
+    k_net_pt_bwd<<<ctas, PB_T, sizeof(PtSmem), s>>>(net->w, net->in_scale, reinterpret_cast<const float4*>(sets), pooled,
+                                                    argmax, n_sets, *scr, place, scr->d2t);
+    k_net_pt_sum<<<blocks_for(PB_PART, 32), 256, 0, s>>>(scr->d2t, ctas, net->grad);
+    k_net_dw3<<<C3, C2 * DW3_G, 0, s>>>(*scr, place, n_sets, net->grad);
     k_net_dhead<<<blocks_for(CH * (2 * C3 + 1) + NOUT * (CH + 1), 256), 256, 0, s>>>(*scr, pooled, hid, n, net->grad);
     LW_LAUNCHED("lw_net_backward");
-    count_launches(8);
+    count_launches(5);
     return LW_OK;
 }
 
