@@ -540,6 +540,12 @@ typedef struct lw_prior_grid {
  * 272-296). Seeds are 64-bit (no 2^23-point limit) and the flood is double buffered (deterministic). */
 int lw_prior_grid_build(lw_prior_grid* g, void* stream);
 
+/* The cell prefix array from its steps: u occupied cells (cells [u], ascending) and each one's first point (first [u]);
+ * start [ncell+1] on the device receives, for every cell, the first point of it or of the next occupied one, n from
+ * there on. What lw_prior_grid.start holds, at the cost of moving the occupied cells instead of all. */
+int lw_prior_starts(const int32_t* cells, const int32_t* first, int64_t u, int64_t n, int64_t ncell, int32_t* start,
+                    void* stream);
+
 /* Distance of n points (pts [n*3]) posed by T (row-major 4x4, host) to the nearest map point, 1e3 beyond the
  * band (mapgrid.py:173-194, PriorGrid.distances :298-305). */
 int lw_prior_distances(const lw_prior_grid* g, const float* pts, int64_t n, const double* T_host, float* out,

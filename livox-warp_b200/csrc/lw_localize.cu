@@ -152,55 +152,127 @@ __global__ void k_seed(lw_prior_grid g) {
 __global__ void k_unpack(lw_prior_grid g) {
     for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < g.ncell; c += (int64_t)gridDim.x * blockDim.x) {
         uint64_t v = g.seed[c];
-        g.nn[c] = v == ~0ULL ? -1 : (int32_t)(v & 0xFFFFFFFFULL);
+        g.nn2[c] = v == ~0ULL ? -1 : (int32_t)(v & 0xFFFFFFFFULL);
     }
 }
 
-// One flood step from `in` to `out`: the nearest of the seeds held `step` cells away in the 26 directions.
-__global__ void k_jfa(lw_prior_grid g, const int32_t* __restrict__ in, int32_t* __restrict__ out, int step) {
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < g.ncell; c += (int64_t)gridDim.x * blockDim.x) {
-        float px, py, pz;
-        cell_centre(g, c, px, py, pz);
-        int ix = (int)(c % g.nx), iy = (int)((c / g.nx) % g.ny), iz = (int)(c / ((int64_t)g.nx * g.ny));
-        int best = in[c];
-        float bd = 1.0e30f;
+// One flood step from `in` to `out`: the nearest of the seeds held STEP cells away in the 26 directions. Bound by instruction
+// issue: a thread per cell of a 32 x 8 patch of a z layer, so that no cell index is divided, in 32 bits where the grid's
+// cells fit (IDX); patches that lie STEP inside the grid read their neighbours without range checks; a seed equal to the
+// last one compared is passed over (it cannot win twice; neighbours along x mostly hold the same). A flat index with its
+// 64-bit divisions and a check per neighbour took 0.57 ms per step on 11.5M cells, 32-bit indices with the checks 0.37.
+constexpr int JFA_X = 32, JFA_Y = 8;
+// LAST also writes the distance field: the winner's distance in whole cm, 255 beyond the band (mapgrid.py:161-170).
+template <class IDX, int STEP, bool LAST>
+__global__ void __launch_bounds__(JFA_X * JFA_Y) k_jfa(lw_prior_grid g, const int32_t* __restrict__ in,
+                                                       int32_t* __restrict__ out, int tiles_x, int tiles_y) {
+    const int x0 = (int)(blockIdx.x % tiles_x) * JFA_X, tile = blockIdx.x / tiles_x;
+    const int y0 = tile % tiles_y * JFA_Y, iz = tile / tiles_y;
+    const int ix = x0 + threadIdx.x, iy = y0 + threadIdx.y;
+    const bool inside = x0 >= STEP && y0 >= STEP && iz >= STEP && x0 + JFA_X + STEP <= g.nx && y0 + JFA_Y + STEP <= g.ny &&
+                        iz + STEP < g.nz;
+    if (ix >= g.nx || iy >= g.ny) return;
+    const IDX nxy = (IDX)g.nx * g.ny, c = iz * nxy + (IDX)iy * g.nx + ix;
+    // the 27 seeds first (independent loads), then the distances
+    int seed[27];
+    if (inside) {
+#pragma unroll
+        for (int r = 0; r < 9; ++r) {
+            const int32_t* row = in + (c + (IDX)(r / 3 - 1) * STEP * nxy + (IDX)(r % 3 - 1) * STEP * g.nx);
+            seed[3 * r] = __ldg(row - STEP);
+            seed[3 * r + 1] = __ldg(row);
+            seed[3 * r + 2] = __ldg(row + STEP);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 27; ++k) {
+            const int jx = ix + (k % 3 - 1) * STEP, jy = iy + (k / 3 % 3 - 1) * STEP, jz = iz + (k / 9 - 1) * STEP;
+            const bool in_grid = jx >= 0 && jy >= 0 && jz >= 0 && jx < g.nx && jy < g.ny && jz < g.nz;
+            seed[k] = in_grid ? __ldg(in + (jz * nxy + (IDX)jy * g.nx + jx)) : -1;
+        }
+    }
+    int any = seed[0];
+#pragma unroll
+    for (int k = 1; k < 27; ++k) any = max(any, seed[k]);
+    int best = seed[13];
+    float bd = 1.0e30f;
+    if (any >= 0) {
+        const float4* __restrict__ P = reinterpret_cast<const float4*>(g.xyz);
+        // cell_centre's expressions
+        const float px = g.origin[0] + ((float)ix + 0.5f) * g.cell;
+        const float py = g.origin[1] + ((float)iy + 0.5f) * g.cell;
+        const float pz = g.origin[2] + ((float)iz + 0.5f) * g.cell;
         if (best >= 0) {
-            const float4 q = ld_pt(reinterpret_cast<const float4*>(g.xyz), best);
-            float ex = px - q.x, ey = py - q.y, ez = pz - q.z;
+            const float4 q = ld_pt(P, best);
+            const float ex = px - q.x, ey = py - q.y, ez = pz - q.z;
             bd = ex * ex + ey * ey + ez * ez;
         }
-        for (int dz = -1; dz <= 1; ++dz)
-            for (int dy = -1; dy <= 1; ++dy)
-                for (int dx = -1; dx <= 1; ++dx) {
-                    int64_t j = grid_flat(g, ix + dx * step, iy + dy * step, iz + dz * step);
-                    if (j < 0 || j == c) continue;
-                    int s = in[j];
-                    if (s < 0 || s == best) continue;
-                    const float4 q = ld_pt(reinterpret_cast<const float4*>(g.xyz), s);
-                    float ex = px - q.x, ey = py - q.y, ez = pz - q.z;
-                    float d2 = ex * ex + ey * ey + ez * ez;
-                    if (d2 < bd) {
-                        bd = d2;
-                        best = s;
-                    }
-                }
-        out[c] = best;
+        int last = -1;
+#pragma unroll
+        for (int k = 0; k < 27; ++k) {
+            const int s = seed[k];
+            if (k == 13 || s < 0 || s == best || s == last) continue;
+            last = s;
+            const float4 q = ld_pt(P, s);
+            const float ex = px - q.x, ey = py - q.y, ez = pz - q.z;
+            const float d2 = ex * ex + ey * ey + ez * ez;
+            if (d2 < bd) {
+                bd = d2;
+                best = s;
+            }
+        }
+    }
+    out[c] = best;
+    if (LAST) {
+        const int v = best < 0 ? 255 : (int)(sqrtf(bd) * 100.0f + 0.5f);
+        g.df[c] = (uint8_t)(v < 255 ? v : 255);
     }
 }
 
-__global__ void k_df(lw_prior_grid g) {
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < g.ncell; c += (int64_t)gridDim.x * blockDim.x) {
-        int s = g.nn[c];
-        if (s < 0) {
-            g.df[c] = 255;
-            continue;
+template <class IDX>
+static void jfa_step(const lw_prior_grid& g, const int32_t* in, int32_t* out, int step, bool last, unsigned tiles, int tx,
+                     int ty, cudaStream_t s) {
+    const dim3 cta(JFA_X, JFA_Y);
+    if (step == 8)
+        k_jfa<IDX, 8, false><<<tiles, cta, 0, s>>>(g, in, out, tx, ty);
+    else if (step == 4)
+        k_jfa<IDX, 4, false><<<tiles, cta, 0, s>>>(g, in, out, tx, ty);
+    else if (step == 2)
+        k_jfa<IDX, 2, false><<<tiles, cta, 0, s>>>(g, in, out, tx, ty);
+    else if (!last)
+        k_jfa<IDX, 1, false><<<tiles, cta, 0, s>>>(g, in, out, tx, ty);
+    else
+        k_jfa<IDX, 1, true><<<tiles, cta, 0, s>>>(g, in, out, tx, ty);
+}
+
+// start[c], the first point of cell c or of the next occupied cell after it, n beyond the last. A warp per run of ST_RUN
+// cells: it finds the occupied cells that lie in its run by binary search, and each lane its own among those few (a warp per
+// occupied cell filling the gap before it left the widest gaps to single warps: 0.2 ms on 11.5M cells).
+constexpr int ST_RUN = 1024;
+
+// The first j in [lo, hi) with cells[j] >= c, hi if none.
+__device__ __forceinline__ int64_t first_cell(const int32_t* __restrict__ cells, int64_t lo, int64_t hi, int64_t c) {
+    while (lo < hi) {
+        const int64_t mid = (lo + hi) >> 1;
+        if ((int64_t)__ldg(cells + mid) < c)
+            lo = mid + 1;
+        else
+            hi = mid;
+    }
+    return lo;
+}
+
+__global__ void k_starts(const int32_t* __restrict__ cells, const int32_t* __restrict__ first, int64_t u, int64_t n,
+                         int64_t ncell, int32_t* __restrict__ start) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * ST_RUN <= ncell; w += nwarps) {
+        const int64_t c0 = w * ST_RUN, c1 = min(c0 + ST_RUN, ncell + 1);
+        const int64_t j0 = first_cell(cells, 0, u, c0), j1 = first_cell(cells, j0, u, c1);
+        for (int64_t c = c0 + lane; c < c1; c += 32) {
+            const int64_t j = first_cell(cells, j0, j1, c);
+            start[c] = j < u ? __ldg(first + j) : (int32_t)n;
         }
-        float px, py, pz;
-        cell_centre(g, c, px, py, pz);
-        const float4 q = ld_pt(reinterpret_cast<const float4*>(g.xyz), s);
-        float d = len3(px - q.x, py - q.y, pz - q.z) * 100.0f;
-        int v = (int)(d + 0.5f);
-        g.df[c] = (uint8_t)(v < 255 ? v : 255);
     }
 }
 
@@ -846,23 +918,38 @@ int lw_prior_grid_build(lw_prior_grid* g, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     int gc = blocks_for(g->ncell, 256, 16 * device_sms());
     int gp = blocks_for(g->n, 256, 16 * device_sms());
+    const int tiles_x = (g->nx + JFA_X - 1) / JFA_X, tiles_y = (g->ny + JFA_Y - 1) / JFA_Y;
+    const int64_t tiles = (int64_t)tiles_x * tiles_y * g->nz;
+    if (tiles > 0x7FFFFFFF) return set_error(LW_ECAPACITY, "lw_prior_grid_build: %lld tiles", (long long)tiles);
     ProfScope prof("grid_build", s);
     k_seed_clear<<<gc, 256, 0, s>>>(*g);
     k_seed<<<gp, 256, 0, s>>>(*g);
     k_unpack<<<gc, 256, 0, s>>>(*g);
     const int steps[5] = {8, 4, 2, 1, 1};  // mapgrid.py:31
-    int32_t* a = g->nn;
-    int32_t* bbuf = g->nn2;
+    int32_t* a = g->nn2;  // an odd number of steps: from nn2 the last lands in nn
+    int32_t* bbuf = g->nn;
     for (int k = 0; k < 5; ++k) {
-        k_jfa<<<gc, 256, 0, s>>>(*g, a, bbuf, steps[k]);
+        if (g->ncell < 0x7FFFFFFF)
+            jfa_step<int32_t>(*g, a, bbuf, steps[k], k == 4, (unsigned)tiles, tiles_x, tiles_y, s);
+        else
+            jfa_step<int64_t>(*g, a, bbuf, steps[k], k == 4, (unsigned)tiles, tiles_x, tiles_y, s);
         int32_t* t = a;
         a = bbuf;
         bbuf = t;
     }
-    if (a != g->nn) LW_CUDA(cudaMemcpyAsync(g->nn, a, g->ncell * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
-    k_df<<<gc, 256, 0, s>>>(*g);
     LW_LAUNCHED("lw_prior_grid_build");
-    count_launches(9);
+    count_launches(8);
+    return LW_OK;
+}
+
+int lw_prior_starts(const int32_t* cells, const int32_t* first, int64_t u, int64_t n, int64_t ncell, int32_t* start,
+                    void* stream) {
+    if (u < 0 || n < 0 || n > 0x7FFFFFFF || ncell < 0 || !start || (u > 0 && (!cells || !first)))
+        return set_error(LW_EINVAL, "lw_prior_starts: bad arguments");
+    k_starts<<<blocks_for((ncell / ST_RUN + 1) * 32, 256, 32 * device_sms()), 256, 0, (cudaStream_t)stream>>>(cells, first, u, n, ncell,
+                                                                                               start);
+    LW_LAUNCHED("lw_prior_starts");
+    count_launches(1);
     return LW_OK;
 }
 

@@ -79,6 +79,8 @@ class PriorGrid:
         counts = np.bincount(key, minlength=ncell)
         start = np.zeros(ncell + 1, np.int32)
         np.cumsum(counts, out=start[1:])
+        key = key[order]
+        steps = np.flatnonzero(np.concatenate([[True], key[1:] != key[:-1]]))  # where the sorted points enter a cell
         xyz = np.ascontiguousarray(xyz[order])
         nrm = nrm[order]
         nrm = np.ascontiguousarray(nrm / np.maximum(np.linalg.norm(nrm, axis=1, keepdims=True), 1e-6),
@@ -86,6 +88,7 @@ class PriorGrid:
         planar = np.ascontiguousarray(planar[order])
         return {"_prepared": True, "xyz": xyz, "normal": nrm, "planarity": planar, "lo": lo, "hi": hi,
                 "origin": origin, "cell": float(cell), "dims": dims, "start": start,
+                "cells": key[steps].astype(np.int32), "first": steps.astype(np.int32),
                 "levels": horizontal_levels(xyz, nrm, planar)}
 
     def __init__(self, host: dict, device=None):
@@ -145,12 +148,17 @@ class PriorGrid:
         s = stream if stream is not None else torch.cuda.current_stream(self.device)
         h = self._host
         with torch.cuda.stream(s):
-            rec = np.empty((self.n, 4), np.float32)
-            rec[:, :3] = h["xyz"]
-            rec[:, 3] = h["planarity"]
-            self.xyzp.copy_(torch.from_numpy(rec))
+            d = self.device
+            # the records are put together on the device: on the host the packing took as long as the copies
+            self.xyzp[:, :3].copy_(torch.from_numpy(h["xyz"]).to(d))
+            self.xyzp[:, 3].copy_(torch.from_numpy(h["planarity"]).to(d))
             self.nrm.copy_(torch.from_numpy(h["normal"]))
-            self.start.copy_(torch.from_numpy(h["start"]))
+            if "cells" in h and "first" in h:  # the prefix array from the occupied cells: few of a grid's cells hold points
+                cells, first = torch.from_numpy(h["cells"]).to(d), torch.from_numpy(h["first"]).to(d)
+                _lib.call("lw_prior_starts", _lib.ptr(cells), _lib.ptr(first), len(cells), self.n, self.ncell,
+                          _lib.ptr(self.start), _lib.stream_ptr(s))
+            else:
+                self.start.copy_(torch.from_numpy(h["start"]))
             seed = torch.empty(self.ncell, dtype=torch.int64, device=self.device)
             nn2 = torch.empty(self.ncell, dtype=torch.int32, device=self.device)
             g = self._struct(seed, nn2)
