@@ -617,6 +617,20 @@ int lw_loc_icp_batch(const lw_prior_grid* g, lw_loc_batch* b, int32_t n_hyp, int
                      int32_t n_stages, const double* dmax, const int32_t* iters, float alpha, int32_t min_count,
                      int32_t blocks_per_sm, int32_t grid, void* stream);
 
+/* Workspace of lw_loc_icp_batch_ws, contents undefined between calls: cap slots, at least tiles * tile of a launch for it to be
+ * used (a launch with more tiles runs without). sorted is 16-byte aligned. */
+typedef struct lw_loc_ws {
+    float* sorted;  /* [cap*4] each hypothesis' points, neighbours together: x, y, z, place in the scan */
+    int32_t* match; /* [cap] nearest map point of each point, in the scans' order */
+    int64_t cap;
+} lw_loc_ws;
+
+/* lw_loc_icp_batch with a workspace (ws may be NULL): the nearest points are found in an order in which a warp's points are
+ * neighbours, each from its match of the iteration before. The same poses, counts and fits, bit for bit. */
+int lw_loc_icp_batch_ws(const lw_prior_grid* g, lw_loc_batch* b, int32_t n_hyp, int32_t n_tiles, int32_t tile,
+                        int32_t n_stages, const double* dmax, const int32_t* iters, float alpha, int32_t min_count,
+                        int32_t blocks_per_sm, int32_t grid, const lw_loc_ws* ws, void* stream);
+
 /* ---- learned initial pose (no counterpart in the reference: its odometry predicts with constant velocity) ---- */
 
 /* A point-set network proposing the ICP start pose: a shared per-point MLP 3 -> 64 -> 128 -> 256 (ReLU), a max

@@ -128,6 +128,134 @@ __device__ int nearest_point(const lw_prior_grid& g, float wx, float wy, float w
     return best >= 0 ? best : seed;
 }
 
+// nearest_point for a query whose answer a moment ago, or in the pose before, was point `prev` (-1: unknown). Points are
+// sorted by cell with x fastest, so the scan order (dz, dy, dx, then index) is the order of the indices and the three cells of
+// a row are one run of points. Where prev lies surely within the 27 cells (closer than a cell less twice BOX_SLACK), its
+// distance bounds the answer before anything is scanned, and rows and cells whose boxes lie farther are passed over; the
+// first minimum is then found among the rest as before. While nothing lies within a cell the 27 seeds are compared in
+// order, a seed equal to the last one once.
+// The runs to scan are listed first (runs: 9 slots of shared memory per lane, this lane's column) and then walked, two points
+// a step: a warp takes as many steps as its busiest lane has points, where walking row by row takes the busiest lane's of
+// every row.
+__device__ int nearest_warm(const lw_prior_grid& g, float wx, float wy, float wz, int prev, int2 (*runs)[32]) {
+    const float4* __restrict__ P = reinterpret_cast<const float4*>(g.xyz);
+    int ix, iy, iz;
+    grid_idx(g, wx, wy, wz, ix, iy, iz);
+    if (ix < -1 || iy < -1 || iz < -1 || ix > g.nx || iy > g.ny || iz > g.nz) return -1;  // none of the 27 is in the grid
+    const float cell2 = g.cell * g.cell;
+    const float fx = (wx - g.origin[0]) - (float)ix * g.cell;
+    const float fy = (wy - g.origin[1]) - (float)iy * g.cell;
+    const float fz = (wz - g.origin[2]) - (float)iz * g.cell;
+    const int64_t nx = g.nx, nxy = nx * g.ny;
+    const int64_t c0 = iz * nxy + iy * nx + ix;
+    const bool own_in = ix >= 0 && iy >= 0 && iz >= 0 && ix < g.nx && iy < g.ny && iz < g.nz;
+    float ub = cell2;
+    if (prev >= 0 && prev < g.n) {
+        const float4 q = ld_pt(P, prev);
+        const float ex = wx - q.x, ey = wy - q.y, ez = wz - q.z;
+        const float d2 = ex * ex + ey * ey + ez * ez;
+        const float sure = g.cell - 2.0f * BOX_SLACK;
+        if (sure > 0.0f && d2 < sure * sure) ub = d2;
+    } else if (own_in) {
+        const int k1 = __ldg(g.start + c0 + 1);
+        for (int k = __ldg(g.start + c0); k < k1; ++k) {
+            const float4 q = ld_pt(P, k);
+            const float ex = wx - q.x, ey = wy - q.y, ez = wz - q.z;
+            ub = fminf(ub, ex * ex + ey * ey + ez * ez);
+        }
+    }
+    ub *= 1.00001f;
+    auto gap2 = [&](float f, int o) {
+        const float l = fmaxf((o < 0 ? f : (o > 0 ? g.cell - f : 0.0f)) - BOX_SLACK, 0.0f);
+        return l * l;
+    };
+    const float xl = gap2(fx, -1), xr = gap2(fx, 1);
+    const int lane = threadIdx.x & 31;
+    int n = 0;
+#pragma unroll
+    for (int dz = -1; dz <= 1; ++dz) {
+        const float z2 = gap2(fz, dz);
+#pragma unroll
+        for (int dy = -1; dy <= 1; ++dy) {
+            const float yz2 = gap2(fy, dy) + z2;
+            const int lo = max(xl + yz2 > ub ? ix : ix - 1, 0), hi = min(xr + yz2 > ub ? ix : ix + 1, g.nx - 1);
+            const bool in = yz2 <= ub && lo <= hi && iz + dz >= 0 && iz + dz < g.nz && iy + dy >= 0 && iy + dy < g.ny;
+            if (in) {
+                const int32_t* row = g.start + (c0 + dz * nxy + dy * nx - ix);
+                const int k0 = __ldg(row + lo), k1 = __ldg(row + hi + 1);
+                if (k0 < k1) runs[n++][lane] = make_int2(k0, k1);
+            }
+        }
+    }
+    int best = -1;
+    float bd = cell2;
+    int j = 0, k = 0, k1 = 0;
+    while (true) {
+        if (k >= k1) {
+            if (j >= n) break;
+            const int2 r = runs[j++][lane];
+            k = r.x;
+            k1 = r.y;
+        }
+        const int l = min(k + 1, k1 - 1);
+        const float4 q = ld_pt(P, k), r = ld_pt(P, l);
+        const float ex = wx - q.x, ey = wy - q.y, ez = wz - q.z;
+        const float d2 = ex * ex + ey * ey + ez * ez;
+        const float fx2 = wx - r.x, fy2 = wy - r.y, fz2 = wz - r.z;
+        const float e2 = fx2 * fx2 + fy2 * fy2 + fz2 * fz2;
+        if (d2 < bd) {
+            bd = d2;
+            best = k;
+        }
+        if (e2 < bd) {
+            bd = e2;
+            best = l;
+        }
+        k += 2;
+    }
+    if (best >= 0) return best;
+    int seed = -1, last = -1;
+    float sd = 1.0e30f;
+    // a row of three seeds at a time, the next row's already on their way
+    auto row_of = [&](int r, int (&v)[3]) {
+        const int z = iz + r / 3 - 1, y = iy + r % 3 - 1;
+        const bool in = r < 9 && z >= 0 && y >= 0 && z < g.nz && y < g.ny;
+        const int32_t* row = g.nn + (in ? z * nxy + y * nx : 0);
+#pragma unroll
+        for (int o = 0; o < 3; ++o) {
+            const int x = ix + o - 1;
+            v[o] = in && x >= 0 && x < g.nx ? __ldg(row + x) : -1;
+        }
+    };
+    int next[3];
+    row_of(0, next);
+#pragma unroll 1
+    for (int r = 0; r < 9; ++r) {
+        const int s0 = next[0], s1 = next[1], s2 = next[2];
+        row_of(r + 1, next);
+        const bool b0 = s0 >= 0 && s0 != last;
+        last = s0 >= 0 ? s0 : last;
+        const bool b1 = s1 >= 0 && s1 != last;
+        last = s1 >= 0 ? s1 : last;
+        const bool b2 = s2 >= 0 && s2 != last;
+        last = s2 >= 0 ? s2 : last;
+        if (!(b0 || b1 || b2)) continue;
+        const float4 q0 = ld_pt(P, b0 ? s0 : last), q1 = ld_pt(P, b1 ? s1 : last), q2 = ld_pt(P, b2 ? s2 : last);
+        auto take = [&](bool on, int s, float4 q) {
+            const float ex = wx - q.x, ey = wy - q.y, ez = wz - q.z;
+            const float d2 = ex * ex + ey * ey + ez * ez;
+            if (on && d2 < sd) {
+                sd = d2;
+                seed = s;
+            }
+        };
+        take(b0, s0, q0);
+        take(b1, s1, q1);
+        take(b2, s2, q2);
+    }
+    return seed;
+}
+
 // ---- grid build (mapgrid.py:105-170, 272-296) -------------------------------------------------------------
 __global__ void k_seed_clear(lw_prior_grid g) {
     for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < g.ncell; c += (int64_t)gridDim.x * blockDim.x)
@@ -330,15 +458,16 @@ __device__ __forceinline__ void tile_range(const lw_loc_batch& b, int tile, int 
 
 // One (hypothesis, point) pair's terms (localize.py:144-167) added to a[k * S], k < LTERMS (S = 1: registers;
 // S = 32: a warp's per-lane columns in shared memory).
-template <int S>
-__device__ __forceinline__ void loc_terms(const lw_prior_grid& g, const LocPose& P, float4 p, float max_d2, float c2,
-                                          float alpha, float* a) {
+// KNOWN: the point's nearest map point s was found before; else it is searched for here.
+template <int S, bool KNOWN>
+__device__ __forceinline__ void loc_terms(const lw_prior_grid& g, const LocPose& P, float4 p, int s, float max_d2,
+                                          float c2, float alpha, float* a) {
     float lx = P.R[0] * p.x + P.R[1] * p.y + P.R[2] * p.z + P.tr[0];
     float ly = P.R[3] * p.x + P.R[4] * p.y + P.R[5] * p.z + P.tr[1];
     float lz = P.R[6] * p.x + P.R[7] * p.y + P.R[8] * p.z + P.tr[2];
     float wx = lx + P.c[0], wy = ly + P.c[1], wz = lz + P.c[2];
-    int s = nearest_point(g, wx, wy, wz);
-    if (s < 0) return;
+    if (!KNOWN) s = nearest_point(g, wx, wy, wz);
+    if (s < 0 || (KNOWN && s >= g.n)) return;
     const float4 q = ld_pt(reinterpret_cast<const float4*>(g.xyz), s);
     float r0 = wx - q.x, r1 = wy - q.y, r2 = wz - q.z;
     if (r0 * r0 + r1 * r1 + r2 * r2 > max_d2) return;
@@ -514,29 +643,112 @@ __device__ __forceinline__ float warp_reduce_scatter32(float (&v)[32], int lane)
     return v[0];
 }
 
-// The next tile of pass `pass` for the calling warp (one atomic per tile, broadcast to the warp).
-__device__ __forceinline__ int next_tile(const lw_loc_batch& b, int pass, int lane) {
-    int t = 0;
-    if (lane == 0) t = atomicAdd(b.next + pass, 1);
-    return __shfl_sync(FULL, t, 0);
+// The tiles of pass `pass` for the calling warp, taken `grab` at a time (one atomic, broadcast to the warp). A tile per atomic
+// made the atomics on the one counter, about 3 ns each, take as long as the searches themselves: 0.26 ms for 88,000
+// tiles; a grab of a quarter of a warp's share still evens out tiles of uneven work.
+struct TileTaker {
+    int t = 0, left = 0;
+    __device__ __forceinline__ int next(const lw_loc_batch& b, int pass, int lane, int grab) {
+        if (left == 0) {
+            int v = 0;
+            if (lane == 0) v = atomicAdd(b.next + pass, grab);
+            t = __shfl_sync(FULL, v, 0);
+            left = grab;
+        }
+        --left;
+        return t++;
+    }
+};
+
+// A hypothesis' scan points, a CTA each, gathered into 25 cm boxes of the sensor frame in Morton order (32 boxes per axis,
+// wrapping) by a counting sort: ws.sorted holds (x, y, z, place in the scan) in slots hyp_tile[h] * tile on, and
+// ws.match is set to "unknown". Only neighbourhood matters: the order within a box is whatever the atomics give.
+constexpr int LS_BITS = 5, LS_BOXES = 1 << (3 * LS_BITS), LS_T = 1024;
+
+__device__ __forceinline__ unsigned spread5(unsigned v) {  // bits 0..4 to every third
+    v = (v | (v << 8)) & 0x100Fu;
+    v = (v | (v << 4)) & 0x10C3u;
+    return (v | (v << 2)) & 0x1249u;
+}
+
+__global__ void __launch_bounds__(LS_T) k_loc_sort(lw_loc_batch b, lw_loc_ws ws, int n_hyp_ub, int n_tiles_ub, int tile) {
+    extern __shared__ int box[];  // [LS_BOXES]
+    __shared__ int sm[33];
+    const int n_hyp = b.dims ? min(__ldg(b.dims), n_hyp_ub) : n_hyp_ub;
+    const int n_tiles = b.dims ? min(__ldg(b.dims + 1), n_tiles_ub) : n_tiles_ub;
+    if ((int64_t)n_tiles * tile > ws.cap) return;
+    for (int h = blockIdx.x; h < n_hyp; h += gridDim.x) {
+        const int t0 = max(b.hyp_tile[h], 0), t1 = min(b.hyp_tile[h + 1], n_tiles);
+        if (t0 >= t1) continue;
+        const int lo = b.tile_lo[t0];
+        if (lo < 0) continue;
+        const int hi = (int)min((int64_t)b.scan_end[h], b.pts_cap);
+        const int n = min(hi - lo, (t1 - t0) * tile);
+        if (n <= 0) continue;
+        auto box_of = [&](float4 p) {
+            const unsigned x = (unsigned)ifloor(p.x * 4.0f) & 31u, y = (unsigned)ifloor(p.y * 4.0f) & 31u,
+                           z = (unsigned)ifloor(p.z * 4.0f) & 31u;
+            return (int)(spread5(x) | (spread5(y) << 1) | (spread5(z) << 2));
+        };
+        __syncthreads();
+        for (int k = threadIdx.x; k < LS_BOXES; k += LS_T) box[k] = 0;
+        __syncthreads();
+        const float4* pts = reinterpret_cast<const float4*>(b.pts) + lo;
+        for (int i = threadIdx.x; i < n; i += LS_T) atomicAdd(&box[box_of(__ldg(pts + i))], 1);
+        __syncthreads();
+        // exclusive scan of the boxes, LS_BOXES / LS_T consecutive ones per thread
+        constexpr int PER = LS_BOXES / LS_T;
+        int sum = 0;
+        for (int k = 0; k < PER; ++k) sum += box[threadIdx.x * PER + k];
+        int tot;
+        int at = block_excl(sum, sm, &tot);
+        for (int k = 0; k < PER; ++k) {
+            const int c = box[threadIdx.x * PER + k];
+            box[threadIdx.x * PER + k] = at;
+            at += c;
+        }
+        __syncthreads();
+        float4* out = reinterpret_cast<float4*>(ws.sorted) + (int64_t)t0 * tile;
+        int32_t* match = ws.match + (int64_t)t0 * tile;
+        for (int i = threadIdx.x; i < n; i += LS_T) {
+            const float4 p = __ldg(pts + i);
+            out[atomicAdd(&box[box_of(p)], 1)] = make_float4(p.x, p.y, p.z, __int_as_float(i));
+            match[i] = -1;
+        }
+    }
 }
 
 // MINB: CTAs of LOC_BLOCK threads the register budget must let reside per SM. With 2 or 3 the per-lane term
 // sums of a tile and the tile's pose live in registers; with 4 to 6 they live in shared memory (a [30][32]
 // column block and one pose per warp, 31 KB per CTA), which frees ~47 registers across the nearest-point search
 // so that two to three times the 2-CTA warp count stays resident.
+//
+// With a workspace (ws) each iteration first finds every point's nearest map point, in an order in which a warp's 32 points
+// are neighbours (k_loc_sort) -- scans come in the order they were fired, whose 32 points lie in as many places: a
+// quarter of the loads hit L1 and half the lanes idled -- starting from the point's match of the iteration before; the
+// terms are then summed from the matches in the scan's own order, so that every sum and pose is the one without a workspace,
+// bit for bit. 256 scans of 2,000-20,000 points, 31 iterations: 13.3 ms, 23.1 without; an iteration is 0.19-0.35 ms of searches
+// (bound by L1's one line a cycle: every lane's loads are lines of their own, about 570 a tile), 0.08 of sums, 0.03 of
+// the tile partials' sums and solves, 0.1 of waiting at the three barriers.
 template <int MINB>
 __global__ void __launch_bounds__(LOC_BLOCK, MINB)
-    k_loc_icp(lw_prior_grid g, lw_loc_batch b, LocArgs la) {
+    k_loc_icp(lw_prior_grid g, lw_loc_batch b, lw_loc_ws ws, LocArgs la) {
     constexpr bool SMEM_ACC = MINB >= 4;
-    __shared__ float s_acc[SMEM_ACC ? LOC_BLOCK / 32 : 1][SMEM_ACC ? LTERMS : 1][32];
+    __shared__ __align__(16) float s_acc[SMEM_ACC ? LOC_BLOCK / 32 : 1][SMEM_ACC ? LTERMS : 1][32];
     __shared__ LocPose s_pose[SMEM_ACC ? LOC_BLOCK / 32 : 1];
+    __shared__ int2 s_runs[SMEM_ACC ? 1 : LOC_BLOCK / 32][9][32];
     __shared__ double sv[32];
     __shared__ int s_stop;
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int n_hyp = b.dims ? min(__ldg(b.dims), la.n_hyp) : la.n_hyp;
     const int n_tiles = b.dims ? min(__ldg(b.dims + 1), la.n_tiles) : la.n_tiles;
+    const bool sorted = ws.sorted != nullptr && (int64_t)n_tiles * la.tile <= ws.cap;
+    // a search's runs: in the term sums' columns, which are free while searching
+    int2(*runs)[32] = SMEM_ACC ? reinterpret_cast<int2(*)[32]>(&s_acc[tid >> 5][0][0]) : s_runs[SMEM_ACC ? 0 : tid >> 5];
+    static_assert(sizeof(int2) * 9 * 32 <= sizeof(float) * LTERMS * 32, "a search's runs fit the term sums' columns");
+    const int warp_id = (blockIdx.x * LOC_BLOCK + tid) >> 5, n_warps = gridDim.x * (LOC_BLOCK / 32);
+    const int grab = max(1, min(8, n_tiles / (4 * n_warps)));
     int it_total = 0;
     for (int stage = 0; stage < la.n_stages; ++stage) {
         const float max_d2 = la.max_d2[stage];
@@ -544,8 +756,38 @@ __global__ void __launch_bounds__(LOC_BLOCK, MINB)
         for (int it = 0; it < la.iters[stage]; ++it, ++it_total) {
             // phase A: warp tiles, handed out in order of arrival, -> float64 tile partials. A tile's partial
             // does not depend on which warp computed it, so the sums of phase B are deterministic.
-            for (;;) {
-                const int tile = next_tile(b, it_total, lane);
+            if (sorted) {
+                for (TileTaker take;;) {
+                    const int tile = take.next(b, it_total, lane, grab);
+                    if (tile >= n_tiles) break;
+                    int h, lo, hi;
+                    tile_range(b, tile, n_hyp, h, lo, hi);
+                    if (h < 0) continue;
+                    LocPose Pr;
+                    LocPose& P = SMEM_ACC ? s_pose[tid >> 5] : Pr;
+                    if (!SMEM_ACC || lane == 0) loc_pose(b.T + 16 * h, P);
+                    __syncwarp();
+                    const int64_t slot0 = (int64_t)tile * la.tile;
+                    int32_t* match = ws.match + (int64_t)max(__ldg(b.hyp_tile + h), 0) * la.tile;
+                    const int count = min(hi - lo, la.tile);
+                    for (int i = lane; i < count; i += 32) {
+                        const float4 p = __ldg(reinterpret_cast<const float4*>(ws.sorted) + slot0 + i);
+                        const int place = __float_as_int(p.w);
+                        if (place < 0 || (match - ws.match) + place >= ws.cap) continue;  // tables that do not fit together
+                        int32_t* m = match + place;
+                        const float lx = P.R[0] * p.x + P.R[1] * p.y + P.R[2] * p.z + P.tr[0];
+                        const float ly = P.R[3] * p.x + P.R[4] * p.y + P.R[5] * p.z + P.tr[1];
+                        const float lz = P.R[6] * p.x + P.R[7] * p.y + P.R[8] * p.z + P.tr[2];
+                        __stcg(m, nearest_warm(g, lx + P.c[0], ly + P.c[1], lz + P.c[2], __ldcg(m), runs));
+                    }
+                    __syncwarp();  // the pose slot is rewritten by the warp's next tile
+                }
+                if (!grid_barrier(b.bar, b.err, 3)) return;
+            }
+            TileTaker take;
+            for (int turn = warp_id;; turn += n_warps) {
+                // the sums alone are even work: tiles in turn; with the searches in them tiles go to the next free warp
+                const int tile = sorted ? turn : take.next(b, it_total, lane, grab);
                 if (tile >= n_tiles) break;
                 int h, lo, hi;
                 tile_range(b, tile, n_hyp, h, lo, hi);
@@ -564,16 +806,28 @@ __global__ void __launch_bounds__(LOC_BLOCK, MINB)
                         float* col = &s_acc[tid >> 5][0][lane];
 #pragma unroll
                         for (int k = 0; k < LTERMS; ++k) col[k * 32] = 0.0f;
-                        for (int i = lo + lane; i < end; i += 32)
-                            loc_terms<32>(g, P, __ldg(reinterpret_cast<const float4*>(b.pts) + i), max_d2, c2,
-                                          la.alpha, col);
+                        if (sorted)
+                            for (int i = lo + lane; i < end; i += 32)
+                                loc_terms<32, true>(g, P, __ldg(reinterpret_cast<const float4*>(b.pts) + i),
+                                                    __ldcg(ws.match + (int64_t)tile * la.tile + (i - lo)), max_d2, c2,
+                                                    la.alpha, col);
+                        else
+                            for (int i = lo + lane; i < end; i += 32)
+                                loc_terms<32, false>(g, P, __ldg(reinterpret_cast<const float4*>(b.pts) + i), -1, max_d2,
+                                                     c2, la.alpha, col);
 #pragma unroll
                         for (int k = 0; k < LTERMS; ++k) v[k] = col[k * 32];
                         __syncwarp();  // the pose slot is rewritten by the warp's next tile
                     } else {
-                        for (int i = lo + lane; i < end; i += 32)
-                            loc_terms<1>(g, P, __ldg(reinterpret_cast<const float4*>(b.pts) + i), max_d2, c2,
-                                         la.alpha, v);
+                        if (sorted)
+                            for (int i = lo + lane; i < end; i += 32)
+                                loc_terms<1, true>(g, P, __ldg(reinterpret_cast<const float4*>(b.pts) + i),
+                                                   __ldcg(ws.match + (int64_t)tile * la.tile + (i - lo)), max_d2, c2,
+                                                   la.alpha, v);
+                        else
+                            for (int i = lo + lane; i < end; i += 32)
+                                loc_terms<1, false>(g, P, __ldg(reinterpret_cast<const float4*>(b.pts) + i), -1, max_d2,
+                                                    c2, la.alpha, v);
                     }
                 }
                 const float sum = warp_reduce_scatter32(v, lane);
@@ -585,7 +839,16 @@ __global__ void __launch_bounds__(LOC_BLOCK, MINB)
                 const int t0 = max(b.hyp_tile[h], 0), t1 = min(b.hyp_tile[h + 1], n_tiles);
                 if (tid < LTERMS) {
                     double s = 0.0;
-                    for (int t = t0; t < t1; ++t) s += __ldcg(b.tile_part + (int64_t)t * 32 + tid);
+                    // in tile order, 16 loads in flight (a scan has hundreds of tiles)
+                    int t = t0;
+                    for (; t + 16 <= t1; t += 16) {
+                        double v[16];
+#pragma unroll
+                        for (int u = 0; u < 16; ++u) v[u] = __ldcg(b.tile_part + (int64_t)(t + u) * 32 + tid);
+#pragma unroll
+                        for (int u = 0; u < 16; ++u) s += v[u];
+                    }
+                    for (; t < t1; ++t) s += __ldcg(b.tile_part + (int64_t)t * 32 + tid);
                     sv[tid] = s;
                 }
                 __syncthreads();
@@ -607,8 +870,8 @@ __global__ void __launch_bounds__(LOC_BLOCK, MINB)
         }
     }
     // evaluation (localize.py:182-205): points within each radius of their nearest map point, per hypothesis
-    for (;;) {
-        const int tile = next_tile(b, it_total, lane);
+    for (TileTaker take;;) {
+        const int tile = take.next(b, it_total, lane, grab);
         if (tile >= n_tiles) break;
         int h, lo, hi;
         tile_range(b, tile, n_hyp, h, lo, hi);
@@ -617,11 +880,16 @@ __global__ void __launch_bounds__(LOC_BLOCK, MINB)
         for (int k = 0; k < 12; ++k) M[k] = (float)__ldcg(b.T + 16 * h + k);
         int c0 = 0, c1 = 0, c2 = 0;
         const int end = min(hi, lo + la.tile);
+        const int64_t slot0 = (int64_t)tile * la.tile;
+        const int32_t* match = sorted ? ws.match + (int64_t)max(__ldg(b.hyp_tile + h), 0) * la.tile : nullptr;
         for (int i = lo + lane; i < end; i += 32) {
-            float4 p = __ldg(reinterpret_cast<const float4*>(b.pts) + i);
+            float4 p = __ldg(sorted ? reinterpret_cast<const float4*>(ws.sorted) + slot0 + (i - lo)
+                                    : reinterpret_cast<const float4*>(b.pts) + i);
             float wx, wy, wz;
             xform(M, p.x, p.y, p.z, wx, wy, wz);
-            int s = nearest_point(g, wx, wy, wz);
+            const int place = sorted ? __float_as_int(p.w) : -1;
+            const bool known = place >= 0 && (match - ws.match) + place < ws.cap;
+            int s = sorted ? nearest_warm(g, wx, wy, wz, known ? __ldcg(match + place) : -1, runs) : nearest_point(g, wx, wy, wz);
             if (s >= 0) {
                 const float4 q = ld_pt(reinterpret_cast<const float4*>(g.xyz), s);
                 float d = len3(wx - q.x, wy - q.y, wz - q.z);
@@ -1044,6 +1312,13 @@ void lw_score_yaw_table(int32_t n_yaw, float yaw0, float dyaw, float* c, float* 
 int lw_loc_icp_batch(const lw_prior_grid* g, lw_loc_batch* b, int32_t n_hyp, int32_t n_tiles, int32_t tile,
                      int32_t n_stages, const double* dmax, const int32_t* iters, float alpha, int32_t min_count,
                      int32_t blocks_per_sm, int32_t grid, void* stream) {
+    return lw_loc_icp_batch_ws(g, b, n_hyp, n_tiles, tile, n_stages, dmax, iters, alpha, min_count, blocks_per_sm, grid,
+                               nullptr, stream);
+}
+
+int lw_loc_icp_batch_ws(const lw_prior_grid* g, lw_loc_batch* b, int32_t n_hyp, int32_t n_tiles, int32_t tile,
+                        int32_t n_stages, const double* dmax, const int32_t* iters, float alpha, int32_t min_count,
+                        int32_t blocks_per_sm, int32_t grid, const lw_loc_ws* ws, void* stream) {
     int r = check_grid(g, "lw_loc_icp_batch");
     if (r != LW_OK) return r;
     if (!b || (n_stages > 0 && (!dmax || !iters)) || n_stages < 0 || n_stages > 8 || n_hyp < 1 || n_tiles < 1)
@@ -1091,7 +1366,24 @@ int lw_loc_icp_batch(const lw_prior_grid* g, lw_loc_batch* b, int32_t n_hyp, int
     if (grid <= 0 || grid > max_grid) grid = max_grid;
     if (grid > b->grid_cap) grid = b->grid_cap;
     ProfScope prof("loc_icp", s);
+    // one search per point repays the sorting only where it is repeated
+    lw_loc_ws w{};
+    if (ws && ws->sorted && ws->match && total_iters > 1) w = *ws;
+    if (((uintptr_t)w.sorted & 15) != 0)
+        return set_error(LW_EINVAL, "lw_loc_icp_batch_ws: the sorted points must be 16-byte aligned");
     k_loc_reset<<<16, 256, 0, s>>>(*b, n_hyp, total_iters);
+    if (w.sorted) {
+        static bool attr_set[64] = {};
+        int dev = 0;
+        LW_CUDA(cudaGetDevice(&dev));
+        if (dev < 0 || dev >= 64 || !attr_set[dev]) {
+            LW_CUDA(cudaFuncSetAttribute(k_loc_sort, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         LS_BOXES * (int)sizeof(int)));
+            if (dev >= 0 && dev < 64) attr_set[dev] = true;
+        }
+        k_loc_sort<<<n_hyp < 4 * sms ? n_hyp : 4 * sms, LS_T, LS_BOXES * sizeof(int), s>>>(*b, w, n_hyp, n_tiles, tile);
+        count_launches(1);
+    }
     // a cooperative launch (every CTA resident: the grid barriers rely on it), made through cudaLaunchKernelEx
     // so that it can also be captured into a CUDA graph
     cudaLaunchConfig_t cfg = {};
@@ -1105,11 +1397,11 @@ int lw_loc_icp_batch(const lw_prior_grid* g, lw_loc_batch* b, int32_t n_hyp, int
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     switch (blocks_per_sm) {
-        case 2: LW_CUDA(cudaLaunchKernelEx(&cfg, k_loc_icp<2>, *g, *b, la)); break;
-        case 3: LW_CUDA(cudaLaunchKernelEx(&cfg, k_loc_icp<3>, *g, *b, la)); break;
-        case 4: LW_CUDA(cudaLaunchKernelEx(&cfg, k_loc_icp<4>, *g, *b, la)); break;
-        case 5: LW_CUDA(cudaLaunchKernelEx(&cfg, k_loc_icp<5>, *g, *b, la)); break;
-        default: LW_CUDA(cudaLaunchKernelEx(&cfg, k_loc_icp<6>, *g, *b, la)); break;
+        case 2: LW_CUDA(cudaLaunchKernelEx(&cfg, k_loc_icp<2>, *g, *b, w, la)); break;
+        case 3: LW_CUDA(cudaLaunchKernelEx(&cfg, k_loc_icp<3>, *g, *b, w, la)); break;
+        case 4: LW_CUDA(cudaLaunchKernelEx(&cfg, k_loc_icp<4>, *g, *b, w, la)); break;
+        case 5: LW_CUDA(cudaLaunchKernelEx(&cfg, k_loc_icp<5>, *g, *b, w, la)); break;
+        default: LW_CUDA(cudaLaunchKernelEx(&cfg, k_loc_icp<6>, *g, *b, w, la)); break;
     }
     LW_LAUNCHED("lw_loc_icp_batch");
     count_launches(2);

@@ -127,6 +127,10 @@ class LocBatch(C.Structure):
     _fields_ = [(n, P) for n in PTRS] + [("pts_cap", i64), ("moved_cap", i32), ("grid_cap", i32)]
 
 
+class LocWs(C.Structure):
+    _fields_ = [("sorted", P), ("match", P), ("cap", i64)]
+
+
 SCORE_MAX_YAW = 1024  # headings lw_score_grid takes per launch (LW_SCORE_MAX_YAW)
 NET_P = 1024
 NET_OFF = {"W1": 0, "B1": 192, "W2": 256, "B2": 8448, "W3": 8576, "B3": 41344, "WH1": 41600, "BH1": 107136,
@@ -232,6 +236,8 @@ _SIGS = {
     "lw_score_maxima": (i32, [P, i32, i32, i32, i32, f32, i32, P, P, P, P]),
     "lw_loc_icp_batch": (i32, [C.POINTER(PriorGrid), C.POINTER(LocBatch), i32, i32, i32, i32, C.POINTER(f64),
                                C.POINTER(i32), f32, i32, i32, i32, P]),
+    "lw_loc_icp_batch_ws": (i32, [C.POINTER(PriorGrid), C.POINTER(LocBatch), i32, i32, i32, i32, C.POINTER(f64),
+                               C.POINTER(i32), f32, i32, i32, i32, C.POINTER(LocWs), P]),
 }
 
 _lib = None

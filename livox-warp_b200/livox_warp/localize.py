@@ -333,6 +333,11 @@ class LocBatch:
         self.moved = torch.zeros(self.ITERS_CAP, dtype=torch.int32, device=d)
         self.next = torch.zeros(self.ITERS_CAP + 1, dtype=torch.int32, device=d)
         self.bar = torch.zeros(2, dtype=torch.int32, device=d)
+        # every point of every tile, sorted by place, and its match (tiles of 32 points always fit)
+        slots = TILES[0] * NT
+        self.sorted = torch.empty((slots, 4), dtype=torch.float32, device=d)
+        self.match = torch.empty(slots, dtype=torch.int32, device=d)
+        self.ws = _lib.LocWs(_lib.ptr(self.sorted), _lib.ptr(self.match), slots)
         self.s = self._struct(dims=False)
         self.s_dims = self._struct(dims=True)
 
@@ -709,8 +714,9 @@ class GlobalLocalizer:
         b = self.batch
         dm = (_lib.f64 * max(1, len(schedule)))(*[float(d) for d, _ in schedule] or [0.0])
         it = (_lib.i32 * max(1, len(schedule)))(*[int(i) for _, i in schedule] or [0])
-        _lib.call("lw_loc_icp_batch", C.byref(self.grid.struct), C.byref(b.s_dims if dims else b.s), int(n_hyp),
-                  int(n_tiles), int(tile), len(schedule), dm, it, ALPHA, MIN_COUNT, int(minb), 0, _lib.stream_ptr(stream))
+        _lib.call("lw_loc_icp_batch_ws", C.byref(self.grid.struct), C.byref(b.s_dims if dims else b.s), int(n_hyp),
+                  int(n_tiles), int(tile), len(schedule), dm, it, ALPHA, MIN_COUNT, int(minb), 0, C.byref(b.ws),
+                  _lib.stream_ptr(stream))
 
     def _put_T(self, Ts, stream):
         b = self.batch
