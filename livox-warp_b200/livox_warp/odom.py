@@ -209,28 +209,24 @@ class Odometry:
     @property
     def traj(self) -> list:
         """(frame id, mid-frame time, 4x4 pose) of every finalised frame (the last TRAJ_CAP kept)."""
+        return [(int(r.k), float(r.t_mid), np.array(r.T, dtype=np.float64).reshape(4, 4)) for r in self._log()]
+
+    def _log(self) -> list:
+        """The trajectory log's records, oldest first (the last TRAJ_CAP kept); only what has been written is copied."""
         n = self.read_state().traj_len
         k = min(n, TRAJ_CAP)
         if k == 0:
             return []
+        size = ctypes.sizeof(_lib.TrajRec)
         with torch.cuda.stream(self.stream):
-            raw = self._traj.cpu().numpy().tobytes()
-        recs = (_lib.TrajRec * TRAJ_CAP).from_buffer_copy(raw)
-        out = []
-        for j in range(n - k, n):
-            r = recs[j % TRAJ_CAP]
-            out.append((int(r.k), float(r.t_mid), np.array(r.T, dtype=np.float64).reshape(4, 4)))
-        return out
+            raw = self._traj[:k * size].cpu().numpy()
+        recs = (_lib.TrajRec * k).from_buffer_copy(raw)
+        return [recs[j % TRAJ_CAP] for j in range(n - k, n)]
 
     def traj_records(self) -> list:
         """traj plus each frame's (ok, iters, corr)."""
-        n = self.read_state().traj_len
-        k = min(n, TRAJ_CAP)
-        with torch.cuda.stream(self.stream):
-            raw = self._traj.cpu().numpy().tobytes()
-        recs = (_lib.TrajRec * TRAJ_CAP).from_buffer_copy(raw)
         return [(int(r.k), float(r.t_mid), np.array(r.T).reshape(4, 4), int(r.ok), int(r.iters), int(r.corr))
-                for r in (recs[j % TRAJ_CAP] for j in range(n - k, n))]
+                for r in self._log()]
 
     @property
     def stats(self) -> dict:
@@ -459,13 +455,7 @@ class Odometry:
     def iteration_log(self) -> np.ndarray:
         """(k, iterations of the first registration, iterations of the last) of every logged frame that
         registered."""
-        n = self.read_state().traj_len
-        k = min(n, TRAJ_CAP)
-        with torch.cuda.stream(self.stream):
-            raw = self._traj.cpu().numpy().tobytes()
-        recs = (_lib.TrajRec * TRAJ_CAP).from_buffer_copy(raw)
-        rows = [(int(r.k), int(r.iters_first), int(r.iters)) for r in (recs[j % TRAJ_CAP] for j in range(n - k, n))
-                if r.ok and r.iters_first > 0]
+        rows = [(int(r.k), int(r.iters_first), int(r.iters)) for r in self._log() if r.ok and r.iters_first > 0]
         return np.array(rows, dtype=np.int64).reshape(-1, 3)
 
     def flush(self, on_frame=None):
