@@ -170,6 +170,11 @@ typedef struct lw_pose_table {
     int32_t* owner_epoch; /* [LW_POSE_SLOTS] */
 } lw_pose_table;
 
+/* A copy of the frame's deskewed points, attributes, times and frame ids -- the first min(*m_dev, m_ub) -- and of the count
+ * (device), so that the frame buffer may be filled again: xyz [m_ub*4] 16-byte aligned, attr, t, frame [m_ub], m [1]. */
+int lw_frame_copy(const lw_frame_buf* fb, const int32_t* m_dev, int64_t m_ub, float* xyz, uint32_t* attr, float* t,
+                  int32_t* frame, int32_t* m, void* stream);
+
 /* Append the staged points with k_min <= floor(max(t,0)/frame_dt) <= k_open to the open frame, in
  * staged order (odom.py:97-123, called from Odometry.push odom.py:626-638). xyz is [n*xyz_stride]. */
 int lw_frame_append(const float* xyz, int32_t xyz_stride, const uint32_t* attr, const float* t, int64_t n,
@@ -359,6 +364,12 @@ int lw_frame_ids(const float* t, int64_t n, float inv_dt, int32_t* out, void* st
  * inv_dt as lw_frame_ids does. Three copies and one launch, no host synchronisation. */
 int lw_stage_batch(const float* xyz_host, const uint32_t* attr_host, const float* t_host, int64_t n, float* xyz_dev,
                    uint32_t* attr_dev, float* t_dev, float inv_dt, int32_t* frame_dev, void* stream);
+
+/* Append n <= cap staged points to the live ring from slot `head` on, wrapping (gpu.py:1403-1419); xyz rows are 3 floats
+ * apart, or 4 and 16-byte aligned. */
+int lw_ring_append(const float* xyz, int32_t xyz_stride, const int32_t* attr, const float* t, const int32_t* frame, int64_t n,
+                   float* ring_xyz, int32_t* ring_attr, float* ring_t, int32_t* ring_frame, int64_t cap, int64_t head,
+                   void* stream);
 
 /* Buffers of the neighbourhood pass, contents undefined between calls: an open-addressed table of cap (a power of two)
  * slots for the bricks of 4 x 4 x 4 voxels that the points lie in (a call clears and uses the first power of two of

@@ -981,6 +981,42 @@ __global__ void k_frame_of(const float* __restrict__ t, int64_t n, float inv_dt,
         out[i] = inv_dt <= 0.0f ? 0 : (int)floorf(fmaxf(t[i], 0.0f) * inv_dt);
 }
 
+// Append n staged points to the live ring at `head` (gpu.py:1403-1419), one thread per point: five arrays' worth of indexed
+// copies and the index arithmetic were nine launches.
+template <int STRIDE>
+__global__ void k_ring_append(const float* __restrict__ xyz, const int32_t* __restrict__ attr, const float* __restrict__ t,
+                              const int32_t* __restrict__ frame, int64_t n, float* __restrict__ ring_xyz,
+                              int32_t* __restrict__ ring_attr, float* __restrict__ ring_t, int32_t* __restrict__ ring_frame,
+                              int64_t cap, int64_t head) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        int64_t j = head + i;
+        if (j >= cap) j -= cap;
+        float x, y, z;
+        load_xyz<STRIDE>(xyz, i, x, y, z);
+        ring_xyz[3 * j] = x;
+        ring_xyz[3 * j + 1] = y;
+        ring_xyz[3 * j + 2] = z;
+        ring_attr[j] = attr[i];
+        ring_t[j] = t[i];
+        ring_frame[j] = frame[i];
+    }
+}
+
+// A copy of a frame's first min(*m, m_ub) points and of the count, in one launch.
+__global__ void k_frame_copy(const float4* __restrict__ xyz, const uint32_t* __restrict__ attr, const float* __restrict__ t,
+                             const int32_t* __restrict__ frame, const int32_t* __restrict__ m, int64_t m_ub,
+                             float4* __restrict__ oxyz, uint32_t* __restrict__ oattr, float* __restrict__ ot,
+                             int32_t* __restrict__ oframe, int32_t* __restrict__ om) {
+    const int64_t n = min((int64_t)*m, m_ub);
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        oxyz[i] = xyz[i];
+        oattr[i] = attr[i];
+        ot[i] = t[i];
+        oframe[i] = frame[i];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *om = *m;
+}
+
 __global__ void k_map_clear(lw_map map) {
     for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < map.cap; s += (int64_t)gridDim.x * blockDim.x) {
         map.keys[s] = EMPTY_KEY;
@@ -1173,6 +1209,41 @@ int lw_stage_batch(const float* xyz_host, const uint32_t* attr_host, const float
     LW_CUDA(cudaMemcpyAsync(t_dev, t_host, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, s));
     k_frame_of<<<blocks_for(n, 256, 8 * device_sms()), 256, 0, s>>>(t_dev, n, inv_dt, frame_dev);
     LW_LAUNCHED("lw_stage_batch");
+    count_launches(1);
+    return LW_OK;
+}
+
+int lw_ring_append(const float* xyz, int32_t xyz_stride, const int32_t* attr, const float* t, const int32_t* frame, int64_t n,
+                   float* ring_xyz, int32_t* ring_attr, float* ring_t, int32_t* ring_frame, int64_t cap, int64_t head,
+                   void* stream) {
+    if (n < 0 || n > cap || head < 0 || (cap > 0 && head >= cap) || (xyz_stride != 3 && xyz_stride != 4))
+        return set_error(LW_EINVAL, "lw_ring_append: bad arguments");
+    if (n == 0) return LW_OK;
+    if (!xyz || !attr || !t || !frame || !ring_xyz || !ring_attr || !ring_t || !ring_frame)
+        return set_error(LW_EINVAL, "lw_ring_append: null argument");
+    if (xyz_stride == 4 && ((uintptr_t)xyz & 15) != 0)
+        return set_error(LW_EINVAL, "lw_ring_append: 4-float rows must be 16-byte aligned");
+    cudaStream_t s = (cudaStream_t)stream;
+    const int grid = blocks_for(n, 256, 8 * device_sms());
+    if (xyz_stride == 4)
+        k_ring_append<4><<<grid, 256, 0, s>>>(xyz, attr, t, frame, n, ring_xyz, ring_attr, ring_t, ring_frame, cap, head);
+    else
+        k_ring_append<3><<<grid, 256, 0, s>>>(xyz, attr, t, frame, n, ring_xyz, ring_attr, ring_t, ring_frame, cap, head);
+    LW_LAUNCHED("lw_ring_append");
+    count_launches(1);
+    return LW_OK;
+}
+
+int lw_frame_copy(const lw_frame_buf* fb, const int32_t* m_dev, int64_t m_ub, float* xyz, uint32_t* attr, float* t,
+                  int32_t* frame, int32_t* m, void* stream) {
+    if (!fb || !fb->f_xyz || !fb->f_attr || !fb->f_t || !fb->f_frame || !m_dev || !xyz || !attr || !t || !frame || !m ||
+        m_ub < 0)
+        return set_error(LW_EINVAL, "lw_frame_copy: bad arguments");
+    if (((uintptr_t)xyz & 15) != 0) return set_error(LW_EINVAL, "lw_frame_copy: xyz must be 16-byte aligned");
+    k_frame_copy<<<blocks_for(m_ub, 256, 4 * device_sms()), 256, 0, (cudaStream_t)stream>>>(
+        reinterpret_cast<const float4*>(fb->f_xyz), fb->f_attr, fb->f_t, fb->f_frame, m_dev, m_ub,
+        reinterpret_cast<float4*>(xyz), attr, t, frame, m);
+    LW_LAUNCHED("lw_frame_copy");
     count_launches(1);
     return LW_OK;
 }

@@ -200,6 +200,8 @@ _SIGS = {
     "lw_register_frame_host": (i32, [P, P, P, i64, f64, C.POINTER(f32), C.POINTER(f64), C.POINTER(OdomParams), P,
                                      C.POINTER(FrameBuf), C.POINTER(RegMap), C.POINTER(GnScratch), P, P, P]),
     "lw_map_insert": (i32, [P, i32, P, P, P, P, i64, P, C.POINTER(View), f32, C.POINTER(Map), P, P]),
+    "lw_ring_append": (i32, [P, i32, P, P, P, i64, P, P, P, P, i64, i64, P]),
+    "lw_frame_copy": (i32, [C.POINTER(FrameBuf), P, i64, P, P, P, P, P, P]),
     "lw_carve": (i32, [P, i32, P, P, P, i64, P, i32, f32, f32, i32, C.POINTER(Map), P, P]),
     "lw_carve_ws": (i32, [P, i32, P, P, P, i64, P, i32, f32, f32, i32, C.POINTER(Map), P, C.POINTER(CarveBuf), P]),
     "lw_map_build": (i32, [C.POINTER(Map), C.POINTER(View), i32, P, P, P, P, P, P, P]),

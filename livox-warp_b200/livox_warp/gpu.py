@@ -108,6 +108,12 @@ def row_stride(x: torch.Tensor) -> int:
     return s if x.stride(1) == 1 and s in (3, 4) and s >= x.shape[1] else 0
 
 
+def _plain(x, n: int, dtype) -> bool:
+    """Whether x holds at least n values one after another, 4 bytes each (of `dtype` when given)."""
+    return (x.dim() == 1 and x.shape[0] >= n and x.is_contiguous() and x.element_size() == 4
+            and (dtype is None or x.dtype == dtype))
+
+
 def _as_xyz(x, device) -> torch.Tensor:
     """Device float32 points of shape (n, 3) or (n, 4) (x, y, z, anything), contiguous, or the (n, 3) x, y, z
     columns of an (n, 4) buffer (rows 4 floats apart: the frame an on_frame callback is handed)."""
@@ -327,6 +333,18 @@ class Pipeline:
             return
         keep = min(n, self.cap)
         off = n - keep
+        stride = row_stride(sx)
+        if (stride and (stride == 3 or sx.data_ptr() % 16 == 0) and sx.shape[0] >= n
+                and sx.device == sa.device == st.device == sf.device == self.ring_xyz.device
+                and _plain(sa, n, None) and _plain(st, n, torch.float32) and _plain(sf, n, torch.int32)):
+            _lib.call("lw_ring_append", C.c_void_p(sx.data_ptr() + 4 * stride * off), stride,
+                      C.c_void_p(sa.data_ptr() + 4 * off), C.c_void_p(st.data_ptr() + 4 * off),
+                      C.c_void_p(sf.data_ptr() + 4 * off), keep, _lib.ptr(self.ring_xyz), _lib.ptr(self.ring_attr),
+                      _lib.ptr(self.ring_t), _lib.ptr(self.ring_frame), self.cap, self.head, _lib.stream_ptr())
+            self.head = (self.head + keep) % self.cap
+            self.filled = min(self.filled + keep, self.cap)
+            return
+        # tensors the kernel cannot read as they are (other strides, other types)
         idx = (torch.arange(keep, device=self.device) + self.head) % self.cap
         self.ring_xyz.index_copy_(0, idx, sx[off:n, :3])
         self.ring_attr.index_copy_(0, idx, sa[off:n].view(torch.int32))

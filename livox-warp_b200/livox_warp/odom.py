@@ -491,12 +491,9 @@ class Odometry:
                 self._snap_next ^= 1
                 if snap["done"] is not None:
                     self.stream.wait_event(snap["done"])  # the copy two frames back has been integrated
-                with torch.cuda.stream(self.stream):
-                    snap["xyz"][:m_ub].copy_(self.f_xyz[:m_ub])
-                    snap["attr"][:m_ub].copy_(self.f_attr[:m_ub])
-                    snap["t"][:m_ub].copy_(self.f_t[:m_ub])
-                    snap["frame"][:m_ub].copy_(self.f_frame[:m_ub])
-                    snap["m"].copy_(self._m_dev)
+                _lib.call("lw_frame_copy", _byref(self.fbuf), _lib.ptr(self._m_dev), m_ub, _lib.ptr(snap["xyz"]),
+                          _lib.ptr(snap["attr"]), _lib.ptr(snap["t"]), _lib.ptr(snap["frame"]), _lib.ptr(snap["m"]),
+                          self._sp())
                 snap["copied"].record(self.stream)
                 snap["m_ub"] = m_ub
                 self._pending = snap
