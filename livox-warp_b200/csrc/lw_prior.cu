@@ -56,10 +56,30 @@ __device__ __forceinline__ void key_unpack(int64_t key, int& ix, int& iy, int& i
 
 // ---- voxel downsample -------------------------------------------------------------------------------------------
 
+// 64 bytes of shared memory added to 64 of global memory as eight 64-bit integers, in one asynchronous operation; both
+// 16-byte aligned. The shared bytes are free again once bulk_read_wait returns.
+__device__ __forceinline__ void bulk_add8(int64_t* dst, const int64_t* src) {
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(src);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.u64 [%0], [%1], 64;" ::"l"(dst), "r"(at)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_read_wait() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
+constexpr int VX_CTA = 256;
+
 // Each point claims its voxel and adds its offset from the voxel centre, colour, intensity and 1 (k_vox_insert).
-template <int STRIDE>
-__global__ void k_vox_insert(const float* __restrict__ xyz, const float* __restrict__ inten,
-                             const float* __restrict__ rgb, int64_t n, VoxArgs a, lw_vox_buf vb) {
+// Bound by the L2's atomic units: eight 64-bit atomics a point kept 2.06 million points at 293 us. BULK hands a point's
+// eight sums over as one asynchronous 64-byte reduction, which the L2 does a sector at a time: 178 us. It needs `acc`
+// 16-byte aligned; other buffers take the atomics. `first` is read before its atomic minimum: points mostly come in
+// order, so a voxel's later ones need none (a value read can only be too high, and then the atomic decides).
+template <int STRIDE, bool BULK>
+__global__ void __launch_bounds__(VX_CTA) k_vox_insert(const float* __restrict__ xyz, const float* __restrict__ inten,
+                                                       const float* __restrict__ rgb, int64_t n, VoxArgs a, lw_vox_buf vb) {
+    __shared__ __align__(16) int64_t row[VX_CTA][8];
+    int64_t* const mine = row[threadIdx.x];
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         float x, y, z;
         ld3<STRIDE>(xyz, i, x, y, z);
@@ -71,19 +91,38 @@ __global__ void k_vox_insert(const float* __restrict__ xyz, const float* __restr
             atomicAdd((unsigned long long*)(vb.stats + 1), 1ull);
             continue;
         }
-        int64_t* acc = vb.acc + 8 * (int64_t)s;
-        atomic_add_i64(acc + 0, to_fix(x - vcentre(ix, a.voxel), a.fix_ofs));
-        atomic_add_i64(acc + 1, to_fix(y - vcentre(iy, a.voxel), a.fix_ofs));
-        atomic_add_i64(acc + 2, to_fix(z - vcentre(iz, a.voxel), a.fix_ofs));
+        int64_t v[8] = {to_fix(x - vcentre(ix, a.voxel), a.fix_ofs), to_fix(y - vcentre(iy, a.voxel), a.fix_ofs),
+                        to_fix(z - vcentre(iz, a.voxel), a.fix_ofs), 0, 0, 0, 0, 1};
         if (rgb) {
-            atomic_add_i64(acc + 3, to_fix(rgb[3 * i], VX_FIX_ATTR));
-            atomic_add_i64(acc + 4, to_fix(rgb[3 * i + 1], VX_FIX_ATTR));
-            atomic_add_i64(acc + 5, to_fix(rgb[3 * i + 2], VX_FIX_ATTR));
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v[3 + c] = to_fix(rgb[3 * i + c], VX_FIX_ATTR);
         }
-        if (inten) atomic_add_i64(acc + 6, to_fix(inten[i], VX_FIX_ATTR));
-        atomic_add_i64(acc + 7, 1);
-        atomicMin((unsigned long long*)(vb.first + s), (unsigned long long)(a.index0 + i));
+        if (inten) v[6] = to_fix(inten[i], VX_FIX_ATTR);
+        int64_t* const acc = vb.acc + 8 * (int64_t)s;
+        if (BULK) {
+            bulk_read_wait();
+#pragma unroll
+            for (int c = 0; c < 4; ++c) reinterpret_cast<longlong2*>(mine)[c] = make_longlong2(v[2 * c], v[2 * c + 1]);
+            bulk_add8(acc, mine);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+                if (v[c] != 0) atomic_add_i64(acc + c, v[c]);
+        }
+        const unsigned long long at = (unsigned long long)(a.index0 + i);
+        unsigned long long* const first = (unsigned long long*)(vb.first + s);
+        if (at < *(volatile unsigned long long*)first) atomicMin(first, at);
     }
+    if (BULK) bulk_wait();
+}
+
+template <int STRIDE>
+void vox_insert(const float* xyz, const float* inten, const float* rgb, int64_t n, const VoxArgs& a, const lw_vox_buf& vb,
+                int grid, cudaStream_t s) {
+    if (((uintptr_t)vb.acc & 15) == 0)
+        k_vox_insert<STRIDE, true><<<grid, VX_CTA, 0, s>>>(xyz, inten, rgb, n, a, vb);
+    else
+        k_vox_insert<STRIDE, false><<<grid, VX_CTA, 0, s>>>(xyz, inten, rgb, n, a, vb);
 }
 
 // A point opens a voxel when it is the voxel's first point; per tile of the chunk, how many do.
@@ -212,42 +251,162 @@ __global__ void k_pc_scatter(const float* __restrict__ xyz, int64_t n, lw_pca_bu
     }
 }
 
-// A thread per sorted position (k_normals): every point within the radius, found in the 27 cells around the
+// The sums over a point's neighbours: the offsets and products as 32-bit partial sums (rint_bits, rint_split), moved to
+// the 64-bit totals before they can overflow. A term is at most 2^20 units a part.
+constexpr int PN_CTA = 256;
+constexpr int PN_CELLS = 8;    // distinct cells whose runs a warp holds at a time
+constexpr int PN_QUEUE = 32;   // neighbours a lane may have waiting, a power of two
+constexpr int PN_STEP = 4;     // candidates per step
+constexpr int PN_DRAIN = 8;    // neighbours summed per drain
+constexpr int PN_FLUSH = 1000; // (PN_FLUSH + PN_DRAIN) 2^20 < 2^31
+
+struct PnSums {
+    long long s1[3] = {0, 0, 0}, s2[6] = {0, 0, 0, 0, 0, 0};
+    uint32_t p1[3] = {0, 0, 0}, hi[6] = {0, 0, 0, 0, 0, 0}, lo[6] = {0, 0, 0, 0, 0, 0};
+    int part = 0, n = 0;
+
+    __device__ __forceinline__ void flush() {
+        const uint32_t off = (uint32_t)part * (uint32_t)RINT_BITS;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            s1[j] += (int)(p1[j] - off);
+            p1[j] = 0;
+        }
+#pragma unroll
+        for (int j = 0; j < 6; ++j) {
+            s2[j] += (long long)(int)(hi[j] - off) * 1048576 + (int)(lo[j] - off);
+            hi[j] = lo[j] = 0;
+        }
+        part = 0;
+    }
+
+    __device__ __forceinline__ void add(float ex, float ey, float ez, const PcaArgs& a) {
+        ++n;
+        const float sum = ex + ey + ez;
+        if (sum != sum) {  // a NaN coordinate: what the conversion makes of it
+            const float e[3] = {ex, ey, ez};
+            const float ee[6] = {ex * ex, ex * ey, ex * ez, ey * ey, ey * ez, ez * ez};
+#pragma unroll
+            for (int j = 0; j < 3; ++j) s1[j] += to_fix(e[j], a.fd);
+#pragma unroll
+            for (int j = 0; j < 6; ++j) s2[j] += to_fix(ee[j], a.fdd);
+            return;
+        }
+        ++part;
+        // fd is a power of two and fdd its square, so the products of the scaled offsets are the scaled products
+        const float ux = ex * a.fd, uy = ey * a.fd, uz = ez * a.fd;
+        p1[0] += (uint32_t)rint_bits(ux);
+        p1[1] += (uint32_t)rint_bits(uy);
+        p1[2] += (uint32_t)rint_bits(uz);
+        const float w[6] = {ux * ux, ux * uy, ux * uz, uy * uy, uy * uz, uz * uz};
+#pragma unroll
+        for (int j = 0; j < 6; ++j) {
+            int h, l;
+            rint_split(w[j], h, l);
+            hi[j] += (uint32_t)h;
+            lo[j] += (uint32_t)l;
+        }
+    }
+};
+
+struct PnSmem {
+    int2 runs[PN_CTA / 32][PN_CELLS][27];
+    int queue[PN_CTA / 32][PN_QUEUE][32];
+};
+
+// A lane per sorted position (k_normals): every point within the radius, found in the 27 cells around the
 // point's own, adds 1, its offset and its offset's outer product in fixed point; then the covariance's
 // eigen-decomposition in float64, the smallest eigenvalue's vector and (l_mid - l_min) / l_max.
-__global__ void __launch_bounds__(256) k_pc_normals(PcaArgs a, lw_pca_buf pb, float* __restrict__ out_nrm,
-                                                    float* __restrict__ out_pl) {
+//
+// Bound by the instructions and their latency (0.56 issued a cycle and scheduler, 12,000 a warp of 32 points: about 40% the
+// float64 eigen-decomposition, a quarter the sums). Three things keep them down. A warp's 32 positions lie in a few cells (five, at seven points a
+// cell), whose 27 lookups are made by the warp's lanes at once, not by every lane for itself. The nine conversions of
+// a neighbour, each of them a quarter-rate instruction, are additions instead (rint_bits). And the candidates within the
+// radius, a third of them, wait in a queue per lane and are summed when most lanes have one: summing them on
+// sight runs the sums for every candidate that any lane accepts. 1.4 million points of a scanned floor, radius four voxels:
+// 1132 -> 883 us. 80 registers for three CTAs an SM: two take 1105 us, four (64 registers) 1050.
+__global__ void __launch_bounds__(PN_CTA, 3) k_pc_normals(PcaArgs a, lw_pca_buf pb, float* __restrict__ out_nrm,
+                                                       float* __restrict__ out_pl) {
+    __shared__ PnSmem sm;
     const int m = *pb.stats;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned full = 0xFFFFFFFFu;
     const float4* __restrict__ pts = reinterpret_cast<const float4*>(pb.sorted);
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < m; q += gridDim.x * blockDim.x) {
-        const float4 P = pts[q];
+    for (int base = (blockIdx.x * PN_CTA + threadIdx.x) & ~31; base < m; base += gridDim.x * PN_CTA) {
+        const int q = base + lane;
+        const bool act = q < m;
+        const float4 P = pts[act ? q : m - 1];
         const int i = __float_as_int(P.w);
         const int ix = ifloor(P.x * a.inv_h), iy = ifloor(P.y * a.inv_h), iz = ifloor(P.z * a.inv_h);
-        int n = 0;
-        long long s1[3] = {0, 0, 0}, s2[6] = {0, 0, 0, 0, 0, 0};
-#pragma unroll 1
-        for (int c = 0; c < 27; ++c) {
-            const int s = find_slot<VX_PROBES>(key_ijk(ix + c / 9 - 1, iy + (c / 3) % 3 - 1, iz + c % 3 - 1),
-                                               pb.keys, a.mask);
-            if (s < 0) continue;
-            const int k0 = __ldg(pb.cell_start + s), k1 = k0 + __ldg(pb.cell_cnt + s);
-#pragma unroll 1
-            for (int k = k0; k < k1; ++k) {
-                const float4 Q = __ldg(pts + k);
-                const float ex = Q.x - P.x, ey = Q.y - P.y, ez = Q.z - P.z;
-                if (ex * ex + ey * ey + ez * ez > a.r2) continue;
-                ++n;
-                s1[0] += to_fix(ex, a.fd);
-                s1[1] += to_fix(ey, a.fd);
-                s1[2] += to_fix(ez, a.fd);
-                s2[0] += to_fix(ex * ex, a.fdd);
-                s2[1] += to_fix(ex * ey, a.fdd);
-                s2[2] += to_fix(ex * ez, a.fdd);
-                s2[3] += to_fix(ey * ey, a.fdd);
-                s2[4] += to_fix(ey * ez, a.fdd);
-                s2[5] += to_fix(ez * ez, a.fdd);
+        // the warp's distinct cells: positions are sorted by cell, so each is a run of lanes
+        const int px = __shfl_up_sync(full, ix, 1), py = __shfl_up_sync(full, iy, 1), pz = __shfl_up_sync(full, iz, 1);
+        unsigned heads = __ballot_sync(full, lane == 0 || px != ix || py != iy || pz != iz);
+        const int cells = __popc(heads), mine = __popc(heads & (full >> (31 - lane))) - 1;
+        PnSums S;
+        for (int c0 = 0; c0 < cells; c0 += PN_CELLS) {
+            const int nc = min(PN_CELLS, cells - c0);
+            int left = 0, r = 0;
+            for (int c = 0; c < nc; ++c) {
+                const int leader = __ffs(heads) - 1;
+                heads &= heads - 1;
+                const int cx = __shfl_sync(full, ix, leader), cy = __shfl_sync(full, iy, leader);
+                const int cz = __shfl_sync(full, iz, leader);
+                int s = -1;
+                if (lane < 27)
+                    s = find_slot<VX_PROBES>(key_ijk(cx + lane / 9 - 1, cy + (lane / 3) % 3 - 1, cz + lane % 3 - 1),
+                                             pb.keys, a.mask);
+                const unsigned occ = __ballot_sync(full, s >= 0);
+                if (s >= 0) {
+                    const int k0 = __ldg(pb.cell_start + s);
+                    sm.runs[warp][c][__popc(occ & ((1u << lane) - 1))] = make_int2(k0, k0 + __ldg(pb.cell_cnt + s));
+                }
+                if (mine == c0 + c) left = __popc(occ);
             }
+            __syncwarp();
+            if (!act) left = 0;
+            const int2* __restrict__ run = sm.runs[warp][mine - c0 >= 0 && mine - c0 < PN_CELLS ? mine - c0 : 0];
+            int k = 0, e = 0, put = 0, got = 0;
+            for (;;) {
+                if (k >= e && r < left) {
+                    const int2 v = run[r++];
+                    k = v.x;
+                    e = v.y;
+                }
+                const bool more = __any_sync(full, k < e);
+                if (more) {
+                    float4 Q[PN_STEP];
+#pragma unroll
+                    for (int u = 0; u < PN_STEP; ++u) Q[u] = __ldg(pts + min(k + u, m - 1));
+#pragma unroll
+                    for (int u = 0; u < PN_STEP; ++u) {
+                        const float ex = Q[u].x - P.x, ey = Q[u].y - P.y, ez = Q[u].z - P.z;
+                        if (k + u < e && !(ex * ex + ey * ey + ez * ez > a.r2)) {
+                            sm.queue[warp][put & (PN_QUEUE - 1)][lane] = k + u;
+                            ++put;
+                        }
+                    }
+                    k += PN_STEP;
+                }
+                // sum once some lane's queue could overflow, when most have a neighbour waiting
+                while (__any_sync(full, put - got > (more ? PN_QUEUE - 2 * PN_STEP : 0))) {
+#pragma unroll 2
+                    for (int u = 0; u < PN_DRAIN; ++u)
+                        if (got < put) {
+                            const float4 Q = __ldg(pts + sm.queue[warp][got & (PN_QUEUE - 1)][lane]);
+                            ++got;
+                            S.add(Q.x - P.x, Q.y - P.y, Q.z - P.z, a);
+                        }
+                    if (S.part >= PN_FLUSH) S.flush();
+                }
+                if (!more) break;
+            }
+            __syncwarp();
         }
+        S.flush();
+        if (!act) continue;
+        const int n = S.n;
+        const long long(&s1)[3] = S.s1;
+        const long long(&s2)[6] = S.s2;
         if (n < 4) {  // prior_map.py:151-154
             out_nrm[3 * (int64_t)i] = out_nrm[3 * (int64_t)i + 1] = out_nrm[3 * (int64_t)i + 2] = 0.0f;
             out_pl[i] = 0.0f;
@@ -336,11 +495,11 @@ int lw_vox_insert(lw_vox_buf* vb, const float* xyz, int32_t xyz_stride, const fl
     a.mask = (int)(vb->cap - 1);
     a.index0 = index0;
     const int sms = device_sms();
-    const int grid = blocks_for(n, 256, 16 * sms);
+    const int grid = blocks_for(n, VX_CTA, 16 * sms);
     if (xyz_stride == 4)
-        k_vox_insert<4><<<grid, 256, 0, s>>>(xyz, intensity, rgb, n, a, *vb);
+        vox_insert<4>(xyz, intensity, rgb, n, a, *vb, grid, s);
     else
-        k_vox_insert<3><<<grid, 256, 0, s>>>(xyz, intensity, rgb, n, a, *vb);
+        vox_insert<3>(xyz, intensity, rgb, n, a, *vb, grid, s);
     const int nt = blocks_for(n, VX_TILE);
     k_vox_count<<<nt, VX_TILE, 0, s>>>(n, index0, *vb);
     k_scan_from<int64_t><<<1, 1024, 0, s>>>(vb->tiles, nt, vb->stats);
@@ -412,7 +571,7 @@ int lw_normals(const float* xyz, int32_t xyz_stride, int64_t n, float radius, lw
         k_pc_scatter<4><<<grid, 256, 0, s>>>(xyz, n, *pb, out_nrm, out_planarity);
     else
         k_pc_scatter<3><<<grid, 256, 0, s>>>(xyz, n, *pb, out_nrm, out_planarity);
-    k_pc_normals<<<blocks_for(n, 256, 16 * sms), 256, 0, s>>>(a, *pb, out_nrm, out_planarity);
+    k_pc_normals<<<blocks_for(n, PN_CTA, 16 * sms), PN_CTA, 0, s>>>(a, *pb, out_nrm, out_planarity);
     LW_LAUNCHED("lw_normals");
     count_launches(6);
     return LW_OK;
