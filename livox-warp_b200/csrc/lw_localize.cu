@@ -982,20 +982,218 @@ __device__ __forceinline__ float soft_count(int n_in, int sum_d2, float tau) {
 // r = SC_POS (32 rg + lane) + j, j < SC_POS, at one heading; the warps of a CTA take consecutive headings. When
 // positions ip and ip + stride are neighbours along x with the same y and z (stride = ny for a meshgrid with y
 // inner), a warp's posed copies of a point differ only in x -- one row of the x-fastest distance field, a few
-// cache lines per gather -- and a thread's positions share the rotated offsets, the posed y and z, their cells and
-// the row; only the x chain is per position (the kernel is issue-bound, so this removes most of its work). A
-// thread whose positions straddle two (y, z) rows (the end of one x run and the start of the next) keeps a second
-// row; one with more, or with rows that are not x runs, takes the general path. Each hypothesis' score is the
-// same whatever the layout. Two positions per thread and six CTAs per SM: on the office coarse search (28M
-// hypotheses x 1024 points) 34.2 ms, against 42.6 / 63.1 ms for four / eight positions at three CTAs per SM and
-// 37.3 ms for one position (more resident warps keep more gathers in flight).
+// cache lines per gather. Each hypothesis' score is the same whatever the layout.
+//
+// The kernel is bound by the instructions it issues, so what a warp's positions share is worked out once: a warp's
+// positions lie in few (y, z) rows (one or two where the x runs are long), and for each row and each of 16 points one lane
+// computes the rotated offsets, the posed y and z, their cells and the row's address, into shared memory. What is left
+// per position and point is the x chain, two positions to a packed instruction, with the floor taken by one addition that
+// rounds down (sc_cell) instead of a quarter-rate conversion. Rows outside the grid and dead positions get an x far outside
+// it and need no test of their own. 3.5M hypotheses x 1024 points of an office: 4.87 -> 2.27 ms, at 88% of the issue slots.
+// A warp whose positions are spread over many rows (list order along y) gains nothing from the table: its hypotheses are
+// left to k_score_rest, and so are all of them when a point is not finite. Four CTAs an SM and eight points in flight:
+// five CTAs take 2.33 ms; positions 32 apart in a thread, 2.4; branches around the gathers, 4.0.
 constexpr int SC_POS = 2;
+constexpr int SC_ROWS = 8;        // (y, z) rows a warp keeps
+constexpr int SC_TAB = 16;        // points per table
+constexpr float SC_FAR = 1.0e30f; // an x outside every grid
+constexpr float SC_HUGE = 1.0e18f;
+constexpr int SC_MAX_NX = 1 << 22;
+constexpr float SC_PENDING = -3.0e38f;  // no score: scores are -1 or more
 
-template <bool WIDE>
-__global__ void __launch_bounds__(SC_THREADS, 6) k_score_grid(lw_prior_grid g, const float* __restrict__ pts, int n_pts,
+struct ScoreRow {
+    float ax, bx;        // the rotated offset's two x terms
+    const uint8_t* row;  // the distance field's row
+};
+
+__device__ __forceinline__ uint64_t f2_pack(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_add_down(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// The cells of two posed x's: floor(f) for f in [-2^22, 2^22), because f + 1.5 x 2^23 rounded down is floor(f) + 1.5 x 2^23
+// there; for any other f, infinities included, a number of 2^22 or more.
+__device__ __forceinline__ uint2 sc_cell(uint64_t wx, uint64_t neg_origin, uint64_t inv_cell) {
+    const uint64_t f = f2_mul(f2_add(wx, neg_origin), inv_cell);
+    const uint64_t t = f2_add_down(f, f2_pack(RINT_MAGIC, RINT_MAGIC));
+    uint2 u;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(u.x), "=r"(u.y) : "l"(t));
+    return make_uint2(u.x - (uint32_t)RINT_BITS, u.y - (uint32_t)RINT_BITS);
+}
+
+// SC_TAB points against a thread's two positions. SAME: both lie in the row e0.
+template <bool SAME>
+__device__ __forceinline__ void score_rows(const ScoreRow* e0, const ScoreRow* e1, int m, uint64_t cx, uint64_t neg_origin,
+                                           uint64_t inv_cell, uint32_t nx, int tau_ceil, int (&n_in)[SC_POS],
+                                           int (&sum_d2)[SC_POS]) {
+#pragma unroll 8
+    for (int k = 0; k < m; ++k) {
+        const float4 v0 = *reinterpret_cast<const float4*>(e0 + k);
+        const float4 v1 = SAME ? v0 : *reinterpret_cast<const float4*>(e1 + k);
+        const uint64_t wx = f2_add(f2_add(cx, f2_pack(v0.x, v1.x)), f2_pack(v0.y, v1.y));
+        const uint2 u = sc_cell(wx, neg_origin, inv_cell);
+        const uint64_t r0 = f2_pack(v0.z, v0.w), r1 = SAME ? r0 : f2_pack(v1.z, v1.w);
+        int d0 = 1024, d1 = 1024;
+        if (u.x < nx) d0 = __ldg(reinterpret_cast<const uint8_t*>(r0) + u.x);
+        if (u.y < nx) d1 = __ldg(reinterpret_cast<const uint8_t*>(r1) + u.y);
+        if (d0 < tau_ceil) {  // d < tau for a whole number of cm
+            ++n_in[0];
+            sum_d2[0] += d0 * d0;
+        }
+        if (d1 < tau_ceil) {
+            ++n_in[1];
+            sum_d2[1] += d1 * d1;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(SC_THREADS, 4) k_score_grid(const __grid_constant__ lw_prior_grid g,
+                                                           const float* __restrict__ pts, int n_pts,
                                                            const float* __restrict__ pos, int64_t n_pos,
                                                            int64_t stride, int64_t n_rg, int n_yaw,
                                                            const YawTab yt, float tau, int tau_ceil, float free_cm,
+                                                           float* __restrict__ out) {
+    static_assert(SC_POS == 2, "a thread's positions are one pair");
+    __shared__ float px[SC_CHUNK], py[SC_CHUNK], pz[SC_CHUNK];
+    __shared__ __align__(16) ScoreRow tab[SC_THREADS / 32][SC_ROWS][SC_TAB + 1];  // + 1: rows start in different banks
+    const unsigned full = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int iyaw = (int)(wid % n_yaw);
+    const int64_t q = wid / n_yaw;
+    const int64_t c = q / n_rg, r0 = ((q - c * n_rg) * 32 + lane) * SC_POS;
+    const float co = yt.c[iyaw], si = yt.s[iyaw];
+    float cx[SC_POS], cy[SC_POS], cz[SC_POS];
+    bool live[SC_POS];
+    int row[SC_POS];
+#pragma unroll
+    for (int j = 0; j < SC_POS; ++j) {
+        const int64_t ip = c + stride * (r0 + j);
+        live[j] = c < stride && ip < n_pos;
+        row[j] = -1;
+        cx[j] = SC_FAR;
+        cy[j] = cz[j] = 0.f;
+        if (live[j]) {
+            const float x = pos[3 * ip], y = pos[3 * ip + 1], z = pos[3 * ip + 2];
+            int ix, iy, iz;
+            grid_idx(g, x, y, z, ix, iy, iz);
+            const int64_t cc = grid_flat(g, ix, iy, iz);
+            // the sensor outside the grid or inside a mapped surface
+            if (cc < 0 || (float)g.df[cc] < free_cm) {
+                out[ip * n_yaw + iyaw] = -1.0f;
+                live[j] = false;
+            } else {
+                cx[j] = x;
+                cy[j] = y;
+                cz[j] = z;
+            }
+        }
+    }
+    // the warp's distinct (y, z), lane k keeping row k's
+    float ty = 0.f, tz = 0.f;
+    int rows = 0;
+    const bool plain = g.nx <= SC_MAX_NX;
+    for (; rows < SC_ROWS && plain; ++rows) {
+        bool open[SC_POS];
+#pragma unroll
+        for (int j = 0; j < SC_POS; ++j)
+            open[j] = live[j] && row[j] < 0 && fabsf(cx[j]) < SC_HUGE && fabsf(cy[j]) < SC_HUGE && fabsf(cz[j]) < SC_HUGE;
+        const unsigned w = __ballot_sync(full, open[0] || open[1]);
+        if (w == 0) break;
+        const int from = __ffs(w) - 1;
+        const float y = __shfl_sync(full, open[0] ? cy[0] : cy[1], from);
+        const float z = __shfl_sync(full, open[0] ? cz[0] : cz[1], from);
+#pragma unroll
+        for (int j = 0; j < SC_POS; ++j)
+            if (open[j] && cy[j] == y && cz[j] == z) row[j] = rows;
+        if (lane == rows) {
+            ty = y;
+            tz = z;
+        }
+    }
+    // positions left over, one not finite, or rows of fewer than eight positions: k_score_rest
+    const int positions = __popc(__ballot_sync(full, live[0])) + __popc(__ballot_sync(full, live[1]));
+    bool fits = __all_sync(full, (!live[0] || row[0] >= 0) && (!live[1] || row[1] >= 0)) &&
+                (rows <= 2 || 8 * rows <= positions);
+    const bool any0 = row[0] >= 0, any1 = row[1] >= 0;
+    const bool same = __all_sync(full, row[0] == row[1] || !any0 || !any1);
+    const int s0 = any0 ? row[0] : (any1 ? row[1] : 0), s1 = any1 ? row[1] : s0;
+    const uint64_t cx2 = f2_pack(any0 ? cx[0] : SC_FAR, any1 ? cx[1] : SC_FAR);
+    const uint64_t neg_origin = f2_pack(-g.origin[0], -g.origin[0]), inv_cell = f2_pack(g.inv_cell, g.inv_cell);
+    int n_in[SC_POS], sum_d2[SC_POS];
+#pragma unroll
+    for (int j = 0; j < SC_POS; ++j) n_in[j] = sum_d2[j] = 0;
+    for (int base = 0; base < n_pts; base += SC_CHUNK) {
+        const int m = min(SC_CHUNK, n_pts - base);
+        __syncthreads();
+        stage_pts(pts, base, m, px, py, pz);
+        bool odd = false;
+        for (int k = threadIdx.x; k < m; k += blockDim.x)
+            odd |= !(fabsf(px[k]) < SC_HUGE && fabsf(py[k]) < SC_HUGE && fabsf(pz[k]) < SC_HUGE);
+        if (__syncthreads_or(odd)) {
+            fits = false;
+            break;
+        }
+        if (fits) {
+            for (int k0 = 0; k0 < m && rows > 0; k0 += SC_TAB) {
+                const int n = min(SC_TAB, m - k0);
+                __syncwarp();
+                for (int r = 0; r < rows; r += 2) {  // 16 points of two rows at a time
+                    const int mine = r + (lane >> 4), k = lane & (SC_TAB - 1);
+                    const float y = __shfl_sync(full, ty, mine & 31), z = __shfl_sync(full, tz, mine & 31);
+                    if (mine < rows && k < n) {
+                        // the reference's expressions (localize.py:89)
+                        const float x0 = px[k0 + k], y0 = py[k0 + k];
+                        const float wy = y + si * x0 + co * y0, wz = z + pz[k0 + k];
+                        const int iy = ifloor((wy - g.origin[1]) * g.inv_cell);
+                        const int iz = ifloor((wz - g.origin[2]) * g.inv_cell);
+                        const bool in = iy >= 0 && iz >= 0 && iy < g.ny && iz < g.nz;
+                        ScoreRow e;
+                        e.ax = in ? co * x0 : SC_FAR;
+                        e.bx = -(si * y0);
+                        e.row = g.df + (in ? ((int64_t)iz * g.ny + iy) * (int64_t)g.nx : 0);
+                        tab[warp][mine][k] = e;
+                    }
+                }
+                __syncwarp();
+                if (same)
+                    score_rows<true>(tab[warp][s0], tab[warp][s0], n, cx2, neg_origin, inv_cell, (uint32_t)g.nx, tau_ceil,
+                                     n_in, sum_d2);
+                else
+                    score_rows<false>(tab[warp][s0], tab[warp][s1], n, cx2, neg_origin, inv_cell, (uint32_t)g.nx, tau_ceil,
+                                      n_in, sum_d2);
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < SC_POS; ++j)
+        if (live[j]) out[(c + stride * (r0 + j)) * n_yaw + iyaw] = fits ? soft_count(n_in[j], sum_d2[j], tau) : SC_PENDING;
+}
+
+// The hypotheses k_score_grid left pending, in the same layout, each thread working out its own row or two: six CTAs an SM
+// of it hide the gathers better than a second way through k_score_grid would (1.00 against 1.34 ms for 0.6M hypotheses x
+// 1024 points in list order).
+template <bool WIDE>
+__global__ void __launch_bounds__(SC_THREADS, 6) k_score_rest(lw_prior_grid g, const float* __restrict__ pts, int n_pts,
+                                                           const float* __restrict__ pos, int64_t n_pos,
+                                                           int64_t stride, int64_t n_rg, int n_yaw,
+                                                           const YawTab yt, float tau, int tau_ceil,
                                                            float* __restrict__ out) {
     using idx_t = typename std::conditional<WIDE, int64_t, int32_t>::type;
     __shared__ float px[SC_CHUNK], py[SC_CHUNK], pz[SC_CHUNK];
@@ -1008,41 +1206,29 @@ __global__ void __launch_bounds__(SC_THREADS, 6) k_score_grid(lw_prior_grid g, c
     float cx[SC_POS];
     bool live[SC_POS], in_b[SC_POS];
     float ya = 0.f, za = 0.f, yb = 0.f, zb = 0.f;
-    int rows = 0;  // distinct (y, z) among the live positions: 0, 1, 2, or 3 for "more"
+    int rows = 0;  // distinct (y, z) among the live positions
 #pragma unroll
     for (int j = 0; j < SC_POS; ++j) {
         const int64_t ip = c + stride * (r0 + j);
-        live[j] = c < stride && ip < n_pos;
+        live[j] = c < stride && ip < n_pos && out[ip * n_yaw + iyaw] == SC_PENDING;
         in_b[j] = false;
         cx[j] = 0.f;
         if (live[j]) {
             const float x = pos[3 * ip], y = pos[3 * ip + 1], z = pos[3 * ip + 2];
-            int ix, iy, iz;
-            grid_idx(g, x, y, z, ix, iy, iz);
-            const int64_t cc = grid_flat(g, ix, iy, iz);
-            // the sensor outside the grid or inside a mapped surface
-            if (cc < 0 || (float)g.df[cc] < free_cm) {
-                out[ip * n_yaw + iyaw] = -1.0f;
-                live[j] = false;
-            } else {
-                cx[j] = x;
-                if (rows == 0) {
-                    ya = y;
-                    za = z;
-                    rows = 1;
-                } else if (y != ya || z != za) {
-                    if (rows == 1) {
-                        yb = y;
-                        zb = z;
-                        rows = 2;
-                    } else if (y != yb || z != zb) {
-                        rows = 3;
-                    }
-                    in_b[j] = rows == 2 && y == yb && z == zb;
-                }
+            cx[j] = x;
+            if (rows == 0) {
+                ya = y;
+                za = z;
+                rows = 1;
+            } else if (y != ya || z != za) {
+                yb = y;
+                zb = z;
+                rows = 2;
+                in_b[j] = y == yb && z == zb;
             }
         }
     }
+    if (!__syncthreads_or(rows > 0)) return;
     int n_in[SC_POS], sum_d2[SC_POS];
 #pragma unroll
     for (int j = 0; j < SC_POS; ++j) n_in[j] = sum_d2[j] = 0;
@@ -1053,51 +1239,42 @@ __global__ void __launch_bounds__(SC_THREADS, 6) k_score_grid(lw_prior_grid g, c
         stage_pts(pts, base, m, px, py, pz);
         __syncthreads();
         if (rows == 0) continue;
-        if (rows <= 2) {
 #pragma unroll 2
-            for (int k = 0; k < m; ++k) {
-                // the reference's expressions (localize.py:89), the shared parts once per row
-                const float ax = co * px[k], bx = si * py[k], ey = si * px[k], fy = co * py[k];
-                const float wya = ya + ey + fy, wza = za + pz[k];
-                const int iya = ifloor((wya - g.origin[1]) * g.inv_cell), iza = ifloor((wza - g.origin[2]) * g.inv_cell);
-                const bool oka = iya >= 0 && iza >= 0 && iya < g.ny && iza < g.nz;
-                const idx_t rowa = ((idx_t)iza * g.ny + iya) * (idx_t)g.nx;
-                idx_t rowb = 0;
-                bool okb = false;
-                if (rows == 2) {
-                    const float wyb = yb + ey + fy, wzb = zb + pz[k];
-                    const int iyb = ifloor((wyb - g.origin[1]) * g.inv_cell), izb = ifloor((wzb - g.origin[2]) * g.inv_cell);
-                    okb = iyb >= 0 && izb >= 0 && iyb < g.ny && izb < g.nz;
-                    rowb = ((idx_t)izb * g.ny + iyb) * (idx_t)g.nx;
-                }
+        for (int k = 0; k < m; ++k) {
+            // the reference's expressions (localize.py:89), the shared parts once per row
+            const float ax = co * px[k], bx = si * py[k], ey = si * px[k], fy = co * py[k];
+            const float wya = ya + ey + fy, wza = za + pz[k];
+            const int iya = ifloor((wya - g.origin[1]) * g.inv_cell), iza = ifloor((wza - g.origin[2]) * g.inv_cell);
+            const bool oka = iya >= 0 && iza >= 0 && iya < g.ny && iza < g.nz;
+            const idx_t rowa = ((idx_t)iza * g.ny + iya) * (idx_t)g.nx;
+            idx_t rowb = 0;
+            bool okb = false;
+            if (rows == 2) {
+                const float wyb = yb + ey + fy, wzb = zb + pz[k];
+                const int iyb = ifloor((wyb - g.origin[1]) * g.inv_cell), izb = ifloor((wzb - g.origin[2]) * g.inv_cell);
+                okb = iyb >= 0 && izb >= 0 && iyb < g.ny && izb < g.nz;
+                rowb = ((idx_t)izb * g.ny + iyb) * (idx_t)g.nx;
+            }
 #pragma unroll
-                for (int j = 0; j < SC_POS; ++j) {
-                    const float wx = cx[j] + ax - bx;
-                    const int ix = ifloor((wx - g.origin[0]) * g.inv_cell);
-                    const bool ok = in_b[j] ? okb : oka;
-                    if (live[j] && ok && ix >= 0 && ix < g.nx) {
-                        const int d = __ldg(df + (in_b[j] ? rowb : rowa) + ix);
-                        if (d < tau_ceil) {  // d < tau for a whole number of cm
-                            ++n_in[j];
-                            sum_d2[j] += d * d;
-                        }
+            for (int j = 0; j < SC_POS; ++j) {
+                const float wx = cx[j] + ax - bx;
+                const int ix = ifloor((wx - g.origin[0]) * g.inv_cell);
+                const bool ok = in_b[j] ? okb : oka;
+                if (live[j] && ok && ix >= 0 && ix < g.nx) {
+                    const int d = __ldg(df + (in_b[j] ? rowb : rowa) + ix);
+                    if (d < tau_ceil) {  // d < tau for a whole number of cm
+                        ++n_in[j];
+                        sum_d2[j] += d * d;
                     }
                 }
             }
-        } else {
-#pragma unroll
-            for (int j = 0; j < SC_POS; ++j)
-                if (live[j]) {
-                    const int64_t ip = c + stride * (r0 + j);
-                    score_chunk(g, px, py, pz, m, cx[j], pos[3 * ip + 1], pos[3 * ip + 2], co, si, tau, n_in[j],
-                                sum_d2[j]);
-                }
         }
     }
 #pragma unroll
     for (int j = 0; j < SC_POS; ++j)
         if (live[j]) out[(c + stride * (r0 + j)) * n_yaw + iyaw] = soft_count(n_in[j], sum_d2[j], tau);
 }
+
 
 // Local maxima of the coarse scores (localize.py:450-483, _local_maxima): hypothesis h = ((iz nx + ix) ny + iy)
 // n_yaw + iyaw is one when its score is positive, at least min_score, and no less than any of its 26 neighbours in
@@ -1256,14 +1433,16 @@ int lw_score_grid(const lw_prior_grid* g, const float* pts, int32_t n_pts, const
     lw_score_yaw_table(n_yaw, yaw0, dyaw, yt.c, yt.s);
     const int tau_ceil = tau_cm > 1024.0f ? 1024 : (int)ceilf(tau_cm);  // distances are whole cm in [0, 255]
     const unsigned blocks = (unsigned)((threads + SC_THREADS - 1) / SC_THREADS);
+    k_score_grid<<<blocks, SC_THREADS, 0, (cudaStream_t)stream>>>(*g, pts, n_pts, pos, n_pos, stride, n_rg, n_yaw, yt, tau_cm,
+                                                                  tau_ceil, free_cm, out);
     if (g->ncell < 0x7FFFFFFF)
-        k_score_grid<false><<<blocks, SC_THREADS, 0, (cudaStream_t)stream>>>(*g, pts, n_pts, pos, n_pos, stride, n_rg,
-                                                                              n_yaw, yt, tau_cm, tau_ceil, free_cm, out);
+        k_score_rest<false><<<blocks, SC_THREADS, 0, (cudaStream_t)stream>>>(*g, pts, n_pts, pos, n_pos, stride, n_rg, n_yaw,
+                                                                             yt, tau_cm, tau_ceil, out);
     else
-        k_score_grid<true><<<blocks, SC_THREADS, 0, (cudaStream_t)stream>>>(*g, pts, n_pts, pos, n_pos, stride, n_rg,
-                                                                             n_yaw, yt, tau_cm, tau_ceil, free_cm, out);
+        k_score_rest<true><<<blocks, SC_THREADS, 0, (cudaStream_t)stream>>>(*g, pts, n_pts, pos, n_pos, stride, n_rg, n_yaw,
+                                                                            yt, tau_cm, tau_ceil, out);
     LW_LAUNCHED("lw_score_grid");
-    count_launches(1);
+    count_launches(2);
     return LW_OK;
 }
 
@@ -1409,3 +1588,4 @@ int lw_loc_icp_batch_ws(const lw_prior_grid* g, lw_loc_batch* b, int32_t n_hyp, 
 }
 
 }  // extern "C"
+
