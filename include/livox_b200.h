@@ -322,11 +322,12 @@ int lw_carve(const float* xyz, int32_t xyz_stride, const uint32_t* attr, const i
              const int32_t* n_dev, int64_t n_ub, const float* poses, int32_t every, float inv_voxel,
              float max_range, int32_t max_steps, lw_map* map, float* ray_stop, void* stream);
 
-/* Workspace of lw_carve_ws, contents undefined between calls: (ray, occupied voxel) pairs, the distinct voxels met and their
+/* Workspace of lw_carve_ws, contents undefined between calls: (ray, occupied voxel) pairs and their times, the distinct voxels met and their
  * planes. Pairs or voxels beyond the capacities are handled without the workspace (slower, same misses); about 16
  * pairs and 4 voxels per ray hold an indoor frame. planes is 16-byte aligned. */
 typedef struct lw_carve_buf {
     int64_t* pairs;   /* [pair_cap] */
+    float* times;     /* [pair_cap] when the pair's ray meets its voxel */
     float* planes;    /* [8 * slot_cap] */
     int32_t* slots;   /* [slot_cap] */
     int64_t* counts;  /* [3] */

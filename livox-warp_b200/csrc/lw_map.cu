@@ -301,35 +301,41 @@ __device__ __forceinline__ bool carve_ray(const float* __restrict__ xyz, const u
     return true;
 }
 
-// Carving, pass 1 (gpu.py:469-495): one thread per ray finds where the ray stops -- short of its end point by a
-// margin that grows at grazing incidence on the end point's local plane -- in voxel units; 0 when not carved.
+// Where a ray stops (gpu.py:469-495), in voxel units: short of its end point by a margin, which carve_margin gives without
+// and ray_stop_at with its growth at grazing incidence on the end point's local plane (never less than without).
+__device__ __forceinline__ float carve_margin(float L, float voxel) {
+    return fmaxf(CARVE_MARGIN_VOXELS * voxel, CARVE_MARGIN_FRACTION * L);
+}
+
+template <int STRIDE>
+__device__ __forceinline__ float ray_stop_at(const float* __restrict__ xyz, const uint32_t* __restrict__ attr,
+                                             const int32_t* __restrict__ frame, const float* __restrict__ poses, int64_t i,
+                                             float inv_voxel, float max_range, const lw_map& map) {
+    float ox, oy, oz, wx, wy, wz, dx, dy, dz, L;
+    if (!carve_ray<STRIDE>(xyz, attr, frame, poses, i, max_range, ox, oy, oz, wx, wy, wz, dx, dy, dz, L)) return 0.0f;
+    const float voxel = 1.0f / inv_voxel;
+    float margin = carve_margin(L, voxel);
+    const float4 pe = local_plane(ifloor(wx * inv_voxel), ifloor(wy * inv_voxel), ifloor(wz * inv_voxel), wx, wy, wz, map,
+                                  (int)(map.cap - 1));
+    if (pe.w > 0.5f) {
+        float cosine = fabsf(pe.x * dx + pe.y * dy + pe.z * dz);
+        margin = fmaxf(margin, CARVE_GRAZING_VOXELS * voxel / fmaxf(cosine, CARVE_MIN_COSINE));
+    }
+    return (L - margin) * inv_voxel;
+}
+
+// Carving, pass 1: one thread per ray; 0 when not carved.
 template <int STRIDE>
 __global__ void k_carve_setup(const float* __restrict__ xyz, const uint32_t* __restrict__ attr,
                               const int32_t* __restrict__ frame, const int* n_dev, int64_t n_ub,
                               const float* __restrict__ poses, int every, float inv_voxel, float max_range, lw_map map,
-                              float* __restrict__ ray_stop, int64_t* __restrict__ counts) {
-    if (counts && blockIdx.x == 0 && threadIdx.x < 3) counts[threadIdx.x] = 0;
+                              float* __restrict__ ray_stop) {
     int64_t n = n_dev ? (int64_t)*n_dev : n_ub;
     if (n > n_ub) n = n_ub;
-    const int mask = (int)(map.cap - 1);
     const int64_t nrays = (n + every - 1) / every;
-    const float voxel = 1.0f / inv_voxel;
     for (int64_t ray = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; ray < nrays;
-         ray += (int64_t)gridDim.x * blockDim.x) {
-        float ox, oy, oz, wx, wy, wz, dx, dy, dz, L;
-        float stop = 0.0f;
-        if (carve_ray<STRIDE>(xyz, attr, frame, poses, ray * every, max_range, ox, oy, oz, wx, wy, wz, dx, dy, dz, L)) {
-            float margin = fmaxf(CARVE_MARGIN_VOXELS * voxel, CARVE_MARGIN_FRACTION * L);
-            const float4 pe = local_plane(ifloor(wx * inv_voxel), ifloor(wy * inv_voxel), ifloor(wz * inv_voxel), wx,
-                                          wy, wz, map, mask);
-            if (pe.w > 0.5f) {
-                float cosine = fabsf(pe.x * dx + pe.y * dy + pe.z * dz);
-                margin = fmaxf(margin, CARVE_GRAZING_VOXELS * voxel / fmaxf(cosine, CARVE_MIN_COSINE));
-            }
-            stop = (L - margin) * inv_voxel;
-        }
-        ray_stop[ray] = stop;
-    }
+         ray += (int64_t)gridDim.x * blockDim.x)
+        ray_stop[ray] = ray_stop_at<STRIDE>(xyz, attr, frame, poses, ray * every, inv_voxel, max_range, map);
 }
 
 // Whether the ray from o along d pierces the voxel with centroid c and local plane pl (gpu.py:563-591): it crosses the
@@ -451,8 +457,11 @@ __global__ void __launch_bounds__(128) k_carve(const float* __restrict__ xyz, co
 // Carving with a workspace. The plane of an occupied voxel is a function of the map alone, which carving does not
 // change (only the miss counters grow), but k_carve fits it again for every ray that meets the voxel: a 27-voxel gather
 // and a float64 eigen-decomposition on the one lane that met it, with its warp waiting. Here the walk only notes
-// which occupied voxels each ray meets; each distinct one is fitted once, a thread each, and a last pass tests the
-// noted (ray, voxel) pairs. The same float operations on the same values, so the misses are k_carve's bit for bit.
+// which occupied voxels each ray meets, and when; each distinct one is fitted once, a thread each; and a last pass tests
+// the noted (ray, voxel) pairs. The walk goes to the stop that the margin has without the end point's plane, which is never
+// short of the true one; the end points' planes are fitted beside the voxels' -- each fit is a chain of dependent float64
+// operations that takes 22 us however few there are -- and the pairs past a ray's true stop are dropped. The same float
+// operations on the same values, so the misses are k_carve's bit for bit.
 //
 // Walk: CW_PARTS lanes per ray, each walking an equal stretch of its length. The times at which a ray crosses the voxel
 // faces of one axis are a running sum that no other axis enters, and the DDA takes the three axes' crossings in
@@ -462,7 +471,8 @@ __global__ void __launch_bounds__(128) k_carve(const float* __restrict__ xyz, co
 // adding-up is repeated). A warp gathers its pairs in shared memory (one atomic on the pair count per warp, not
 // per round of probes: 22 us). map.bcnt, zero between calls, marks a voxel as met and then holds its place among
 // the distinct ones plus one; the last CTA of the pair pass zeroes it again.
-// For 10,000 rays the four passes take 22 + 14 + 21 + 7 us where k_carve's two took 22 + 175.
+// For 10,000 rays the three passes take 15 + 24 + 9 us where k_carve's two took 22 + 175, and a pass of its own for the stops 22 + 14 +
+// 21 + 7.
 constexpr int CW_PARTS = 4, CW_DEEP = 8, CW_THREADS = 128;
 constexpr int CW_QUEUE = 512;  // pairs a warp gathers before it writes them out
 
@@ -472,11 +482,13 @@ __device__ __forceinline__ void key_voxel(int64_t key, int& ix, int& iy, int& iz
     iz = (int)((key >> 42) & KEY_MASK) - (int)KEY_BIAS;
 }
 
-// Whether a (ray, voxel) pair's voxel is pierced, with its plane fitted here (the lists were full).
+// Whether a (ray, voxel) pair's voxel, met at `when`, is pierced, with its planes fitted here (the lists were full).
 template <int STRIDE>
 __device__ __noinline__ bool carve_alone(const float* __restrict__ xyz, const uint32_t* __restrict__ attr,
                                          const int32_t* __restrict__ frame, const float* __restrict__ poses, int64_t pair,
-                                         int every, float inv_voxel, float max_range, const lw_map& map) {
+                                         float when, int every, float inv_voxel, float max_range, const lw_map& map) {
+    const float stop = ray_stop_at<STRIDE>(xyz, attr, frame, poses, (pair >> 32) * every, inv_voxel, max_range, map);
+    if (!(stop > 1.0f && when < stop)) return false;
     float ox, oy, oz, wx, wy, wz, dx, dy, dz, L;
     carve_ray<STRIDE>(xyz, attr, frame, poses, (pair >> 32) * every, max_range, ox, oy, oz, wx, wy, wz, dx, dy, dz, L);
     const int s = (int)(pair & 0xffffffff);
@@ -492,7 +504,7 @@ template <int STRIDE>
 __global__ void __launch_bounds__(CW_THREADS) k_carve_walk(
     const float* __restrict__ xyz, const uint32_t* __restrict__ attr, const int32_t* __restrict__ frame,
     const int* n_dev, int64_t n_ub, const float* __restrict__ poses, int every, float inv_voxel, float max_range,
-    int max_steps, lw_map map, const float* __restrict__ ray_stop, lw_carve_buf cb) {
+    int max_steps, lw_map map, lw_carve_buf cb) {
     int64_t n = n_dev ? (int64_t)*n_dev : n_ub;
     if (n > n_ub) n = n_ub;
     const int mask = (int)(map.cap - 1);
@@ -502,7 +514,9 @@ __global__ void __launch_bounds__(CW_THREADS) k_carve_walk(
     constexpr int RAYS = 32 / CW_PARTS;  // of a warp
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     __shared__ int64_t queues[CW_THREADS / 32][CW_QUEUE];
+    __shared__ float queue_t[CW_THREADS / 32][CW_QUEUE];
     int64_t* queue = queues[threadIdx.x >> 5];  // the pairs this warp has met and not written out yet
+    float* when = queue_t[threadIdx.x >> 5];    // and when
     int queued = 0;
     // write the queued pairs out, and list the voxels that no ray had met before
     auto flush = [&]() {
@@ -519,8 +533,10 @@ __global__ void __launch_bounds__(CW_THREADS) k_carve_walk(
                 s = (int)(pair & 0xffffffff);
                 if (p + i0 + lane < cb.pair_cap) {
                     cb.pairs[p + i0 + lane] = pair;
+                    cb.times[p + i0 + lane] = when[i0 + lane];
                     first = *(volatile int*)(map.bcnt + s) == 0 && atomicExch(map.bcnt + s, 1) == 0;
-                } else if (carve_alone<STRIDE>(xyz, attr, frame, poses, pair, every, inv_voxel, max_range, map)) {
+                } else if (carve_alone<STRIDE>(xyz, attr, frame, poses, pair, when[i0 + lane], every, inv_voxel,
+                                               max_range, map)) {
                     atomicAdd(map.miss + s, every);
                 }
             }
@@ -541,10 +557,13 @@ __global__ void __launch_bounds__(CW_THREADS) k_carve_walk(
     };
     for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * RAYS < nrays; w += nwarps) {
         const int64_t ray = w * RAYS + lane / CW_PARTS;
-        float stop = ray < nrays ? ray_stop[ray] : 0.0f;
-        bool on = stop > 1.0f;
-        float ox = 0.f, oy = 0.f, oz = 0.f, wx, wy, wz, dx = 0.f, dy = 0.f, dz = 0.f, L;
-        if (on) carve_ray<STRIDE>(xyz, attr, frame, poses, ray * every, max_range, ox, oy, oz, wx, wy, wz, dx, dy, dz, L);
+        float ox = 0.f, oy = 0.f, oz = 0.f, wx, wy, wz, dx = 0.f, dy = 0.f, dz = 0.f, L, stop = 0.0f;
+        bool on = false;
+        if (ray < nrays &&
+            carve_ray<STRIDE>(xyz, attr, frame, poses, ray * every, max_range, ox, oy, oz, wx, wy, wz, dx, dy, dz, L)) {
+            stop = (L - carve_margin(L, 1.0f / inv_voxel)) * inv_voxel;
+            on = stop > 1.0f;
+        }
         const float posx = ox * inv_voxel, posy = oy * inv_voxel, posz = oz * inv_voxel;
         int ix = ifloor(posx), iy = ifloor(posy), iz = ifloor(posz);
         int sx = 1, sy = 1, sz = 1;
@@ -615,6 +634,7 @@ __global__ void __launch_bounds__(CW_THREADS) k_carve_walk(
         while (true) {
             int64_t key[CW_DEEP], got[CW_DEEP];
             int h[CW_DEEP];
+            float at_t[CW_DEEP];
 #pragma unroll
             for (int k = 0; k < CW_DEEP; ++k) {
                 // the next crossing; on ties z before y before x, as the comparisons x < y && x < z, y < z have it
@@ -631,6 +651,7 @@ __global__ void __launch_bounds__(CW_THREADS) k_carve_walk(
                 tmy = by ? tmy + tdy : tmy;
                 tmz = bz ? tmz + tdz : tmz;
                 key[k] = at;
+                at_t[k] = t;
                 h[k] = slot_hash(at) & mask;
                 got[k] = on ? __ldg(map.keys + h[k]) : EMPTY_KEY;
             }
@@ -666,7 +687,10 @@ __global__ void __launch_bounds__(CW_THREADS) k_carve_walk(
 #pragma unroll
                 for (int k = 0; k < CW_DEEP; ++k) {
                     const unsigned hits = __ballot_sync(0xffffffffu, cnt[k] > 0);
-                    if (cnt[k] > 0) queue[queued + __popc(hits & below)] = (ray << 32) | (int64_t)s[k];
+                    if (cnt[k] > 0) {
+                        queue[queued + __popc(hits & below)] = (ray << 32) | (int64_t)s[k];
+                        when[queued + __popc(hits & below)] = at_t[k];
+                    }
                     queued += __popc(hits);
                 }
             }
@@ -676,12 +700,26 @@ __global__ void __launch_bounds__(CW_THREADS) k_carve_walk(
     }
 }
 
-// The voxels met, a thread each: centroid in planes[2 p], local plane in planes[2 p + 1].
-__global__ void __launch_bounds__(64) k_carve_planes(lw_map map, lw_carve_buf cb) {
+// The rays' stops and the voxels met, a thread each: centroid in planes[2 p], local plane in planes[2 p + 1].
+template <int STRIDE>
+__global__ void __launch_bounds__(64) k_carve_planes(const float* __restrict__ xyz, const uint32_t* __restrict__ attr,
+                                                     const int32_t* __restrict__ frame, const int* n_dev, int64_t n_ub,
+                                                     const float* __restrict__ poses, int every, float inv_voxel,
+                                                     float max_range, lw_map map, float* __restrict__ ray_stop,
+                                                     lw_carve_buf cb) {
+    int64_t n = n_dev ? (int64_t)*n_dev : n_ub;
+    if (n > n_ub) n = n_ub;
+    const int64_t rays = ((n + every - 1) / every + 31) & ~(int64_t)31;  // whole warps of either
     const int64_t m = min(cb.counts[1], cb.slot_cap);
     const int mask = (int)(map.cap - 1);
     float4* __restrict__ out = reinterpret_cast<float4*>(cb.planes);
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < m; p += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rays + m; i += (int64_t)gridDim.x * blockDim.x) {
+        if (i < rays) {
+            if (i * every < n)
+                ray_stop[i] = ray_stop_at<STRIDE>(xyz, attr, frame, poses, i * every, inv_voxel, max_range, map);
+            continue;
+        }
+        const int64_t p = i - rays;
         const int s = cb.slots[p];
         int ix, iy, iz;
         key_voxel(map.keys[s], ix, iy, iz);
@@ -698,7 +736,7 @@ template <int STRIDE>
 __global__ void __launch_bounds__(256) k_carve_pairs(const float* __restrict__ xyz, const uint32_t* __restrict__ attr,
                                                      const int32_t* __restrict__ frame, const float* __restrict__ poses,
                                                      int every, float inv_voxel, float max_range, lw_map map,
-                                                     lw_carve_buf cb) {
+                                                     const float* __restrict__ ray_stop, lw_carve_buf cb) {
     __shared__ int last;
     const int64_t np = min(cb.counts[0], cb.pair_cap);
     const float voxel = 1.0f / inv_voxel;
@@ -706,6 +744,8 @@ __global__ void __launch_bounds__(256) k_carve_pairs(const float* __restrict__ x
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < np; p += (int64_t)gridDim.x * blockDim.x) {
         const int64_t pair = cb.pairs[p];
         const int s = (int)(pair & 0xffffffff);
+        const float stop = ray_stop[pair >> 32];
+        if (!(stop > 1.0f && cb.times[p] < stop)) continue;
         const int q = map.bcnt[s];
         bool hit;
         if (q > 0) {
@@ -715,7 +755,7 @@ __global__ void __launch_bounds__(256) k_carve_pairs(const float* __restrict__ x
             const float4 c = __ldg(planes + 2 * (int64_t)(q - 1));
             hit = pierces(c.x, c.y, c.z, __ldg(planes + 2 * (int64_t)(q - 1) + 1), ox, oy, oz, dx, dy, dz, voxel);
         } else {
-            hit = carve_alone<STRIDE>(xyz, attr, frame, poses, pair, every, inv_voxel, max_range, map);
+            hit = carve_alone<STRIDE>(xyz, attr, frame, poses, pair, cb.times[p], every, inv_voxel, max_range, map);
         }
         if (hit) atomicAdd(map.miss + s, every);
     }
@@ -1087,12 +1127,12 @@ int lw_carve(const float* xyz, int32_t xyz_stride, const uint32_t* attr, const i
     ProfScope prof("carve", s);
     if (xyz_stride == 4) {
         k_carve_setup<4><<<grid1, 64, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range, *map,
-                                              ray_stop, nullptr);
+                                              ray_stop);
         k_carve<4><<<grid, 128, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range, max_steps,
                                         *map, ray_stop);
     } else {
         k_carve_setup<3><<<grid1, 64, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range, *map,
-                                              ray_stop, nullptr);
+                                              ray_stop);
         k_carve<3><<<grid, 128, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range, max_steps,
                                         *map, ray_stop);
     }
@@ -1108,7 +1148,7 @@ int lw_carve_ws(const float* xyz, int32_t xyz_stride, const uint32_t* attr, cons
     if (r != LW_OK) return r;
     if (!xyz || !attr || !frame || !poses || !ray_stop || (xyz_stride != 3 && xyz_stride != 4))
         return set_error(LW_EINVAL, "lw_carve_ws: bad arguments");
-    if (!cb || !cb->pairs || !cb->planes || !cb->slots || !cb->counts || cb->pair_cap < 0 || cb->slot_cap < 0 ||
+    if (!cb || !cb->pairs || !cb->times || !cb->planes || !cb->slots || !cb->counts || cb->pair_cap < 0 || cb->slot_cap < 0 ||
         cb->slot_cap >= 0x7FFFFFFF || ((uintptr_t)cb->planes & 15) != 0)
         return set_error(LW_EINVAL, "lw_carve_ws: incomplete workspace");
     if (n_ub > 0x7FFFFFFF) return set_error(LW_ECAPACITY, "lw_carve_ws: more than 2^31 - 1 points");
@@ -1117,28 +1157,25 @@ int lw_carve_ws(const float* xyz, int32_t xyz_stride, const uint32_t* attr, cons
     cudaStream_t s = (cudaStream_t)stream;
     const int64_t rays = (n_ub + every - 1) / every;
     const int sms = device_sms();
-    const int grid1 = blocks_for(rays, 64, 16 * sms);                 // a thread per ray
     const int grid2 = blocks_for(rays * CW_PARTS, CW_THREADS, 16 * sms);
-    const int grid3 = blocks_for(rays, 64, 8 * sms);                  // a thread per distinct voxel met
+    const int grid3 = blocks_for(2 * rays, 64, 16 * sms);             // a thread per ray and per distinct voxel met
     const int grid4 = blocks_for(4 * rays, 256, 4 * sms);             // a thread per pair
     ProfScope prof("carve", s);
-    if (xyz_stride == 4) {
-        k_carve_setup<4><<<grid1, 64, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range, *map,
-                                              ray_stop, cb->counts);
-        k_carve_walk<4><<<grid2, CW_THREADS, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range,
-                                              max_steps, *map, ray_stop, *cb);
-        k_carve_planes<<<grid3, 64, 0, s>>>(*map, *cb);
-        k_carve_pairs<4><<<grid4, 256, 0, s>>>(xyz, attr, frame, poses, every, inv_voxel, max_range, *map, *cb);
-    } else {
-        k_carve_setup<3><<<grid1, 64, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range, *map,
-                                              ray_stop, cb->counts);
-        k_carve_walk<3><<<grid2, CW_THREADS, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range,
-                                              max_steps, *map, ray_stop, *cb);
-        k_carve_planes<<<grid3, 64, 0, s>>>(*map, *cb);
-        k_carve_pairs<3><<<grid4, 256, 0, s>>>(xyz, attr, frame, poses, every, inv_voxel, max_range, *map, *cb);
-    }
+    LW_CUDA(cudaMemsetAsync(cb->counts, 0, 3 * sizeof(int64_t), s));
+    auto run = [&](auto stride) {
+        constexpr int S = decltype(stride)::value;
+        k_carve_walk<S><<<grid2, CW_THREADS, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range,
+                                                     max_steps, *map, *cb);
+        k_carve_planes<S><<<grid3, 64, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range, *map,
+                                               ray_stop, *cb);
+        k_carve_pairs<S><<<grid4, 256, 0, s>>>(xyz, attr, frame, poses, every, inv_voxel, max_range, *map, ray_stop, *cb);
+    };
+    if (xyz_stride == 4)
+        run(std::integral_constant<int, 4>{});
+    else
+        run(std::integral_constant<int, 3>{});
     LW_LAUNCHED("lw_carve_ws");
-    count_launches(4);
+    count_launches(3);
     return LW_OK;
 }
 

@@ -87,7 +87,7 @@ class Map(C.Structure):
 
 
 class CarveBuf(C.Structure):
-    PTRS = ("pairs", "planes", "slots", "counts")
+    PTRS = ("pairs", "times", "planes", "slots", "counts")
     _fields_ = [(n, P) for n in PTRS] + [("pair_cap", i64), ("slot_cap", i64)]
 
 

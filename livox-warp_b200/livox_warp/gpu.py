@@ -390,7 +390,8 @@ class Pipeline:
         if rays > self._carve_rays:
             r = 1 << (rays - 1).bit_length()
             pairs, slots, d = 16 * r, min(4 * r, self.map_cap), self.device
-            t = (torch.empty(pairs, dtype=torch.int64, device=d), torch.empty((slots, 8), dtype=torch.float32, device=d),
+            t = (torch.empty(pairs, dtype=torch.int64, device=d), torch.empty(pairs, dtype=torch.float32, device=d),
+                 torch.empty((slots, 8), dtype=torch.float32, device=d),
                  torch.empty(slots, dtype=torch.int32, device=d), torch.zeros(3, dtype=torch.int64, device=d))
             self._carve_t.append(t)
             self._carve_buf = _lib.CarveBuf(*(_lib.ptr(x) for x in t), pairs, slots)

@@ -80,6 +80,7 @@ def _compare(mapped, n, every, max_steps, pairs, slots):
     n = min(n, len(sf))
     stop = torch.zeros(max(n, 1), dtype=torch.float32, device="cuda")
     bufs = (torch.empty(max(pairs, 1), dtype=torch.int64, device="cuda"),
+            torch.empty(max(pairs, 1), dtype=torch.float32, device="cuda"),
             torch.empty((max(slots, 1), 8), dtype=torch.float32, device="cuda"),
             torch.empty(max(slots, 1), dtype=torch.int32, device="cuda"),
             torch.full((3,), 99, dtype=torch.int64, device="cuda"))
