@@ -645,15 +645,19 @@ __device__ __forceinline__ float warp_reduce_scatter32(float (&v)[32], int lane)
 
 // The tiles of pass `pass` for the calling warp, taken `grab` at a time (one atomic, broadcast to the warp). A tile per atomic
 // made the atomics on the one counter, about 3 ns each, take as long as the searches themselves: 0.26 ms for 88,000
-// tiles; a grab of a quarter of a warp's share still evens out tiles of uneven work.
+// tiles. A grab is a quarter of a warp's share, and the last quarter of the tiles goes out singly, so that no warp is a
+// whole grab behind at the barrier: 256 scans 13.4 -> 12.9 ms (singles for the last tenth 13.2, five eighths 13.0, pairs
+// 13.2).
 struct TileTaker {
     int t = 0, left = 0;
-    __device__ __forceinline__ int next(const lw_loc_batch& b, int pass, int lane, int grab) {
+    __device__ __forceinline__ int next(const lw_loc_batch& b, int pass, int lane, int grab, int n_tiles) {
         if (left == 0) {
             int v = 0;
-            if (lane == 0) v = atomicAdd(b.next + pass, grab);
-            t = __shfl_sync(FULL, v, 0);
-            left = grab;
+            if (lane == 0) v = atomicAdd(b.next + pass, 1);
+            v = __shfl_sync(FULL, v, 0);
+            const int big = (int)((int64_t)n_tiles * 3 / 4) / grab;
+            t = v < big ? v * grab : big * grab + (v - big);
+            left = v < big ? grab : 1;
         }
         --left;
         return t++;
@@ -727,9 +731,10 @@ __global__ void __launch_bounds__(LS_T) k_loc_sort(lw_loc_batch b, lw_loc_ws ws,
 // are neighbours (k_loc_sort) -- scans come in the order they were fired, whose 32 points lie in as many places: a
 // quarter of the loads hit L1 and half the lanes idled -- starting from the point's match of the iteration before; the
 // terms are then summed from the matches in the scan's own order, so that every sum and pose is the one without a workspace,
-// bit for bit. 256 scans of 2,000-20,000 points, 31 iterations: 13.3 ms, 23.1 without; an iteration is 0.19-0.35 ms of searches
+// bit for bit. 256 scans of 2,000-20,000 points, 31 iterations: 12.8 ms, 23.1 without; an iteration is 0.19-0.35 ms of searches
 // (bound by L1's one line a cycle: every lane's loads are lines of their own, about 570 a tile), 0.08 of sums, 0.03 of
-// the tile partials' sums and solves, 0.1 of waiting at the three barriers.
+// the tile partials' sums and solves, 0.08 of waiting at the three barriers. The sorted points are read past L1, which
+// the map's lines need.
 template <int MINB>
 __global__ void __launch_bounds__(LOC_BLOCK, MINB)
     k_loc_icp(lw_prior_grid g, lw_loc_batch b, lw_loc_ws ws, LocArgs la) {
@@ -758,7 +763,7 @@ __global__ void __launch_bounds__(LOC_BLOCK, MINB)
             // does not depend on which warp computed it, so the sums of phase B are deterministic.
             if (sorted) {
                 for (TileTaker take;;) {
-                    const int tile = take.next(b, it_total, lane, grab);
+                    const int tile = take.next(b, it_total, lane, grab, n_tiles);
                     if (tile >= n_tiles) break;
                     int h, lo, hi;
                     tile_range(b, tile, n_hyp, h, lo, hi);
@@ -771,7 +776,7 @@ __global__ void __launch_bounds__(LOC_BLOCK, MINB)
                     int32_t* match = ws.match + (int64_t)max(__ldg(b.hyp_tile + h), 0) * la.tile;
                     const int count = min(hi - lo, la.tile);
                     for (int i = lane; i < count; i += 32) {
-                        const float4 p = __ldg(reinterpret_cast<const float4*>(ws.sorted) + slot0 + i);
+                        const float4 p = __ldcs(reinterpret_cast<const float4*>(ws.sorted) + slot0 + i);
                         const int place = __float_as_int(p.w);
                         if (place < 0 || (match - ws.match) + place >= ws.cap) continue;  // tables that do not fit together
                         int32_t* m = match + place;
@@ -787,7 +792,7 @@ __global__ void __launch_bounds__(LOC_BLOCK, MINB)
             TileTaker take;
             for (int turn = warp_id;; turn += n_warps) {
                 // the sums alone are even work: tiles in turn; with the searches in them tiles go to the next free warp
-                const int tile = sorted ? turn : take.next(b, it_total, lane, grab);
+                const int tile = sorted ? turn : take.next(b, it_total, lane, grab, n_tiles);
                 if (tile >= n_tiles) break;
                 int h, lo, hi;
                 tile_range(b, tile, n_hyp, h, lo, hi);
@@ -839,14 +844,14 @@ __global__ void __launch_bounds__(LOC_BLOCK, MINB)
                 const int t0 = max(b.hyp_tile[h], 0), t1 = min(b.hyp_tile[h + 1], n_tiles);
                 if (tid < LTERMS) {
                     double s = 0.0;
-                    // in tile order, 16 loads in flight (a scan has hundreds of tiles)
+                    // in tile order, 32 loads in flight (a scan has hundreds of tiles)
                     int t = t0;
-                    for (; t + 16 <= t1; t += 16) {
-                        double v[16];
+                    for (; t + 32 <= t1; t += 32) {
+                        double v[32];
 #pragma unroll
-                        for (int u = 0; u < 16; ++u) v[u] = __ldcg(b.tile_part + (int64_t)(t + u) * 32 + tid);
+                        for (int u = 0; u < 32; ++u) v[u] = __ldcg(b.tile_part + (int64_t)(t + u) * 32 + tid);
 #pragma unroll
-                        for (int u = 0; u < 16; ++u) s += v[u];
+                        for (int u = 0; u < 32; ++u) s += v[u];
                     }
                     for (; t < t1; ++t) s += __ldcg(b.tile_part + (int64_t)t * 32 + tid);
                     sv[tid] = s;
@@ -871,7 +876,7 @@ __global__ void __launch_bounds__(LOC_BLOCK, MINB)
     }
     // evaluation (localize.py:182-205): points within each radius of their nearest map point, per hypothesis
     for (TileTaker take;;) {
-        const int tile = take.next(b, it_total, lane, grab);
+        const int tile = take.next(b, it_total, lane, grab, n_tiles);
         if (tile >= n_tiles) break;
         int h, lo, hi;
         tile_range(b, tile, n_hyp, h, lo, hi);
