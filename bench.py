@@ -368,8 +368,9 @@ def pose_drift(odom, traj, oracle_poses: dict) -> dict:
 
 # DRAM bytes (read + write) per launch from one ncu capture of the sequence (profiles/k_gn_k_carve_sequence.md,
 # rounded as summarised there) and of the coarse search (profiles/k_score_grid_office_coarse.md)
-SEQ_TRAFFIC = {"gn": 2_186_752, "carve": 6_774_848}  # gn: thinning + iterations (mean of two full launches); carve: setup + walk
-SEQ_TRAFFIC_SRC = "ncu dram__bytes_read.sum + dram__bytes_write.sum, profiles/k_gn_k_carve_sequence.md"
+SEQ_TRAFFIC = {"gn": 2_186_752, "carve": 6_870_400}  # gn: thinning + iterations; carve: walk + planes + pairs (means of two)
+SEQ_TRAFFIC_SRC = ("ncu dram__bytes_read.sum + dram__bytes_write.sum, profiles/k_gn_k_carve_sequence.md (gn), "
+                   "profiles/k_carve_passes.md (carve)")
 SINGLE_TRAFFIC = {"gn": 1_387_776}  # ncu, one timed launch of the single-frame case (1,387,520 B read, 256 written)
 SINGLE_TRAFFIC_SRC = "ncu dram__bytes_read.sum + dram__bytes_write.sum, profiles/k_gn_single_frame.md"
 COARSE_TRAFFIC = 42_780_928 + 71_592_448
@@ -1558,7 +1559,7 @@ def run_prior(a, rank: int, world: int, local: int):
             "achieved": round(ach, 3), "peak": peak["hbm_gbs"], "unit": "GB/s", "frac": round(ach / peak["hbm_gbs"], 5),
             "traffic": None, "peak_source": peak["source"], "algorithmic_bytes_per_launch": ins_bytes,
             "avg_ms": round(ins_ms, 4),
-            "limiter": "five int64 atomics per point on its voxel's line (about four points share a 20 mm voxel)"}
+            "limiter": "one 64-byte bulk reduction per point on its voxel's line (about four points share a 20 mm voxel)"}
     line = {"metric": metric, "value": round(value, 1), "unit": "points/s", "n_gpus": world, "steps": a.steps,
             "warmup": a.warmup, "ms_per_step": round(avg_ms, 4), "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f32 in, int64 fixed-point sums, f64 PCA", "data": "synthetic",

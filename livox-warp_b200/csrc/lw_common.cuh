@@ -166,8 +166,8 @@ __device__ __forceinline__ void atomic_add_i64(int64_t* a, int64_t v) {
 // float -> int64 fixed point, round to nearest even (llrintf on the host).
 __device__ __forceinline__ int64_t to_fix(float v, float scale) { return __float2ll_rn(v * scale); }
 
-// to_fix for sums of many terms, without the float -> int64 conversion (a quarter-rate or slower instruction; six to nine of
-// them per term bound the neighbourhood kernels). Adding 1.5 x 2^23 to a float below 2^22 in magnitude rounds it to
+// to_fix for sums of many terms, without the float -> int64 conversion (a quarter-rate or slower instruction; nine of them
+// per term of a neighbourhood's sums). Adding 1.5 x 2^23 to a float below 2^22 in magnitude rounds it to
 // the nearest integer, ties to even as the conversion does, and leaves that integer in the low bits. A product v below
 // 2^42 is split as v = hi 2^20 + lo with hi = rint(v 2^-20) and lo exact and at most 2^19, so
 // rint(v) = hi 2^20 + rint(lo): two 32-bit integers, each from one addition.

@@ -994,7 +994,7 @@ __device__ __forceinline__ float soft_count(int n_in, int sum_d2, float tau) {
 // computes the rotated offsets, the posed y and z, their cells and the row's address, into shared memory. What is left
 // per position and point is the x chain, two positions to a packed instruction, with the floor taken by one addition that
 // rounds down (sc_cell) instead of a quarter-rate conversion. Rows outside the grid and dead positions get an x far outside
-// it and need no test of their own. 3.5M hypotheses x 1024 points of an office: 4.87 -> 2.27 ms, at 88% of the issue slots.
+// it and need no test of their own. 3.5M hypotheses x 1024 points of an office: 4.87 -> 2.27 ms, at 84% of the issue slots.
 // A warp whose positions are spread over many rows (list order along y) gains nothing from the table: its hypotheses are
 // left to k_score_rest, and so are all of them when a point is not finite. Four CTAs an SM and eight points in flight:
 // five CTAs take 2.33 ms; positions 32 apart in a thread, 2.4; branches around the gathers, 4.0.
