@@ -374,7 +374,8 @@ int lw_ring_append(const float* xyz, int32_t xyz_stride, const int32_t* attr, co
 
 /* Buffers of the neighbourhood pass, contents undefined between calls: an open-addressed table of cap (a power of two)
  * slots for the bricks of 4 x 4 x 4 voxels that the points lie in (a call clears and uses the first power of two of
- * at least 2 n slots) and dense per-voxel arrays (at most one voxel per point), numbered brick by brick. */
+ * at least 2 n slots) and dense per-voxel arrays (at most one voxel per point), numbered brick by brick. With cap >= 2 n
+ * every point finds room; a smaller table may run out, and which bricks it then holds depends on timing. */
 typedef struct lw_nbr_buf {
     int64_t* keys;       /* [cap] brick keys, -1 empty */
     int64_t* acc;        /* [cap*4] fixed-point sums of x, y, z (LW_FIX_W units) and the point count, then the means */
@@ -494,7 +495,7 @@ int lw_ground(const float* xyz, int32_t xyz_stride, const float* nrm, const int3
 
 /* Buffers of the Euclidean clustering, contents undefined between calls. A call gathers the voxels into bricks of
  * 4 x 4 x 4 in an open-addressed table (the first power of two of at least 2 n of its cap slots) and numbers them
- * brick by brick. */
+ * brick by brick. Room as in lw_nbr_buf. */
 typedef struct lw_cluster_buf {
     int64_t* keys;       /* [cap] brick keys, -1 empty */
     int64_t* acc;        /* [cap*4] the bricks' masks of occupied voxels and first voxels */

@@ -28,6 +28,33 @@ __device__ __forceinline__ int64_t brick_of(int ix, int iy, int iz, int& bit) {
     return brick_key(x >> 2, y >> 2, z >> 2);
 }
 
+// The table of the bricks. Its load may come to a half (a cloud sparser than a brick), and the bricks of a floor are a regular
+// lattice, which slot_hash -- one multiplication, one shift -- lays in clumps: 2^20 bricks of a flat grid in 2^21 slots
+// lost 250 to a window of 64 probes, differing ones with the order of arrival. So the keys are mixed by two rounds, which
+// leave the longest chain of the same grid at 34 (45 over all lattices and halls tried, up to 3M bricks), and the window
+// is 256: a random table at half load has a chain that long once in 10^15 calls. A table smaller than twice
+// the points serves as far as it goes (loads up to 0.8); bricks it has no room for are reported as such.
+constexpr int BRICK_PROBES = 256;
+
+__host__ __device__ __forceinline__ int brick_hash(int64_t k) {
+    uint64_t h = (uint64_t)k * HASH_MULT;
+    h ^= h >> 32;
+    h *= HASH_MULT;
+    h ^= h >> 29;
+    return (int)(h & 0x7FFFFFFFULL);
+}
+
+// Slot of the brick, or -1.
+__device__ __forceinline__ int find_brick(int64_t key, const int64_t* __restrict__ keys, int mask) {
+    return find_from<BRICK_PROBES>(brick_hash(key), key, keys, mask);
+}
+
+// Slot of the brick, claimed if it has none yet; -1 when its window is full.
+__device__ __forceinline__ int claim_brick(int64_t key, int64_t* keys, int mask) {
+    bool claimed;
+    return claim_from<BRICK_PROBES>(brick_hash(key), key, keys, mask, &claimed);
+}
+
 // Slots a hash of at most n bricks takes: the power of two from 2 n up, at least 1024 and at most cap.
 inline int64_t brick_slots(int64_t n, int64_t cap) {
     int64_t h = 1024;
@@ -110,7 +137,7 @@ __device__ __forceinline__ void brick_rows(const int64_t* keys, const int32_t* b
             const int64_t k = keys[lead];
             const int64_t nk = brick_key((k & BRICK_MASK) + (c % 3 - 1), (k >> 19 & BRICK_MASK) + (c / 3 % 3 - 1),
                                          (k >> 38 & BRICK_MASK) + (c / 9 - 1));
-            s = c == 13 ? lead : find_slot(nk, keys, hash_mask);
+            s = c == 13 ? lead : find_brick(nk, keys, hash_mask);
             rows.mask[r][c] = s < 0 ? 0ull : mask_of(s, r, c, lead);
             rows.base[r][c] = s < 0 ? 0 : base[s];
         }

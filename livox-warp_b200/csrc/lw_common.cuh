@@ -70,10 +70,10 @@ __host__ __device__ __forceinline__ int slot_hash(int64_t k) {
     return (int)(h & 0x7FFFFFFFLL);
 }
 
-// Slot holding `key`, or -1 (gpu.py:254-265). P probes (the prior-map table takes 128, prior_map.py:36).
-template <int P = PROBES>
-__device__ __forceinline__ int find_slot(int64_t key, const int64_t* __restrict__ keys, int mask) {
-    int h = slot_hash(key) & mask;
+// Slot holding `key`, or -1, P slots from `hash` on.
+template <int P>
+__device__ __forceinline__ int find_from(int hash, int64_t key, const int64_t* __restrict__ keys, int mask) {
+    int h = hash & mask;
 #pragma unroll 1
     for (int p = 0; p < P; ++p) {
         int s = (h + p) & mask;
@@ -84,11 +84,17 @@ __device__ __forceinline__ int find_slot(int64_t key, const int64_t* __restrict_
     return -1;
 }
 
-// Find the slot of `key` or claim an empty one. Returns the slot and sets *claimed when this call turned an
-// empty slot into `key`; -1 when the probe window of P slots is full (gpu.py:396-412).
+// Slot holding `key`, or -1 (gpu.py:254-265). P probes (the prior-map table takes 128, prior_map.py:36).
 template <int P = PROBES>
-__device__ __forceinline__ int claim_slot(int64_t key, int64_t* keys, int mask, bool* claimed) {
-    int h = slot_hash(key) & mask;
+__device__ __forceinline__ int find_slot(int64_t key, const int64_t* __restrict__ keys, int mask) {
+    return find_from<P>(slot_hash(key), key, keys, mask);
+}
+
+// Find the slot of `key` or claim an empty one, P slots from `hash` on. Returns the slot and sets *claimed when this call
+// turned an empty slot into `key`; -1 when the probe window is full (gpu.py:396-412).
+template <int P>
+__device__ __forceinline__ int claim_from(int hash, int64_t key, int64_t* keys, int mask, bool* claimed) {
+    int h = hash & mask;
     *claimed = false;
 #pragma unroll 1
     for (int p = 0; p < P; ++p) {
@@ -106,6 +112,11 @@ __device__ __forceinline__ int claim_slot(int64_t key, int64_t* keys, int mask, 
         }
     }
     return -1;
+}
+
+template <int P = PROBES>
+__device__ __forceinline__ int claim_slot(int64_t key, int64_t* keys, int mask, bool* claimed) {
+    return claim_from<P>(slot_hash(key), key, keys, mask, claimed);
 }
 
 // ---- attribute fields (gpu.py:124-141) -----------------------------------------------------------------

@@ -10,7 +10,8 @@
 // -- all within 3 voxels along each axis (a centroid lies inside its voxel, and voxels are radius / 3 wide), found
 // through the masks of the 27 bricks around it (lw_bricks.cuh) -- and their weighted offsets and outer products are
 // summed as int64 fixed point too; the covariance and its eigen-decomposition are float64. Every point's count,
-// normal and curvature is then independent of thread order and of where keys land in the table.
+// normal and curvature is then independent of thread order and of where keys land in the table. (A table smaller than two
+// slots a point can run out of room; which points it then leaves out depends on their order of arrival.)
 //
 // Layout of the caller's buffers: keys, v_slot / vidx and v_w hold the bricks' keys, masks' halves and bases in the first
 // brick_slots(n) slots (so a call clears what its points can fill, not the whole table); acc holds voxel v's sums and
@@ -64,8 +65,7 @@ __global__ void k_nb_insert(const float* __restrict__ xyz, const int* n_dev, int
         float x, y, z;
         int bit;
         const int64_t key = nb_brick<STRIDE>(xyz, i, a, x, y, z, bit);
-        bool claimed;
-        const int s = claim_slot(key, nb.keys, a.mask, &claimed);
+        const int s = claim_brick(key, nb.keys, a.mask);
         if (s >= 0) {
             unsigned* half = reinterpret_cast<unsigned*>((bit & 32) ? nb.vidx : nb.v_slot) + s;
             const unsigned b = 1u << (bit & 31);

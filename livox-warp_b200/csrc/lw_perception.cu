@@ -167,8 +167,7 @@ __global__ void k_cl_insert(const float* __restrict__ xyz, const int* __restrict
             ld3<STRIDE>(xyz, i, x, y, z);
             int bit;
             const int64_t key = brick_of(ifloor(x * a.inv_v), ifloor(y * a.inv_v), ifloor(z * a.inv_v), bit);
-            bool claimed;
-            s = claim_slot(key, cb.keys, a.mask, &claimed);
+            s = claim_brick(key, cb.keys, a.mask);
             if (s >= 0) {
                 uint64_t* m = cl_masks(cb) + s;
                 if ((*(volatile uint64_t*)m >> bit & 1) == 0) atomicOr((unsigned long long*)m, 1ull << bit);
