@@ -322,8 +322,8 @@ int lw_carve(const float* xyz, int32_t xyz_stride, const uint32_t* attr, const i
              const int32_t* n_dev, int64_t n_ub, const float* poses, int32_t every, float inv_voxel,
              float max_range, int32_t max_steps, lw_map* map, float* ray_stop, void* stream);
 
-/* Workspace of lw_carve_ws, contents undefined between calls: (ray, occupied voxel) pairs and their times, the distinct voxels met and their
- * planes. Pairs or voxels beyond the capacities are handled without the workspace (slower, same misses); about 16
+/* Workspace of lw_carve_ws, one per call in flight: (ray, occupied voxel) pairs and their times, the distinct voxels met and
+ * their planes, all undefined between calls, and marks, 0 between calls. Pairs or voxels beyond the capacities are handled without the workspace (slower, same misses); about 16
  * pairs and 4 voxels per ray hold an indoor frame. planes is 16-byte aligned. */
 typedef struct lw_carve_buf {
     int64_t* pairs;   /* [pair_cap] */
@@ -332,10 +332,11 @@ typedef struct lw_carve_buf {
     int32_t* slots;   /* [slot_cap] */
     int64_t* counts;  /* [3] */
     int64_t pair_cap, slot_cap;
+    int32_t* marks;   /* [map cap]; NULL: the map's bcnt serves, and no insertion into the map may run meanwhile */
 } lw_carve_buf;
 
-/* lw_carve with a workspace: each occupied voxel the rays meet has its plane fitted once instead of once per ray (it
- * uses the map's bcnt scratch). The same misses, bit for bit. */
+/* lw_carve with a workspace: each occupied voxel the rays meet has its plane fitted once instead of once per ray. The same
+ * misses, bit for bit; of the map it writes them alone. */
 int lw_carve_ws(const float* xyz, int32_t xyz_stride, const uint32_t* attr, const int32_t* frame,
                 const int32_t* n_dev, int64_t n_ub, const float* poses, int32_t every, float inv_voxel,
                 float max_range, int32_t max_steps, lw_map* map, float* ray_stop, lw_carve_buf* cb, void* stream);

@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(128) k_carve(const float* __restrict__ xyz, co
 // the very steps the whole walk takes. Bound by the issue of the DDA's steps and the probes' latency: for 10,000 rays of
 // about 100 steps 13.7 us, against 22 us with 8 lanes repeating the whole DDA and 16.6 us with 8 stretches (the
 // adding-up is repeated). A warp gathers its pairs in shared memory (one atomic on the pair count per warp, not
-// per round of probes: 22 us). map.bcnt, zero between calls, marks a voxel as met and then holds its place among
+// per round of probes: 22 us). cb.marks, zero between calls, marks a voxel as met and then holds its place among
 // the distinct ones plus one; the last CTA of the pair pass zeroes it again.
 // For 10,000 rays the three passes take 15 + 24 + 9 us where k_carve's two took 22 + 175, and a pass of its own for the stops 22 + 14 +
 // 21 + 7.
@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(CW_THREADS) k_carve_walk(
                 if (p + i0 + lane < cb.pair_cap) {
                     cb.pairs[p + i0 + lane] = pair;
                     cb.times[p + i0 + lane] = when[i0 + lane];
-                    first = *(volatile int*)(map.bcnt + s) == 0 && atomicExch(map.bcnt + s, 1) == 0;
+                    first = *(volatile int*)(cb.marks + s) == 0 && atomicExch(cb.marks + s, 1) == 0;
                 } else if (carve_alone<STRIDE>(xyz, attr, frame, poses, pair, when[i0 + lane], every, inv_voxel,
                                                max_range, map)) {
                     atomicAdd(map.miss + s, every);
@@ -549,7 +549,7 @@ __global__ void __launch_bounds__(CW_THREADS) k_carve_walk(
                 if (q < cb.slot_cap)
                     cb.slots[q] = s;
                 else
-                    *(volatile int*)(map.bcnt + s) = 0;  // no room: the pair pass fits this voxel itself
+                    *(volatile int*)(cb.marks + s) = 0;  // no room: the pair pass fits this voxel itself
             }
         }
         __syncwarp();
@@ -727,11 +727,11 @@ __global__ void __launch_bounds__(64) k_carve_planes(const float* __restrict__ x
         centroid(map, s, cx, cy, cz);
         out[2 * p] = make_float4(cx, cy, cz, 0.0f);
         out[2 * p + 1] = local_plane(ix, iy, iz, cx, cy, cz, map, mask);
-        map.bcnt[s] = (int)p + 1;
+        cb.marks[s] = (int)p + 1;
     }
 }
 
-// The pairs, a thread each; the last CTA out puts map.bcnt back to zero for the slots met.
+// The pairs, a thread each; the last CTA out puts cb.marks back to zero for the slots met.
 template <int STRIDE>
 __global__ void __launch_bounds__(256) k_carve_pairs(const float* __restrict__ xyz, const uint32_t* __restrict__ attr,
                                                      const int32_t* __restrict__ frame, const float* __restrict__ poses,
@@ -746,7 +746,7 @@ __global__ void __launch_bounds__(256) k_carve_pairs(const float* __restrict__ x
         const int s = (int)(pair & 0xffffffff);
         const float stop = ray_stop[pair >> 32];
         if (!(stop > 1.0f && cb.times[p] < stop)) continue;
-        const int q = map.bcnt[s];
+        const int q = cb.marks[s];
         bool hit;
         if (q > 0) {
             float ox, oy, oz, wx, wy, wz, dx, dy, dz, L;
@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(256) k_carve_pairs(const float* __restrict__ x
     if (!last) return;
     const int64_t m = min(cb.counts[1], cb.slot_cap);
 #pragma unroll 4
-    for (int64_t p = threadIdx.x; p < m; p += blockDim.x) map.bcnt[cb.slots[p]] = 0;
+    for (int64_t p = threadIdx.x; p < m; p += blockDim.x) cb.marks[cb.slots[p]] = 0;
 }
 
 // =====================================================================================================
@@ -1155,6 +1155,8 @@ int lw_carve_ws(const float* xyz, int32_t xyz_stride, const uint32_t* attr, cons
     if (n_ub <= 0) return LW_OK;
     if (every < 1) every = 1;
     cudaStream_t s = (cudaStream_t)stream;
+    lw_carve_buf b = *cb;
+    if (!b.marks) b.marks = map->bcnt;
     const int64_t rays = (n_ub + every - 1) / every;
     const int sms = device_sms();
     const int grid2 = blocks_for(rays * CW_PARTS, CW_THREADS, 16 * sms);
@@ -1165,10 +1167,10 @@ int lw_carve_ws(const float* xyz, int32_t xyz_stride, const uint32_t* attr, cons
     auto run = [&](auto stride) {
         constexpr int S = decltype(stride)::value;
         k_carve_walk<S><<<grid2, CW_THREADS, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range,
-                                                     max_steps, *map, *cb);
+                                                     max_steps, *map, b);
         k_carve_planes<S><<<grid3, 64, 0, s>>>(xyz, attr, frame, n_dev, n_ub, poses, every, inv_voxel, max_range, *map,
-                                               ray_stop, *cb);
-        k_carve_pairs<S><<<grid4, 256, 0, s>>>(xyz, attr, frame, poses, every, inv_voxel, max_range, *map, ray_stop, *cb);
+                                               ray_stop, b);
+        k_carve_pairs<S><<<grid4, 256, 0, s>>>(xyz, attr, frame, poses, every, inv_voxel, max_range, *map, ray_stop, b);
     };
     if (xyz_stride == 4)
         run(std::integral_constant<int, 4>{});

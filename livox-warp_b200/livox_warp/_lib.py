@@ -88,7 +88,7 @@ class Map(C.Structure):
 
 class CarveBuf(C.Structure):
     PTRS = ("pairs", "times", "planes", "slots", "counts")
-    _fields_ = [(n, P) for n in PTRS] + [("pair_cap", i64), ("slot_cap", i64)]
+    _fields_ = [(n, P) for n in PTRS] + [("pair_cap", i64), ("slot_cap", i64), ("marks", P)]
 
 
 class ClusterBuf(C.Structure):

@@ -207,6 +207,7 @@ class Pipeline:
         self.cl_tid = torch.full((MAX_CLUSTERS,), -1, dtype=torch.int32, device=d)
         self._slot = torch.zeros(n, dtype=torch.int32, device=d)  # per-point scratch of the insert passes
         self._carve_rays, self._carve_t, self._carve_buf = 0, [], None  # lw_carve_ws's workspace
+        self._carve_marks = torch.zeros(m, dtype=torch.int32, device=d)  # its own: an insertion may run beside a carve
         self._carve_ws(1 << 15)  # what a frame takes, made here so that no frame waits for an allocation
         self._tiles = torch.zeros(max(m, self.cap) // 1024 + 2, dtype=torch.int32, device=d)
         self.total = torch.zeros(1, dtype=torch.int32, device=d)
@@ -380,9 +381,10 @@ class Pipeline:
         sx = _as_xyz(sx, self.device)
         every = max(1, int(every))
         rays = (n + every - 1) // every
+        ws = self._carve_ws(rays)
         _lib.call("lw_carve_ws", _lib.ptr(sx), row_stride(sx), _lib.ptr(sa), _lib.ptr(sf), _lib.ptr(n_dev), n,
                   _lib.ptr(self.poses), every, 1.0 / max(voxel, 1e-4), float(max_range), int(max_steps),
-                  C_ref(self.map_struct), _lib.ptr(self._scratch(n)), C_ref(self._carve_ws(rays)), _lib.stream_ptr())
+                  C_ref(self.map_struct), _lib.ptr(self._carve_t[-1][-1]), C_ref(ws), _lib.stream_ptr())
 
     def _carve_ws(self, rays: int) -> _lib.CarveBuf:
         """lw_carve_ws's workspace for at least `rays` rays. It grows by doubling, and the smaller ones are kept: a
@@ -392,9 +394,10 @@ class Pipeline:
             pairs, slots, d = 16 * r, min(4 * r, self.map_cap), self.device
             t = (torch.empty(pairs, dtype=torch.int64, device=d), torch.empty(pairs, dtype=torch.float32, device=d),
                  torch.empty((slots, 8), dtype=torch.float32, device=d),
-                 torch.empty(slots, dtype=torch.int32, device=d), torch.zeros(3, dtype=torch.int64, device=d))
+                 torch.empty(slots, dtype=torch.int32, device=d), torch.zeros(3, dtype=torch.int64, device=d),
+                 torch.empty(r, dtype=torch.float32, device=d))  # the last: where each ray stops
             self._carve_t.append(t)
-            self._carve_buf = _lib.CarveBuf(*(_lib.ptr(x) for x in t), pairs, slots)
+            self._carve_buf = _lib.CarveBuf(*(_lib.ptr(x) for x in t[:5]), pairs, slots, _lib.ptr(self._carve_marks))
             self._carve_rays = r
         return self._carve_buf
 
