@@ -1,5 +1,7 @@
 """What Pipeline.carve may touch: the misses, and a workspace of its own."""
 
+import threading
+
 import pytest
 import torch
 
@@ -50,3 +52,50 @@ def test_carving_leaves_the_insertion_scratch_alone(mapped, every):
         pipe._map_bcnt.copy_(count)
         pipe._slot.copy_(slot)
         pipe.map_miss.zero_()
+
+
+def test_carves_from_several_streams_and_threads_take_turns(mapped):
+    """Four threads with a stream each, carving at the same time with different strides: every call counts what it counts
+    alone."""
+    pipe, (sx, sa, sf) = mapped
+    strides, rounds = (1, 2, 3, 5), 12
+    want = sum(_want(pipe, sx, sa, sf, e) for e in strides) * rounds
+    torch.cuda.synchronize()
+    start, failed = threading.Barrier(len(strides)), []
+
+    def work(every):
+        try:
+            stream = torch.cuda.Stream()
+            start.wait(10.0)
+            with torch.cuda.stream(stream):
+                for _ in range(rounds):
+                    pipe.carve(sx, sa, sf, len(sf), VOXEL, every=every)
+            stream.synchronize()
+        except Exception as e:  # noqa: BLE001
+            failed.append(e)
+
+    threads = [threading.Thread(target=work, args=(e,)) for e in strides]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
+    got = pipe.map_miss.clone()
+    pipe.map_miss.zero_()
+    assert torch.equal(got, want)
+    assert int(pipe._carve_marks.abs().sum()) == 0
+
+
+def test_a_captured_carve_counts_like_an_eager_one(mapped):
+    pipe, (sx, sa, sf) = mapped
+    want = _want(pipe, sx, sa, sf, 2)
+    pipe.carve(sx, sa, sf, len(sf), VOXEL, every=2)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        pipe.carve(sx, sa, sf, len(sf), VOXEL, every=2)
+    g.replay()
+    pipe.carve(sx, sa, sf, len(sf), VOXEL, every=2)
+    torch.cuda.synchronize()
+    got = pipe.map_miss.clone()
+    pipe.map_miss.zero_()
+    assert torch.equal(got, 3 * want)
