@@ -560,6 +560,11 @@ int lw_prior_grid_build(lw_prior_grid* g, void* stream);
 int lw_prior_starts(const int32_t* cells, const int32_t* first, int64_t u, int64_t n, int64_t ncell, int32_t* start,
                     void* stream);
 
+/* Host: 1 when start [ncell+1] (host, never falling) is what lw_prior_starts makes of cells and first [u] (host) and n, 0 when
+ * not. */
+int lw_prior_starts_match(const int32_t* start, const int32_t* cells, const int32_t* first, int64_t u, int64_t n,
+                          int64_t ncell);
+
 /* Distance of n points (pts [n*3]) posed by T (row-major 4x4, host) to the nearest map point, 1e3 beyond the
  * band (mapgrid.py:173-194, PriorGrid.distances :298-305). */
 int lw_prior_distances(const lw_prior_grid* g, const float* pts, int64_t n, const double* T_host, float* out,

@@ -1392,6 +1392,20 @@ int lw_prior_grid_build(lw_prior_grid* g, void* stream) {
     return LW_OK;
 }
 
+// An array that never falls, holds first[j] at cells[j] and first[j + 1] one further on is first[j + 1] from there to
+// cells[j + 1]: the two ends of every occupied cell tell for all cells.
+int lw_prior_starts_match(const int32_t* start, const int32_t* cells, const int32_t* first, int64_t u, int64_t n,
+                          int64_t ncell) {
+    if (!start || !cells || !first || u <= 0 || ncell <= 0 || start[0] != 0 || start[ncell] != n) return 0;
+    int64_t last = -1;
+    for (int64_t j = 0; j < u; ++j) {
+        const int64_t c = cells[j], end = j + 1 < u ? first[j + 1] : n;
+        if (c <= last || c >= ncell || start[c] != first[j] || start[c + 1] != end) return 0;
+        last = c;
+    }
+    return 1;
+}
+
 int lw_prior_starts(const int32_t* cells, const int32_t* first, int64_t u, int64_t n, int64_t ncell, int32_t* start,
                     void* stream) {
     if (u < 0 || n < 0 || n > 0x7FFFFFFF || ncell < 0 || !start || (u > 0 && (!cells || !first)))

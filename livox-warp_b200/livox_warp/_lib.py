@@ -231,6 +231,7 @@ _SIGS = {
                                    C.POINTER(GnScratch), C.POINTER(PoseTable), i32, P, i64, C.POINTER(InitNet),
                                    C.POINTER(NetWork), P]),
     "lw_prior_starts": (i32, [P, P, i64, i64, i64, P, P]),
+    "lw_prior_starts_match": (i32, [P, P, P, i64, i64, i64]),
     "lw_prior_distances": (i32, [C.POINTER(PriorGrid), P, i64, C.POINTER(f64), P, P]),
     "lw_score_grid": (i32, [C.POINTER(PriorGrid), P, i32, P, i64, i64, i32, f32, f32, f32, f32, P, P]),
     "lw_score_list": (i32, [C.POINTER(PriorGrid), P, i32, P, i64, f32, P, P]),

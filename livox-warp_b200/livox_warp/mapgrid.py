@@ -147,26 +147,44 @@ class PriorGrid:
         t0 = time.perf_counter()
         s = stream if stream is not None else torch.cuda.current_stream(self.device)
         h = self._host
+        # a prepared map may have been put together elsewhere (a file, another program): any numeric arrays of these shapes
+        xyz = np.ascontiguousarray(h["xyz"], dtype=np.float32)
+        planar = np.ascontiguousarray(h["planarity"], dtype=np.float32)
+        if planar.shape != (self.n,):
+            planar = np.broadcast_to(planar, (self.n,)).copy()
+        steps = None
+        if "cells" in h and "first" in h:
+            steps = [np.ascontiguousarray(h[k], dtype=np.int32) for k in ("cells", "first")]
         with torch.cuda.stream(s):
             d = self.device
             # the records are put together on the device: on the host the packing took as long as the copies
-            self.xyzp[:, :3].copy_(torch.from_numpy(h["xyz"]).to(d))
-            self.xyzp[:, 3].copy_(torch.from_numpy(h["planarity"]).to(d))
+            self.xyzp[:, :3].copy_(torch.from_numpy(xyz).to(d))
+            self.xyzp[:, 3].copy_(torch.from_numpy(planar).to(d))
             self.nrm.copy_(torch.from_numpy(h["normal"]))
-            if "cells" in h and "first" in h:  # the prefix array from the occupied cells: few of a grid's cells hold points
-                cells, first = torch.from_numpy(h["cells"]).to(d), torch.from_numpy(h["first"]).to(d)
+            if steps is not None:  # the prefix array from the occupied cells: few of a grid's cells hold points
+                cells, first = (torch.from_numpy(v).to(d) for v in steps)
                 _lib.call("lw_prior_starts", _lib.ptr(cells), _lib.ptr(first), len(cells), self.n, self.ncell,
                           _lib.ptr(self.start), _lib.stream_ptr(s))
-            else:
-                self.start.copy_(torch.from_numpy(h["start"]))
             seed = torch.empty(self.ncell, dtype=torch.int64, device=self.device)
             nn2 = torch.empty(self.ncell, dtype=torch.int32, device=self.device)
             g = self._struct(seed, nn2)
             _lib.call("lw_prior_grid_build", C.byref(g), _lib.stream_ptr(s))
+            # `start` says where each cell's points are, whatever else the map holds; it is looked at while the flood, which
+            # does not read it, runs on the device
+            if steps is None or not self._steps_of(h["start"], *steps):
+                self.start.copy_(torch.from_numpy(h["start"]))
         s.synchronize()
         del seed, nn2
         self.build_s = time.perf_counter() - t0
         self.ready = True
+
+    def _steps_of(self, start, cells, first) -> bool:
+        """Whether `start` is the prefix array that (cells, first) stand for."""
+        start = np.ascontiguousarray(start, dtype=np.int32)
+        if start.shape != (self.ncell + 1,) or cells.shape != first.shape or cells.ndim != 1:
+            return False
+        p = [C.c_void_p(v.ctypes.data) for v in (start, cells, first)]
+        return bool(_lib.load().lw_prior_starts_match(*p, len(cells), self.n, self.ncell))
 
     def distances(self, pts: torch.Tensor, n: int, T_map_from_pts: np.ndarray, out: torch.Tensor, stream=None):
         """Distance to the map of the first n points of `pts` ([*, 3] float32, in a frame that T maps into the
