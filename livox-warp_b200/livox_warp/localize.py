@@ -47,6 +47,7 @@ SCHEDULE_REFINE = ((0.30, 6), (0.12, 8), (0.05, 8))  # GlobalLocalizer.refine de
 ALPHA = 0.05  # along-surface weight of a planar correspondence, localize.py:523
 MIN_COUNT = 30  # matches below which a hypothesis keeps its pose, localize.py:538
 TILES = (32, 64, 128)  # points per warp tile the autotuner tries
+GRAPH_TILE = 256  # the one of register_graph and evaluate
 BUDGETS = (3, 4, 5, 6)  # resident CTAs per SM of the register budgets it tries (the library also has 2)
 CANDIDATES = tuple((t, m) for t in TILES for m in BUDGETS)
 
@@ -333,8 +334,9 @@ class LocBatch:
         self.moved = torch.zeros(self.ITERS_CAP, dtype=torch.int32, device=d)
         self.next = torch.zeros(self.ITERS_CAP + 1, dtype=torch.int32, device=d)
         self.bar = torch.zeros(2, dtype=torch.int32, device=d)
-        # every point of every tile, sorted by place, and its match (tiles of 32 points always fit)
-        slots = TILES[0] * NT
+        # every point of every tile, sorted by place, and its match: a scan's last tile may be part empty, so a batch of
+        # pts_cap points in hyp_cap scans takes up to this many slots in tiles of up to GRAPH_TILE
+        slots = self.pts_cap + GRAPH_TILE * self.hyp_cap
         self.sorted = torch.empty((slots, 4), dtype=torch.float32, device=d)
         self.match = torch.empty(slots, dtype=torch.int32, device=d)
         self.ws = _lib.LocWs(_lib.ptr(self.sorted), _lib.ptr(self.match), slots)
@@ -847,7 +849,7 @@ class GlobalLocalizer:
         pts = np.asarray(pts, dtype=np.float32)
         self._upload_pts([pts], stream)
         k = len(Ts)
-        return self._run(np.zeros(k, np.int64), np.full(k, len(pts), np.int64), Ts, (), stream, tile=256).fit
+        return self._run(np.zeros(k, np.int64), np.full(k, len(pts), np.int64), Ts, (), stream, tile=GRAPH_TILE).fit
 
     # ---- many hypotheses, uneven scans --------------------------------------------------------------
 
@@ -881,7 +883,7 @@ class GlobalLocalizer:
             b.pts[:n].copy_(pts4, non_blocking=True)
         return self._run(lo, hi, T0s, schedule, stream, tile, blocks_per_sm)
 
-    def register_graph(self, lo, hi, schedule=SCHEDULE_ICP, tile: int = 256, stream=None, blocks_per_sm: int = 3):
+    def register_graph(self, lo, hi, schedule=SCHEDULE_ICP, tile: int = GRAPH_TILE, stream=None, blocks_per_sm: int = 3):
         """A CUDA graph of the batched launch for the staged batch's shape class: the hypothesis and tile counts
         are read on the device (lw_loc_batch.dims), so one capture replays over any batch up to the buffers'
         capacity with that schedule and tile. Returns a callable that stages (lo, hi, T0s) and replays it."""
