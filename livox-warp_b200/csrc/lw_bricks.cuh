@@ -103,7 +103,13 @@ struct BrickRows {
     int32_t base[BRICK_ROWS][27];
 };
 
-// For the 32 voxels of a CTA, lane l of every warp serving voxel l, in the order of their numbers (slot: the voxel's
+// Voxels that a CTA walking neighbourhoods takes at a time: 32, or 8 up to 64 points an SM -- one wave of such CTAs, eight to an
+// SM -- where 32 would leave most of the chip idle and each CTA with a chain of up to 32 lone bricks to look up, four at a
+// time. A perception frame of 500 / 6,000 sparse points: 357 / 501 us with 32, 274 / 410 with 8 (274 / 414 before there were
+// bricks); from 12,000 on 32 is as good.
+inline int brick_voxels(int64_t n, int sms) { return n > 64 * (int64_t)sms ? 32 : 8; }
+
+// For the up to 32 voxels of a CTA, lane l of every warp serving voxel l, in the order of their numbers (slot: the voxel's
 // brick, -1 for none; every thread calls), run(row) with the bricks around the lane's own brick in rows.mask[row],
 // rows.base[row]. Voxels of a brick are neighbours in number, so 32 of them lie in a few bricks, whose 27 neighbours are
 // looked up side by side, BRICK_ROWS bricks at a time. The warps share out the 27 bricks (warp w takes w, w + BRICK_WARPS, ...):

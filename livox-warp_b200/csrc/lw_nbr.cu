@@ -29,6 +29,7 @@ constexpr int NB_REACH = 3;                    // voxels per axis: radius / (rad
 struct NbArgs {
     float inv_h, r2;
     int mask, want_normals;
+    int per;       // voxels per CTA
     int64_t vcap;  // voxel records the buffers hold
     double sensor[3];
 };
@@ -139,8 +140,8 @@ __global__ void __launch_bounds__(BRICK_CTA, 8) k_nb_voxel(NbArgs a, lw_nbr_buf 
     __shared__ long long part[BRICK_WARPS - 1][10][32];
     const int64_t m = nb_voxels(nb, a.vcap);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int64_t j0 = (int64_t)blockIdx.x * 32; j0 < m; j0 += (int64_t)gridDim.x * 32) {
-        const int64_t j = j0 + lane;
+    for (int64_t j0 = (int64_t)blockIdx.x * a.per; j0 < m; j0 += (int64_t)gridDim.x * a.per) {
+        const int64_t j = lane < a.per ? j0 + lane : m;
         const int slot = j < m ? __float_as_int(nb.v_cnt[j]) : -1;
         const float4 P = j < m ? *reinterpret_cast<const float4*>(nb.acc + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
         long long W = 0, s1[3] = {0, 0, 0}, s2[6] = {0, 0, 0, 0, 0, 0};
@@ -308,6 +309,7 @@ int lw_neighborhoods(const float* xyz, int32_t xyz_stride, const int32_t* n_dev,
         a.vcap -= 1;
     }
     const int sms = device_sms();
+    a.per = brick_voxels(n_ub, sms);
     if (n_ub <= 0) {
         LW_CUDA(cudaMemsetAsync(nb->m, 0, sizeof(int32_t), s));
         return LW_OK;
@@ -325,7 +327,7 @@ int lw_neighborhoods(const float* xyz, int32_t xyz_stride, const int32_t* n_dev,
         k_nb_sum<3><<<grid, 256, 0, s>>>(xyz, n_dev, n_ub, a, b);
     // at most one voxel per point
     k_nb_mean<<<grid, 256, 0, s>>>(b, a.vcap);
-    k_nb_voxel<<<blocks_for(n_ub, 32, 64 * sms), BRICK_CTA, 0, s>>>(a, b);
+    k_nb_voxel<<<blocks_for(n_ub, a.per, 64 * sms), BRICK_CTA, 0, s>>>(a, b);
     k_nb_gather<<<grid, 256, 0, s>>>(n_dev, n_ub, a.want_normals, b, out_cnt, out_nrm, out_curv);
     LW_LAUNCHED("lw_neighborhoods");
     count_launches(7);

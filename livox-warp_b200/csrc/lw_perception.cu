@@ -131,6 +131,8 @@ struct ClArgs {
     float inv_v;
     int mask, use_gnd;
     int64_t slots;  // brick slots used
+    int per;        // voxels that a warp of k_cl_brick and a CTA of k_cl_join take at a time
+    int run;        // rounds of 32 nodes a warp of k_cl_stats takes
     float connect2;
     int reach;
     float min_pts;
@@ -311,15 +313,15 @@ __global__ void __launch_bounds__(32 * CL_WARPS) k_cl_brick(ClArgs a, lw_cluster
     int* node = node_s[warp];
     uint64_t* link = link_s[warp];
     const int64_t nwarps = (int64_t)gridDim.x * CL_WARPS;
-    for (int64_t w = (int64_t)blockIdx.x * CL_WARPS + warp; w * 32 < m; w += nwarps) {
-        const int64_t v0 = w * 32 + lane;
-        const int slot0 = v0 < m ? cl_brick(cb)[v0] : -1;
-        // the bricks whose first voxel is among the warp's 32
+    for (int64_t w = (int64_t)blockIdx.x * CL_WARPS + warp; w * a.per < m; w += nwarps) {
+        const int64_t v0 = w * a.per + lane;
+        const int slot0 = lane < a.per && v0 < m ? cl_brick(cb)[v0] : -1;
+        // the bricks whose first voxel is among the warp's
         unsigned leads = __ballot_sync(0xffffffffu, slot0 >= 0 && cl_bases(cb, a.slots)[max(slot0, 0)] == (int)v0);
         for (; leads; leads &= leads - 1) {
             const int src = __ffs(leads) - 1;
             const int slot = __shfl_sync(0xffffffffu, slot0, src);
-            const int64_t base = w * 32 + src;
+            const int64_t base = w * a.per + src;
             const uint64_t mask = cl_masks(cb)[slot];
             const int n = popc64(mask);
             for (int k = lane; k < n; k += 32) {
@@ -375,9 +377,9 @@ __global__ void __launch_bounds__(BRICK_CTA) k_cl_join(ClArgs a, lw_cluster_buf 
     const int m = *cb.m;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int R = a.reach;
-    for (int64_t j0 = (int64_t)blockIdx.x * 32; j0 < m; j0 += (int64_t)gridDim.x * 32) {
+    for (int64_t j0 = (int64_t)blockIdx.x * a.per; j0 < m; j0 += (int64_t)gridDim.x * a.per) {
         const int64_t v = j0 + lane;
-        const bool live = v < m;
+        const bool live = lane < a.per && v < m;
         const int slot = live ? cl_brick(cb)[v] : -1;
         float px = 0.f, py = 0.f, pz = 0.f;
         int me = 0;
@@ -464,21 +466,21 @@ __global__ void k_cl_uf_flatten(lw_cluster_buf cb) {
 }
 
 // Per-root statistics: exact fixed-point sums and point counts (in the root's own voxel sums), float min / max of the
-// node centroids. Most nodes of a scene share one root, so a warp takes 32 x CL_RUN consecutive nodes, each lane gathers
+// node centroids. Most nodes of a scene share one root, so a warp takes up to 32 x CL_RUN consecutive nodes, each lane gathers
 // what belongs to the warp's usual root in registers and the warp adds it with ten atomics; the other nodes add their own
 // (1.0 ms for 0.3M nodes when every node did, on the same ten words).
-constexpr int CL_RUN = 16;
+constexpr int CL_RUN = 16;  // fewer where not every SM would get a warp: each round is a chain of loads
 
-__global__ void k_cl_stats(lw_cluster_buf cb) {
+__global__ void k_cl_stats(lw_cluster_buf cb, int run) {
     const int m = *cb.m;
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t j0 = warp * 32 * CL_RUN; j0 < m; j0 += nwarps * 32 * CL_RUN) {
+    for (int64_t j0 = warp * 32 * run; j0 < m; j0 += nwarps * 32 * run) {
         long long sum[4] = {0, 0, 0, 0};
         float lo[3] = {1.0e30f, 1.0e30f, 1.0e30f}, hi[3] = {-1.0e30f, -1.0e30f, -1.0e30f};
         int usual = -1;
-        for (int u = 0; u < CL_RUN; ++u) {
+        for (int u = 0; u < run; ++u) {
             const int64_t j = j0 + 32 * u + lane;
             const int r = j < m ? cb.label[j] : -1;
             const bool other = r >= 0 && r != (int)j;  // a root's own sums are in place
@@ -651,6 +653,9 @@ int lw_cluster(const float* xyz, int32_t xyz_stride, const int32_t* gnd, int32_t
     a.min_pts = min_pts;
     a.max_out = max_out;
     const int sms = device_sms();
+    a.per = brick_voxels(n_ub, sms);
+    const int64_t run = n_ub / (32 * (int64_t)sms);
+    a.run = run < 1 ? 1 : run > CL_RUN ? CL_RUN : (int)run;
     int grid = blocks_for(n_ub, 256, 8 * sms);
     int nt = blocks_for(n_ub, CTILE);
     ProfScope prof("cluster", s);
@@ -667,11 +672,11 @@ int lw_cluster(const float* xyz, int32_t xyz_stride, const int32_t* gnd, int32_t
     k_cl_node_count<<<nt, CTILE, 0, s>>>(n_dev, n_ub, *cb);
     k_cl_node_scatter<<<nt, CTILE, 0, s>>>(n_dev, n_ub, *cb);
     // at most one node per point
-    const int gridj = blocks_for(n_ub, 32, 64 * sms);
-    k_cl_brick<<<blocks_for(n_ub, 32 * CL_WARPS, 64 * sms), 32 * CL_WARPS, 0, s>>>(a, *cb);
+    const int gridj = blocks_for(n_ub, a.per, 64 * sms);
+    k_cl_brick<<<blocks_for(n_ub, a.per * CL_WARPS, 64 * sms), 32 * CL_WARPS, 0, s>>>(a, *cb);
     k_cl_join<<<gridj, BRICK_CTA, 0, s>>>(a, *cb);
     k_cl_uf_flatten<<<grid, 256, 0, s>>>(*cb);
-    k_cl_stats<<<blocks_for((n_ub + CL_RUN - 1) / CL_RUN, 128, 16 * sms), 128, 0, s>>>(*cb);
+    k_cl_stats<<<blocks_for((n_ub + a.run - 1) / a.run, 128, 16 * sms), 128, 0, s>>>(*cb, a.run);
     k_cl_flag<<<nt, CTILE, 0, s>>>(*cb, a);
     k_cl_compact<<<nt, CTILE, 0, s>>>(*cb, a);
     k_cl_gather<<<grid, 256, 0, s>>>(n_dev, n_ub, *cb, out_cid);
