@@ -383,12 +383,12 @@ typedef struct lw_nbr_buf {
     int32_t* vidx;       /* [cap] upper half of each brick's mask of occupied voxels */
     int32_t* v_slot;     /* [cap] lower half */
     int32_t* slot_of_pt; /* [pt_cap] voxel of each point, -1 when the table was full */
-    float* v_xyz;        /* [cap*3] not used */
+    float* v_xyz;        /* not used, not NULL */
     int32_t* v_w;        /* [cap] number of each brick's first voxel */
     float* v_cnt;        /* [cap] point-weighted neighbour count (a voxel's brick before that) */
     float* v_nrm;        /* [cap*3] unit normals */
     float* v_curv;       /* [cap] curvature */
-    int32_t* tiles;      /* [cap/1024 + 1] not used */
+    int32_t* tiles;      /* not used, not NULL */
     int32_t* m;          /* [1] voxels */
     int64_t cap, pt_cap;
 } lw_nbr_buf;
@@ -500,15 +500,15 @@ int lw_ground(const float* xyz, int32_t xyz_stride, const float* nrm, const int3
 typedef struct lw_cluster_buf {
     int64_t* keys;       /* [cap] brick keys, -1 empty */
     int64_t* acc;        /* [cap*4] the bricks' masks of occupied voxels and first voxels */
-    int32_t* first;      /* [cap] not used */
-    int32_t* vidx;       /* [cap] not used */
+    int32_t* first;      /* not used */
+    int32_t* vidx;       /* not used */
     int32_t* slot_of_pt; /* [pt_cap] voxel of a point, -1 for ground and when the table was full */
     int32_t* tiles;      /* [pt_cap/1024 + 2] */
     int32_t* node_slot;  /* [pt_cap] voxel of a node */
     float* v_xyz;        /* [pt_cap*3] node centroids */
     int32_t* v_w;        /* [pt_cap] node point counts */
     int32_t* edge_off;   /* [pt_cap + 1] node of a voxel */
-    int32_t* edges;      /* [edge_cap] not used (may be NULL with edge_cap 0) */
+    int32_t* edges;      /* not used */
     int32_t* label;      /* [pt_cap] component of a node: its smallest node index */
     int64_t* st_sum;     /* [pt_cap*4] per-voxel, then per-root fixed-point sums and count */
     float* st_lo;        /* [pt_cap*3] per-root minimum corner */
@@ -693,14 +693,14 @@ int lw_net_forward(const lw_initnet* net, const float* sets, int32_t n, float* p
 typedef struct lw_net_scratch {
     float* dz3;       /* [2n*256] gradient of each channel's argmax point */
     uint16_t* h2g;    /* [2n*256*128] bf16: layer-2 activations of each set's distinct argmax points */
-    float* d2t;       /* [128][2n*256] CTAs' sums of the layer-1 and layer-2 gradients */
-    float* h1t;       /* [65][2n*256] not used */
-    float* d1t;       /* [64][2n*256] not used */
-    float* xt;        /* [4][2n*256] place of each channel's point among its set's (int32) */
+    float* d2t;       /* [2n*8576] CTAs' sums of the layer-1 and layer-2 gradients (at most a CTA per set) */
+    float* h1t;       /* not used */
+    float* d1t;       /* not used */
+    float* xt;        /* [2n*256] place of each channel's point among its set's (int32) */
     float* dzh;       /* [n][128] */
     float* dout;      /* [n][6] */
     float* dpool;     /* [2n][256] */
-    float* part;      /* [64 * 8448] not used */
+    float* part;      /* not used */
     float* loss;      /* [n] per-sample loss */
     int32_t n_cap;
     int32_t pad_;

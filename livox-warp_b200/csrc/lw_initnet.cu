@@ -1031,7 +1031,8 @@ int lw_net_backward(const lw_initnet* net, const float* sets, int32_t n, const f
         LW_CUDA(cudaFuncSetAttribute(k_net_pt_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PtSmem)));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    // d2t holds the CTAs' sums (at most one CTA per set, 32768 floats of d2t per set), xt the channels' places
+    // d2t holds the CTAs' sums (at most one CTA per set), xt the channels' places
+    static_assert(PB_PART == 8576, "d2t's floats per set");
     const int ctas = n_sets < 2 * device_sms() ? n_sets : 2 * device_sms();
     int32_t* place = reinterpret_cast<int32_t*>(scr->xt);
     k_net_pt_bwd<<<ctas, PB_T, sizeof(PtSmem), s>>>(net->w, net->in_scale, reinterpret_cast<const float4*>(sets), pooled,

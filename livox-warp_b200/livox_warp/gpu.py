@@ -469,12 +469,12 @@ class Pipeline:
                           "vidx": torch.zeros(cap, dtype=torch.int32, device=d),
                           "v_slot": torch.zeros(cap, dtype=torch.int32, device=d),
                           "slot_of_pt": torch.zeros(self.work_cap, dtype=torch.int32, device=d),
-                          "v_xyz": torch.zeros((cap, 3), dtype=torch.float32, device=d),
+                          "v_xyz": torch.zeros(1, dtype=torch.float32, device=d),  # not used
                           "v_w": torch.zeros(cap, dtype=torch.int32, device=d),
                           "v_cnt": torch.zeros(cap, dtype=torch.float32, device=d),
                           "v_nrm": torch.zeros((cap, 3), dtype=torch.float32, device=d),
                           "v_curv": torch.zeros(cap, dtype=torch.float32, device=d),
-                          "tiles": torch.zeros(cap // 1024 + 2, dtype=torch.int32, device=d),
+                          "tiles": torch.zeros(1, dtype=torch.int32, device=d),  # not used
                           "m": torch.zeros(1, dtype=torch.int32, device=d)}
             self._nb = _lib.NbrBuf(*(_lib.ptr(self._nb_t[k]).value for k in _lib.NbrBuf.PTRS), cap, self.work_cap)
         t0 = time.perf_counter()

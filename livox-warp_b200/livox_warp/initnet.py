@@ -75,9 +75,10 @@ class InitNet:
         d = self.device
         K = 2 * n * 256
         f = lambda *shape: torch.zeros(*shape, dtype=torch.float32, device=d)  # noqa: E731
-        self._scr = {"dz3": f(K), "h2g": torch.zeros(K * 128, dtype=torch.int16, device=d), "d2t": f(128 * K),
-                     "h1t": f(65 * K), "d1t": f(64 * K), "xt": f(4 * K), "dzh": f(n * 128), "dout": f(n * 6),
-                     "dpool": f(n * 512), "part": f(64 * 8448), "loss": f(n)}
+        # h1t, d1t and part are not used
+        self._scr = {"dz3": f(K), "h2g": torch.zeros(K * 128, dtype=torch.int16, device=d), "d2t": f(2 * n * 8576),
+                     "h1t": f(1), "d1t": f(1), "xt": f(K), "dzh": f(n * 128), "dout": f(n * 6),
+                     "dpool": f(n * 512), "part": f(1), "loss": f(n)}
         self.scr = _lib.NetScratch(*(_lib.ptr(self._scr[k]).value for k in _lib.NetScratch.PTRS), n, 0)
         self._fwd = {"pooled": f(n * 512), "argmax": torch.zeros(n * 512, dtype=torch.int32, device=d),
                      "hid": f(n * 128), "step": f(n * 6), "err": torch.zeros(1, dtype=torch.int32, device=d)}

@@ -117,7 +117,8 @@ class Tracker:
 
 
 class Perception:
-    """Ground labels, clusters and tracks of the pipeline's visible points (perception.py:391)."""
+    """Ground labels, clusters and tracks of the pipeline's visible points (perception.py:391). cluster_slots bounds the
+    clusters' table; edge_factor sizes nothing, since no edge list is kept."""
 
     def __init__(self, pipe: Pipeline, device=None, cluster_slots: int = 1 << 20, edge_factor: int = 64):
         _lib.load()
@@ -135,15 +136,15 @@ class Perception:
         self._t = {
             "keys": torch.full((c,), -1, dtype=torch.int64, device=d),
             "acc": torch.zeros((c, 4), dtype=torch.int64, device=d),
-            "first": torch.full((c,), _lib.INT32_MAX, dtype=torch.int32, device=d),
-            "vidx": torch.zeros(c, dtype=torch.int32, device=d),
+            "first": torch.zeros(1, dtype=torch.int32, device=d),  # not used
+            "vidx": torch.zeros(1, dtype=torch.int32, device=d),  # not used
             "slot_of_pt": torch.zeros(n, dtype=torch.int32, device=d),
             "tiles": torch.zeros(n // 1024 + 2, dtype=torch.int32, device=d),
             "node_slot": torch.zeros(n, dtype=torch.int32, device=d),
             "v_xyz": torch.zeros((n, 3), dtype=torch.float32, device=d),
             "v_w": torch.zeros(n, dtype=torch.int32, device=d),
             "edge_off": torch.zeros(n + 1, dtype=torch.int32, device=d),
-            "edges": torch.zeros(1, dtype=torch.int32, device=d),  # no edge list is kept (edge_factor sizes nothing)
+            "edges": torch.zeros(1, dtype=torch.int32, device=d),  # not used
             "label": torch.zeros(n, dtype=torch.int32, device=d),
             "st_sum": torch.zeros((n, 4), dtype=torch.int64, device=d),
             "st_lo": torch.full((n, 3), 1.0e30, dtype=torch.float32, device=d),
