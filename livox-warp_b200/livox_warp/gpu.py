@@ -207,7 +207,8 @@ class Pipeline:
         self.cl_tid = torch.full((MAX_CLUSTERS,), -1, dtype=torch.int32, device=d)
         self._slot = torch.zeros(n, dtype=torch.int32, device=d)  # per-point scratch of the insert passes
         self._carve_rays, self._carve_t, self._carve_buf = 0, [], None  # lw_carve_ws's workspace
-        self._carve_lock, self._carve_stream = threading.Lock(), None  # held while a carve is launched; the last one's stream
+        # held while a carve is launched; the end of the last one (an event: its stream may be gone by the next)
+        self._carve_lock, self._carve_done = threading.Lock(), torch.cuda.Event()
         self._carve_marks = torch.zeros(m, dtype=torch.int32, device=d)  # its own: an insertion may run beside a carve
         self._carve_ws(1 << 15)  # what a frame takes, made here so that no frame waits for an allocation
         self._tiles = torch.zeros(max(m, self.cap) // 1024 + 2, dtype=torch.int32, device=d)
@@ -387,25 +388,15 @@ class Pipeline:
         s = torch.cuda.current_stream()
         with self._carve_lock:
             ws = self._carve_ws(rays)
-            self._carve_turn(s)
+            # a capture neither waits (what it records runs later) nor is waited for
+            capturing = torch.cuda.is_current_stream_capturing()
+            if not capturing:
+                s.wait_event(self._carve_done)
             _lib.call("lw_carve_ws", _lib.ptr(sx), row_stride(sx), _lib.ptr(sa), _lib.ptr(sf), _lib.ptr(n_dev), n,
                       _lib.ptr(self.poses), every, 1.0 / max(voxel, 1e-4), float(max_range), int(max_steps),
                       C_ref(self.map_struct), _lib.ptr(self._carve_t[-1][-1]), C_ref(ws), _lib.stream_ptr(s))
-
-    def _carve_turn(self, s):
-        """Let stream `s` wait for the carve before when that went to another stream. A capture neither waits (what it
-        records runs later) nor is waited for."""
-        last = self._carve_stream
-        if last is not None and last.cuda_stream == s.cuda_stream:
-            return
-        if torch.cuda.is_current_stream_capturing():
-            return
-        if last is not None:
-            with torch.cuda.stream(last):
-                capturing = torch.cuda.is_current_stream_capturing()
             if not capturing:
-                s.wait_stream(last)
-        self._carve_stream = s
+                self._carve_done.record(s)
 
     def _carve_ws(self, rays: int) -> _lib.CarveBuf:
         """lw_carve_ws's workspace for at least `rays` rays. It grows by doubling, and the smaller ones are kept: a

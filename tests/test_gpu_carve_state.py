@@ -99,3 +99,26 @@ def test_a_captured_carve_counts_like_an_eager_one(mapped):
     got = pipe.map_miss.clone()
     pipe.map_miss.zero_()
     assert torch.equal(got, 3 * want)
+
+
+def test_the_stream_of_the_carve_before_may_be_gone(mapped):
+    """A carve on a stream the caller made and has destroyed since, then one on another stream: nothing of the first
+    stream is kept."""
+    import ctypes
+
+    pipe, (sx, sa, sf) = mapped
+    want = _want(pipe, sx, sa, sf, 2)
+    cudart = torch.cuda.cudart()
+    raw = ctypes.c_void_p()
+    assert int(cudart.cudaStreamCreate(ctypes.addressof(raw))) == 0
+    stream = torch.cuda.ExternalStream(raw.value)
+    with torch.cuda.stream(stream):
+        pipe.carve(sx, sa, sf, len(sf), VOXEL, every=2)
+    stream.synchronize()
+    del stream
+    assert int(cudart.cudaStreamDestroy(raw.value)) == 0
+    pipe.carve(sx, sa, sf, len(sf), VOXEL, every=2)
+    torch.cuda.synchronize()
+    got = pipe.map_miss.clone()
+    pipe.map_miss.zero_()
+    assert torch.equal(got, 2 * want)
