@@ -114,6 +114,12 @@ def _plain(x, n: int, dtype) -> bool:
             and (dtype is None or x.dtype == dtype))
 
 
+def _foreign(s) -> bool:
+    """Whether the stream was made outside torch (torch.cuda.ExternalStream, whose id is its handle): such a stream can be
+    destroyed; torch's own last as long as the process."""
+    return s.cuda_stream != 0 and s.stream_id == s.cuda_stream
+
+
 def _as_xyz(x, device) -> torch.Tensor:
     """Device float32 points of shape (n, 3) or (n, 4) (x, y, z, anything), contiguous, or the (n, 3) x, y, z
     columns of an (n, 4) buffer (rows 4 floats apart: the frame an on_frame callback is handed)."""
@@ -207,8 +213,8 @@ class Pipeline:
         self.cl_tid = torch.full((MAX_CLUSTERS,), -1, dtype=torch.int32, device=d)
         self._slot = torch.zeros(n, dtype=torch.int32, device=d)  # per-point scratch of the insert passes
         self._carve_rays, self._carve_t, self._carve_buf = 0, [], None  # lw_carve_ws's workspace
-        # held while a carve is launched; the end of the last one (an event: its stream may be gone by the next)
-        self._carve_lock, self._carve_done = threading.Lock(), torch.cuda.Event()
+        self._carve_lock = threading.Lock()  # held while a carve is launched
+        self._carve_stream, self._carve_done = None, torch.cuda.Event()  # the last one's stream; its end (see _carve_wait)
         self._carve_marks = torch.zeros(m, dtype=torch.int32, device=d)  # its own: an insertion may run beside a carve
         self._carve_ws(1 << 15)  # what a frame takes, made here so that no frame waits for an allocation
         self._tiles = torch.zeros(max(m, self.cap) // 1024 + 2, dtype=torch.int32, device=d)
@@ -387,19 +393,36 @@ class Pipeline:
         rays = (n + every - 1) // every
         s = torch.cuda.current_stream()
         with self._carve_lock:
-            ws = self._carve_ws(rays)
+            ws, stop = self._carve_ws(rays)
             # a capture neither waits (what it records runs later) nor is waited for
             capturing = torch.cuda.is_current_stream_capturing()
             if not capturing:
-                s.wait_event(self._carve_done)
+                self._carve_wait(s)
             _lib.call("lw_carve_ws", _lib.ptr(sx), row_stride(sx), _lib.ptr(sa), _lib.ptr(sf), _lib.ptr(n_dev), n,
                       _lib.ptr(self.poses), every, 1.0 / max(voxel, 1e-4), float(max_range), int(max_steps),
-                      C_ref(self.map_struct), _lib.ptr(self._carve_t[-1][-1]), C_ref(ws), _lib.stream_ptr(s))
+                      C_ref(self.map_struct), stop, ws, _lib.stream_ptr(s))
             if not capturing:
-                self._carve_done.record(s)
+                if _foreign(s):
+                    self._carve_done.record(s)
+                self._carve_stream = s
 
-    def _carve_ws(self, rays: int) -> _lib.CarveBuf:
-        """lw_carve_ws's workspace for at least `rays` rays. It grows by doubling, and the smaller ones are kept: a
+    def _carve_wait(self, s):
+        """Let stream `s` wait for the carve before, unless that went to the same stream. A stream of the caller's own
+        making may be gone by now: of one the end of its carve is kept as an event, and nothing else. (An event for
+        every carve took 14 us of the host a call.)"""
+        last = self._carve_stream
+        if last is None:
+            return
+        if _foreign(last):
+            s.wait_event(self._carve_done)
+        elif last.cuda_stream != s.cuda_stream:
+            with torch.cuda.stream(last):
+                capturing = torch.cuda.is_current_stream_capturing()
+            if not capturing:  # (torch.cuda.graph starts a capture on an idle device)
+                s.wait_stream(last)
+
+    def _carve_ws(self, rays: int):
+        """lw_carve_ws's workspace for at least `rays` rays, and where each ray's stop goes. It grows by doubling, and the smaller ones are kept: a
         stream other than the one they were made on may still be using them."""
         if rays > self._carve_rays:
             r = 1 << (rays - 1).bit_length()
@@ -410,8 +433,8 @@ class Pipeline:
                  torch.empty(r, dtype=torch.float32, device=d))  # the last: where each ray stops
             self._carve_t.append(t)
             self._carve_buf = _lib.CarveBuf(*(_lib.ptr(x) for x in t[:5]), pairs, slots, _lib.ptr(self._carve_marks))
-            self._carve_rays = r
-        return self._carve_buf
+            self._carve_rays, self._carve_refs = r, (C_ref(self._carve_buf), _lib.ptr(t[5]))
+        return self._carve_refs
 
     def ingest(self, xyz, attr, t, n: int, view: View, map_on: bool, voxel: float):
         """Stage, ring and map in one call, without odometry (gpu.py:1454-1462)."""

@@ -106,12 +106,15 @@ def test_the_stream_of_the_carve_before_may_be_gone(mapped):
     stream is kept."""
     import ctypes
 
+    from livox_warp import gpu
+
     pipe, (sx, sa, sf) = mapped
     want = _want(pipe, sx, sa, sf, 2)
     cudart = torch.cuda.cudart()
     raw = ctypes.c_void_p()
     assert int(cudart.cudaStreamCreate(ctypes.addressof(raw))) == 0
     stream = torch.cuda.ExternalStream(raw.value)
+    assert gpu._foreign(stream) and not gpu._foreign(torch.cuda.Stream()) and not gpu._foreign(torch.cuda.current_stream())
     with torch.cuda.stream(stream):
         pipe.carve(sx, sa, sf, len(sf), VOXEL, every=2)
     stream.synchronize()
