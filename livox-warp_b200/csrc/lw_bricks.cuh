@@ -64,6 +64,34 @@ inline int64_t brick_slots(int64_t n, int64_t cap) {
 
 __device__ __forceinline__ int popc64(uint64_t v) { return __popcll(v); }
 
+// The slot of each lane's brick (every lane calls; live: the lane has a point; -1 without room), claimed where it has none
+// yet, and the points' voxels marked: mark(s, bits) sets `bits` in the mask of the brick in slot s.
+// Every point finds the table empty when a call starts, and the L2 takes one operation a cycle on a word: with a claim and a
+// mark a point, 200,000 points of one brick take 60 us. So a brick is claimed by one of the warp's lanes in it, and marked by
+// that one too where eight or more share it: 8 us.
+constexpr int BRICK_SHARED = 8;
+
+template <class Mark>
+__device__ __forceinline__ int enter_brick(bool live, int64_t key, int bit, int64_t* keys, int mask, const Mark& mark) {
+    constexpr unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned group = __match_any_sync(full, (unsigned long long)(live ? key : EMPTY_KEY));
+    const int leader = __ffs(group) - 1;
+    int s = -1;
+    if (live && lane == leader) s = claim_brick(key, keys, mask);
+    s = __shfl_sync(full, s, leader);
+    uint64_t bits = live && s >= 0 ? 1ull << bit : 0ull;
+    for (unsigned b = __ballot_sync(full, live && lane == leader && __popc(group) >= BRICK_SHARED); b; b &= b - 1) {
+        const int lead = __ffs(b) - 1;
+        const bool in = leader == lead;
+        const unsigned lo = __reduce_or_sync(full, in ? (unsigned)bits : 0u);
+        const unsigned hi = __reduce_or_sync(full, in ? (unsigned)(bits >> 32) : 0u);
+        if (in) bits = lane == lead ? (uint64_t)lo | (uint64_t)hi << 32 : 0ull;
+    }
+    if (bits) mark(s, bits);
+    return s;
+}
+
 // The n-th set bit of a mask, from 0.
 __device__ __forceinline__ int nth_bit(uint64_t mask, int n) {
     uint32_t h = (uint32_t)mask;

@@ -174,6 +174,20 @@ __device__ __forceinline__ float atomic_max_float(float* a, float v) {
 __device__ __forceinline__ void atomic_add_i64(int64_t* a, int64_t v) {
     atomicAdd((unsigned long long*)a, (unsigned long long)v);
 }
+// N 64-bit integers in shared memory added to N in global memory in one asynchronous operation; both 16-byte aligned, N
+// even. The shared ones are free again once bulk_read_wait returns, the sums are there once bulk_wait does.
+template <int N>
+__device__ __forceinline__ void bulk_add(int64_t* dst, const int64_t* src) {
+    static_assert(N % 2 == 0, "a multiple of 16 bytes");
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(src);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.u64 [%0], [%1], %2;" ::"l"(dst), "r"(at), "n"(8 * N)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_read_wait() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 // float -> int64 fixed point, round to nearest even (llrintf on the host).
 __device__ __forceinline__ int64_t to_fix(float v, float scale) { return __float2ll_rn(v * scale); }
 

@@ -132,6 +132,7 @@ struct ClArgs {
     int mask, use_gnd;
     int64_t slots;  // brick slots used
     int per;        // voxels that a warp of k_cl_brick and a CTA of k_cl_join take at a time
+    int sms;
     int run;        // rounds of 32 nodes a warp of k_cl_stats takes
     float connect2;
     int reach;
@@ -162,20 +163,22 @@ __global__ void k_cl_insert(const float* __restrict__ xyz, const int* __restrict
                             int64_t n_ub, ClArgs a, lw_cluster_buf cb) {
     int64_t n = n_dev ? (int64_t)*n_dev : n_ub;
     if (n > n_ub) n = n_ub;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        int s = -1;
-        if (!(a.use_gnd && gnd[i] != 0)) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < n; i0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = i0 + lane;
+        const bool live = i < n && !(a.use_gnd && gnd[i] != 0);
+        int bit = 0;
+        int64_t key = EMPTY_KEY;
+        if (live) {
             float x, y, z;
             ld3<STRIDE>(xyz, i, x, y, z);
-            int bit;
-            const int64_t key = brick_of(ifloor(x * a.inv_v), ifloor(y * a.inv_v), ifloor(z * a.inv_v), bit);
-            s = claim_brick(key, cb.keys, a.mask);
-            if (s >= 0) {
-                uint64_t* m = cl_masks(cb) + s;
-                if ((*(volatile uint64_t*)m >> bit & 1) == 0) atomicOr((unsigned long long*)m, 1ull << bit);
-            }
+            key = brick_of(ifloor(x * a.inv_v), ifloor(y * a.inv_v), ifloor(z * a.inv_v), bit);
         }
-        cb.slot_of_pt[i] = s;
+        const int s = enter_brick(live, key, bit, cb.keys, a.mask, [&](int slot, uint64_t bits) {
+            uint64_t* m = cl_masks(cb) + slot;
+            if ((~*(volatile uint64_t*)m & bits) != 0) atomicOr((unsigned long long*)m, (unsigned long long)bits);
+        });
+        if (i < n) cb.slot_of_pt[i] = s;
     }
 }
 
@@ -188,12 +191,19 @@ __global__ void __launch_bounds__(CTILE) k_cl_number(lw_cluster_buf cb, ClArgs a
     });
 }
 
-// Pass 3: exact fixed-point sums per voxel, and the lowest point index (it orders the nodes).
-template <int STRIDE>
-__global__ void k_cl_sum(const float* __restrict__ xyz, const int* n_dev, int64_t n_ub, ClArgs a, lw_cluster_buf cb) {
+// Pass 3: exact fixed-point sums per voxel (BULK: by one 32-byte reduction a point, as in k_nb_sum; it needs st_sum 16-byte
+// aligned, other buffers take the atomics), and the lowest point index (it orders the nodes; read before its atomic
+// minimum: a value read can only be too high, and then the atomic decides).
+constexpr int CL_SUM_CTA = 256;
+
+template <int STRIDE, bool BULK>
+__global__ void __launch_bounds__(CL_SUM_CTA) k_cl_sum(const float* __restrict__ xyz, const int* n_dev, int64_t n_ub,
+                                                       ClArgs a, lw_cluster_buf cb) {
     int64_t n = n_dev ? (int64_t)*n_dev : n_ub;
     if (n > n_ub) n = n_ub;
     const float FW = (float)LW_FIX_W;
+    __shared__ __align__(16) int64_t row[CL_SUM_CTA][4];
+    int64_t* const mine = row[threadIdx.x];
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int s = cb.slot_of_pt[i];
         if (s < 0) continue;
@@ -202,13 +212,30 @@ __global__ void k_cl_sum(const float* __restrict__ xyz, const int* n_dev, int64_
         int bit;
         brick_of(ifloor(x * a.inv_v), ifloor(y * a.inv_v), ifloor(z * a.inv_v), bit);
         const int64_t v = (int64_t)cl_bases(cb, a.slots)[s] + popc64(cl_masks(cb)[s] & ((1ull << bit) - 1));
-        atomic_add_i64(cb.st_sum + 4 * v + 0, to_fix(x, FW));
-        atomic_add_i64(cb.st_sum + 4 * v + 1, to_fix(y, FW));
-        atomic_add_i64(cb.st_sum + 4 * v + 2, to_fix(z, FW));
-        atomic_add_i64(cb.st_sum + 4 * v + 3, 1);
-        atomicMin(cb.dense + v, (int)i);
+        if (BULK) {
+            bulk_read_wait();
+            reinterpret_cast<longlong2*>(mine)[0] = make_longlong2(to_fix(x, FW), to_fix(y, FW));
+            reinterpret_cast<longlong2*>(mine)[1] = make_longlong2(to_fix(z, FW), 1);
+            bulk_add<4>(cb.st_sum + 4 * v, mine);
+        } else {
+            atomic_add_i64(cb.st_sum + 4 * v + 0, to_fix(x, FW));
+            atomic_add_i64(cb.st_sum + 4 * v + 1, to_fix(y, FW));
+            atomic_add_i64(cb.st_sum + 4 * v + 2, to_fix(z, FW));
+            atomic_add_i64(cb.st_sum + 4 * v + 3, 1);
+        }
+        if ((int)i < *(volatile int32_t*)(cb.dense + v)) atomicMin(cb.dense + v, (int)i);
         cb.slot_of_pt[i] = (int)v;
     }
+    if (BULK) bulk_wait();
+}
+
+template <int STRIDE>
+void cl_sum(const float* xyz, const int* n_dev, int64_t n_ub, const ClArgs& a, const lw_cluster_buf& cb, cudaStream_t s) {
+    const int grid = blocks_for(n_ub, CL_SUM_CTA, 8 * a.sms);
+    if (((uintptr_t)cb.st_sum & 15) == 0)
+        k_cl_sum<STRIDE, true><<<grid, CL_SUM_CTA, 0, s>>>(xyz, n_dev, n_ub, a, cb);
+    else
+        k_cl_sum<STRIDE, false><<<grid, CL_SUM_CTA, 0, s>>>(xyz, n_dev, n_ub, a, cb);
 }
 
 // Pass 4/5: the nodes are the voxels in the order of their first point: per-tile counts, then the scatter.
@@ -654,6 +681,7 @@ int lw_cluster(const float* xyz, int32_t xyz_stride, const int32_t* gnd, int32_t
     a.max_out = max_out;
     const int sms = device_sms();
     a.per = brick_voxels(n_ub, sms);
+    a.sms = sms;
     const int64_t run = n_ub / (32 * (int64_t)sms);
     a.run = run < 1 ? 1 : run > CL_RUN ? CL_RUN : (int)run;
     int grid = blocks_for(n_ub, 256, 8 * sms);
@@ -666,9 +694,9 @@ int lw_cluster(const float* xyz, int32_t xyz_stride, const int32_t* gnd, int32_t
         k_cl_insert<3><<<grid, 256, 0, s>>>(xyz, gnd, n_dev, n_ub, a, *cb);
     k_cl_number<<<blocks_for(a.slots, CTILE), CTILE, 0, s>>>(*cb, a);
     if (xyz_stride == 4)
-        k_cl_sum<4><<<grid, 256, 0, s>>>(xyz, n_dev, n_ub, a, *cb);
+        cl_sum<4>(xyz, n_dev, n_ub, a, *cb, s);
     else
-        k_cl_sum<3><<<grid, 256, 0, s>>>(xyz, n_dev, n_ub, a, *cb);
+        cl_sum<3>(xyz, n_dev, n_ub, a, *cb, s);
     k_cl_node_count<<<nt, CTILE, 0, s>>>(n_dev, n_ub, *cb);
     k_cl_node_scatter<<<nt, CTILE, 0, s>>>(n_dev, n_ub, *cb);
     // at most one node per point

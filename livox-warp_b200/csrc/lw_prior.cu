@@ -56,18 +56,6 @@ __device__ __forceinline__ void key_unpack(int64_t key, int& ix, int& iy, int& i
 
 // ---- voxel downsample -------------------------------------------------------------------------------------------
 
-// 64 bytes of shared memory added to 64 of global memory as eight 64-bit integers, in one asynchronous operation; both
-// 16-byte aligned. The shared bytes are free again once bulk_read_wait returns.
-__device__ __forceinline__ void bulk_add8(int64_t* dst, const int64_t* src) {
-    const uint32_t at = (uint32_t)__cvta_generic_to_shared(src);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.u64 [%0], [%1], 64;" ::"l"(dst), "r"(at)
-                 : "memory");
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
-__device__ __forceinline__ void bulk_read_wait() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
 constexpr int VX_CTA = 256;
 
 // Each point claims its voxel and adds its offset from the voxel centre, colour, intensity and 1 (k_vox_insert).
@@ -103,7 +91,7 @@ __global__ void __launch_bounds__(VX_CTA) k_vox_insert(const float* __restrict__
             bulk_read_wait();
 #pragma unroll
             for (int c = 0; c < 4; ++c) reinterpret_cast<longlong2*>(mine)[c] = make_longlong2(v[2 * c], v[2 * c + 1]);
-            bulk_add8(acc, mine);
+            bulk_add<8>(acc, mine);
         } else {
 #pragma unroll
             for (int c = 0; c < 8; ++c)
