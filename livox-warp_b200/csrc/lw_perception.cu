@@ -133,7 +133,6 @@ struct ClArgs {
     int64_t slots;  // brick slots used
     int per;        // voxels that a warp of k_cl_brick and a CTA of k_cl_join take at a time
     int sms;
-    int run;        // rounds of 32 nodes a warp of k_cl_stats takes
     float connect2;
     int reach;
     float min_pts;
@@ -496,10 +495,13 @@ __global__ void k_cl_uf_flatten(lw_cluster_buf cb) {
 // node centroids. Most nodes of a scene share one root, so a warp takes up to 32 x CL_RUN consecutive nodes, each lane gathers
 // what belongs to the warp's usual root in registers and the warp adds it with ten atomics; the other nodes add their own
 // (1.0 ms for 0.3M nodes when every node did, on the same ten words).
-constexpr int CL_RUN = 16;  // fewer where not every SM would get a warp: each round is a chain of loads
+// A round is a chain of loads, so there are several only where every SM gets eight warps all the same: 210,000 points in 300
+// clumps take 36 us by rounds counted by the points, 5 by the nodes; a room of 400,000 points, 15 and 3.
+constexpr int CL_RUN = 16;
 
-__global__ void k_cl_stats(lw_cluster_buf cb, int run) {
+__global__ void k_cl_stats(lw_cluster_buf cb, ClArgs a) {
     const int m = *cb.m;
+    const int run = max(1, min(CL_RUN, m / (32 * 8 * a.sms)));
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -514,7 +516,7 @@ __global__ void k_cl_stats(lw_cluster_buf cb, int run) {
             const unsigned some = __ballot_sync(0xffffffffu, other);
             if (some == 0) continue;
             if (usual < 0) {
-                // the root that most of the first lanes share: the median lane's
+                // the first such lane's root, or, where most of the others have another, the first of those lanes'
                 usual = __shfl_sync(0xffffffffu, r, __ffs(some) - 1);
                 const unsigned same = __ballot_sync(0xffffffffu, other && r == usual);
                 if (2 * __popc(same) < __popc(some)) {
@@ -682,8 +684,6 @@ int lw_cluster(const float* xyz, int32_t xyz_stride, const int32_t* gnd, int32_t
     const int sms = device_sms();
     a.per = brick_voxels(n_ub, sms);
     a.sms = sms;
-    const int64_t run = n_ub / (32 * (int64_t)sms);
-    a.run = run < 1 ? 1 : run > CL_RUN ? CL_RUN : (int)run;
     int grid = blocks_for(n_ub, 256, 8 * sms);
     int nt = blocks_for(n_ub, CTILE);
     ProfScope prof("cluster", s);
@@ -704,7 +704,9 @@ int lw_cluster(const float* xyz, int32_t xyz_stride, const int32_t* gnd, int32_t
     k_cl_brick<<<blocks_for(n_ub, a.per * CL_WARPS, 64 * sms), 32 * CL_WARPS, 0, s>>>(a, *cb);
     k_cl_join<<<gridj, BRICK_CTA, 0, s>>>(a, *cb);
     k_cl_uf_flatten<<<grid, 256, 0, s>>>(*cb);
-    k_cl_stats<<<blocks_for((n_ub + a.run - 1) / a.run, 128, 16 * sms), 128, 0, s>>>(*cb, a.run);
+    // four warps to a CTA: two rounds of eight warps an SM, or CL_RUN rounds of 32 nodes a warp, whichever are more
+    const int full = blocks_for(n_ub, 128 * CL_RUN, 16 * sms);
+    k_cl_stats<<<blocks_for(n_ub, 128, full > 4 * sms ? full : 4 * sms), 128, 0, s>>>(*cb, a);
     k_cl_flag<<<nt, CTILE, 0, s>>>(*cb, a);
     k_cl_compact<<<nt, CTILE, 0, s>>>(*cb, a);
     k_cl_gather<<<grid, 256, 0, s>>>(n_dev, n_ub, *cb, out_cid);
