@@ -735,22 +735,25 @@ __global__ void __launch_bounds__(LS_T) k_loc_sort(lw_loc_batch b, lw_loc_ws ws,
 // (bound by L1's one line a cycle: every lane's loads are lines of their own, about 570 a tile), 0.08 of sums, 0.03 of
 // the tile partials' sums and solves, 0.08 of waiting at the three barriers. The sorted points are read past L1, which
 // the map's lines need.
-template <int MINB>
+// WS: a workspace was handed in (whether a batch's tiles fit it is known on the device alone). Without one, as in an
+// evaluation, the kernel is compiled without the sorted ways, whose registers and shared memory are in its way: 20,000 points
+// at 8 poses 487 us with them, 474 without.
+template <int MINB, bool WS>
 __global__ void __launch_bounds__(LOC_BLOCK, MINB)
     k_loc_icp(lw_prior_grid g, lw_loc_batch b, lw_loc_ws ws, LocArgs la) {
     constexpr bool SMEM_ACC = MINB >= 4;
     __shared__ __align__(16) float s_acc[SMEM_ACC ? LOC_BLOCK / 32 : 1][SMEM_ACC ? LTERMS : 1][32];
     __shared__ LocPose s_pose[SMEM_ACC ? LOC_BLOCK / 32 : 1];
-    __shared__ int2 s_runs[SMEM_ACC ? 1 : LOC_BLOCK / 32][9][32];
+    __shared__ int2 s_runs[SMEM_ACC || !WS ? 1 : LOC_BLOCK / 32][WS ? 9 : 1][32];
     __shared__ double sv[32];
     __shared__ int s_stop;
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int n_hyp = b.dims ? min(__ldg(b.dims), la.n_hyp) : la.n_hyp;
     const int n_tiles = b.dims ? min(__ldg(b.dims + 1), la.n_tiles) : la.n_tiles;
-    const bool sorted = ws.sorted != nullptr && (int64_t)n_tiles * la.tile <= ws.cap;
+    const bool sorted = WS && (int64_t)n_tiles * la.tile <= ws.cap;
     // a search's runs: in the term sums' columns, which are free while searching
-    int2(*runs)[32] = SMEM_ACC ? reinterpret_cast<int2(*)[32]>(&s_acc[tid >> 5][0][0]) : s_runs[SMEM_ACC ? 0 : tid >> 5];
+    int2(*runs)[32] = SMEM_ACC ? reinterpret_cast<int2(*)[32]>(&s_acc[tid >> 5][0][0]) : s_runs[SMEM_ACC || !WS ? 0 : tid >> 5];
     static_assert(sizeof(int2) * 9 * 32 <= sizeof(float) * LTERMS * 32, "a search's runs fit the term sums' columns");
     const int warp_id = (blockIdx.x * LOC_BLOCK + tid) >> 5, n_warps = gridDim.x * (LOC_BLOCK / 32);
     const int grab = max(1, min(8, n_tiles / (4 * n_warps)));
@@ -1552,11 +1555,16 @@ int lw_loc_icp_batch_ws(const lw_prior_grid* g, lw_loc_batch* b, int32_t n_hyp, 
     if (blocks_per_sm == 0) blocks_per_sm = 3;
     if (blocks_per_sm < 2 || blocks_per_sm > 6)
         return set_error(LW_EINVAL, "lw_loc_icp_batch: blocks_per_sm must be 0 or 2..6");
-    const void* fn = blocks_per_sm == 2   ? (const void*)k_loc_icp<2>
-                     : blocks_per_sm == 3 ? (const void*)k_loc_icp<3>
-                     : blocks_per_sm == 4 ? (const void*)k_loc_icp<4>
-                     : blocks_per_sm == 5 ? (const void*)k_loc_icp<5>
-                                          : (const void*)k_loc_icp<6>;
+    // one search per point repays the sorting only where it is repeated
+    lw_loc_ws w{};
+    if (ws && ws->sorted && ws->match && total_iters > 1) w = *ws;
+    if (((uintptr_t)w.sorted & 15) != 0)
+        return set_error(LW_EINVAL, "lw_loc_icp_batch_ws: the sorted points must be 16-byte aligned");
+    using Kernel = void (*)(lw_prior_grid, lw_loc_batch, lw_loc_ws, LocArgs);
+    static const Kernel kernels[2][5] = {
+        {k_loc_icp<2, false>, k_loc_icp<3, false>, k_loc_icp<4, false>, k_loc_icp<5, false>, k_loc_icp<6, false>},
+        {k_loc_icp<2, true>, k_loc_icp<3, true>, k_loc_icp<4, true>, k_loc_icp<5, true>, k_loc_icp<6, true>}};
+    const Kernel fn = kernels[w.sorted ? 1 : 0][blocks_per_sm - 2];
     int per_sm = 0;
     LW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, LOC_BLOCK, 0));
     if (per_sm < 1) return set_error(LW_EINVAL, "lw_loc_icp_batch: the kernel does not fit on an SM");
@@ -1564,11 +1572,6 @@ int lw_loc_icp_batch_ws(const lw_prior_grid* g, lw_loc_batch* b, int32_t n_hyp, 
     if (grid <= 0 || grid > max_grid) grid = max_grid;
     if (grid > b->grid_cap) grid = b->grid_cap;
     ProfScope prof("loc_icp", s);
-    // one search per point repays the sorting only where it is repeated
-    lw_loc_ws w{};
-    if (ws && ws->sorted && ws->match && total_iters > 1) w = *ws;
-    if (((uintptr_t)w.sorted & 15) != 0)
-        return set_error(LW_EINVAL, "lw_loc_icp_batch_ws: the sorted points must be 16-byte aligned");
     k_loc_reset<<<16, 256, 0, s>>>(*b, n_hyp, total_iters);
     if (w.sorted) {
         static bool attr_set[64] = {};
@@ -1594,13 +1597,7 @@ int lw_loc_icp_batch_ws(const lw_prior_grid* g, lw_loc_batch* b, int32_t n_hyp, 
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    switch (blocks_per_sm) {
-        case 2: LW_CUDA(cudaLaunchKernelEx(&cfg, k_loc_icp<2>, *g, *b, w, la)); break;
-        case 3: LW_CUDA(cudaLaunchKernelEx(&cfg, k_loc_icp<3>, *g, *b, w, la)); break;
-        case 4: LW_CUDA(cudaLaunchKernelEx(&cfg, k_loc_icp<4>, *g, *b, w, la)); break;
-        case 5: LW_CUDA(cudaLaunchKernelEx(&cfg, k_loc_icp<5>, *g, *b, w, la)); break;
-        default: LW_CUDA(cudaLaunchKernelEx(&cfg, k_loc_icp<6>, *g, *b, w, la)); break;
-    }
+    LW_CUDA(cudaLaunchKernelEx(&cfg, fn, *g, *b, w, la));
     LW_LAUNCHED("lw_loc_icp_batch");
     count_launches(2);
     return LW_OK;
