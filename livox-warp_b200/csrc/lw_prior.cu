@@ -220,11 +220,18 @@ __global__ void k_pc_start(lw_pca_buf pb) {
     int tot;
     const int r = block_excl(v, sm, &tot);
     if (v > 0) pb.cell_start[s] = pb.tiles[blockIdx.x] + r;
+    __syncthreads();
+    if (blockIdx.x == 0 && threadIdx.x == 0) pb.tiles[0] = 0;  // from here on k_pc_scatter's count
 }
+
+// Each point's record into its cell's run; in tiles[0] five times the occupied cells less twice the points, a cell counted by
+// its first point, over every CTA's points or, of more than 256 CTAs, over every PC_SAMPLE-th's: what pn_few goes by.
+constexpr int PC_SAMPLE = 16;
 
 template <int STRIDE>
 __global__ void k_pc_scatter(const float* __restrict__ xyz, int64_t n, lw_pca_buf pb, float* __restrict__ out_nrm,
                              float* __restrict__ out_pl) {
+    int sum = 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int s = pb.slot_of_pt[i];
         if (s < 0) {  // not placed: no neighbourhood to fit
@@ -234,9 +241,14 @@ __global__ void k_pc_scatter(const float* __restrict__ xyz, int64_t n, lw_pca_bu
         }
         float x, y, z;
         ld3<STRIDE>(xyz, i, x, y, z);
-        const int64_t q = (int64_t)pb.cell_start[s] + pb.rank_of_pt[i];
+        const int rank = pb.rank_of_pt[i];
+        const int64_t q = (int64_t)pb.cell_start[s] + rank;
         reinterpret_cast<float4*>(pb.sorted)[q] = make_float4(x, y, z, __int_as_float((int)i));
+        sum += rank == 0 ? 5 - 2 : -2;
     }
+    if (gridDim.x > 256 && blockIdx.x % PC_SAMPLE != 0) return;
+    sum = warp_sum_i(sum);
+    if ((threadIdx.x & 31) == 0 && sum != 0) atomicAdd(pb.tiles, sum);
 }
 
 // The sums over a point's neighbours: the offsets and products as 32-bit partial sums (rint_bits, rint_split), moved to
@@ -302,6 +314,52 @@ struct PnSmem {
     int queue[PN_CTA / 32][PN_QUEUE][32];
 };
 
+// Whether the points are so few to a cell that a lane per point looks its own cells up (k_pc_normals_few). The line is where the
+// two take the same time, whatever the size: 1.0M / 0.2M points of a surface, few-to-a-cell way and shared way, us:
+// 1.2 points a cell 672 / 185 and 877 / 215, 2.0 662 / 181 and 732 / 191, 2.5 671 / 189 and 674 / 188, 3.0 682 / 198 and
+// 647 / 182, 5.2 656 / 212 and 534 / 179. (By the warp instead of for all, a mixture of the two took up to 1160.)
+__device__ __forceinline__ bool pn_few(const lw_pca_buf& pb) { return pb.tiles[0] > 0; }
+
+// Point i's normal and planarity from its n neighbours' sums.
+__device__ __forceinline__ void pn_write(int n, const long long (&s1)[3], const long long (&s2)[6], const PcaArgs& a, int i,
+                                         float* __restrict__ out_nrm, float* __restrict__ out_pl) {
+    if (n < 4) {  // prior_map.py:151-154
+        out_nrm[3 * (int64_t)i] = out_nrm[3 * (int64_t)i + 1] = out_nrm[3 * (int64_t)i + 2] = 0.0f;
+        out_pl[i] = 0.0f;
+        return;
+    }
+    const double inv = 1.0 / (double)n;
+    const double mu[3] = {(double)s1[0] / a.fd64 * inv, (double)s1[1] / a.fd64 * inv,
+                          (double)s1[2] / a.fd64 * inv};
+    const int up[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
+    double C[9], ev[3], Qm[9];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) C[r * 3 + c] = (double)s2[up[r * 3 + c]] / a.fdd64 * inv - mu[r] * mu[c];
+    jacobi_eig<3>(C, ev, Qm);
+    // the eigenvalues' order, as prior_map.py:157-164 picks it
+    int lo = 0, hi = 0;
+    if (ev[1] < ev[lo]) lo = 1;
+    if (ev[1] > ev[hi]) hi = 1;
+    if (ev[2] < ev[lo]) lo = 2;
+    if (ev[2] > ev[hi]) hi = 2;
+    const int mid = lo == hi ? lo : 3 - lo - hi;
+    // selects instead of indexing with lo / mid / hi keep ev and Qm in registers
+    auto at = [](const double* v, int k) { return k == 0 ? v[0] : (k == 1 ? v[1] : v[2]); };
+    double nx = at(Qm, lo), ny = at(Qm + 3, lo), nz = at(Qm + 6, lo);
+    const double nl = sqrt(nx * nx + ny * ny + nz * nz);
+    if (nl > 0.0) {
+        nx /= nl;
+        ny /= nl;
+        nz /= nl;
+    }
+    out_nrm[3 * (int64_t)i + 0] = (float)nx;
+    out_nrm[3 * (int64_t)i + 1] = (float)ny;
+    out_nrm[3 * (int64_t)i + 2] = (float)nz;
+    out_pl[i] = (float)((at(ev, mid) - at(ev, lo)) / fmax(at(ev, hi), 1.0e-12));
+}
+
 // A lane per sorted position (k_normals): every point within the radius, found in the 27 cells around the
 // point's own, adds 1, its offset and its offset's outer product in fixed point; then the covariance's
 // eigen-decomposition in float64, the smallest eigenvalue's vector and (l_mid - l_min) / l_max.
@@ -316,6 +374,7 @@ struct PnSmem {
 __global__ void __launch_bounds__(PN_CTA, 3) k_pc_normals(PcaArgs a, lw_pca_buf pb, float* __restrict__ out_nrm,
                                                        float* __restrict__ out_pl) {
     __shared__ PnSmem sm;
+    if (pn_few(pb)) return;
     const int m = *pb.stats;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned full = 0xFFFFFFFFu;
@@ -392,44 +451,47 @@ __global__ void __launch_bounds__(PN_CTA, 3) k_pc_normals(PcaArgs a, lw_pca_buf 
         }
         S.flush();
         if (!act) continue;
-        const int n = S.n;
-        const long long(&s1)[3] = S.s1;
-        const long long(&s2)[6] = S.s2;
-        if (n < 4) {  // prior_map.py:151-154
-            out_nrm[3 * (int64_t)i] = out_nrm[3 * (int64_t)i + 1] = out_nrm[3 * (int64_t)i + 2] = 0.0f;
-            out_pl[i] = 0.0f;
-            continue;
+        pn_write(S.n, S.s1, S.s2, a, i, out_nrm, out_pl);
+    }
+}
+
+// k_pc_normals where points are few to a cell: a thread per sorted position for itself. Bound by the latency of its 27 lookups, so
+// by the warps in flight: four CTAs an SM, and no shared memory, which L1 needs. 200,000 lone points 126 us a call; 160
+// in the shared way, whose warps look up their 32 cells one after another.
+__global__ void __launch_bounds__(PN_CTA, 4) k_pc_normals_few(PcaArgs a, lw_pca_buf pb, float* __restrict__ out_nrm,
+                                                              float* __restrict__ out_pl) {
+    if (!pn_few(pb)) return;
+    const int m = *pb.stats;
+    const float4* __restrict__ pts = reinterpret_cast<const float4*>(pb.sorted);
+    for (int q = blockIdx.x * PN_CTA + threadIdx.x; q < m; q += gridDim.x * PN_CTA) {
+        const float4 P = pts[q];
+        const int ix = ifloor(P.x * a.inv_h), iy = ifloor(P.y * a.inv_h), iz = ifloor(P.z * a.inv_h);
+        int n = 0;
+        long long s1[3] = {0, 0, 0}, s2[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll 1
+        for (int c = 0; c < 27; ++c) {
+            const int s = find_slot<VX_PROBES>(key_ijk(ix + c / 9 - 1, iy + (c / 3) % 3 - 1, iz + c % 3 - 1), pb.keys,
+                                               a.mask);
+            if (s < 0) continue;
+            const int k0 = __ldg(pb.cell_start + s), k1 = k0 + __ldg(pb.cell_cnt + s);
+#pragma unroll 1
+            for (int k = k0; k < k1; ++k) {
+                const float4 Q = __ldg(pts + k);
+                const float ex = Q.x - P.x, ey = Q.y - P.y, ez = Q.z - P.z;
+                if (ex * ex + ey * ey + ez * ez > a.r2) continue;
+                ++n;
+                s1[0] += to_fix(ex, a.fd);
+                s1[1] += to_fix(ey, a.fd);
+                s1[2] += to_fix(ez, a.fd);
+                s2[0] += to_fix(ex * ex, a.fdd);
+                s2[1] += to_fix(ex * ey, a.fdd);
+                s2[2] += to_fix(ex * ez, a.fdd);
+                s2[3] += to_fix(ey * ey, a.fdd);
+                s2[4] += to_fix(ey * ez, a.fdd);
+                s2[5] += to_fix(ez * ez, a.fdd);
+            }
         }
-        const double inv = 1.0 / (double)n;
-        const double mu[3] = {(double)s1[0] / a.fd64 * inv, (double)s1[1] / a.fd64 * inv,
-                              (double)s1[2] / a.fd64 * inv};
-        const int up[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
-        double C[9], ev[3], Qm[9];
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) C[r * 3 + c] = (double)s2[up[r * 3 + c]] / a.fdd64 * inv - mu[r] * mu[c];
-        jacobi_eig<3>(C, ev, Qm);
-        // the eigenvalues' order, as prior_map.py:157-164 picks it
-        int lo = 0, hi = 0;
-        if (ev[1] < ev[lo]) lo = 1;
-        if (ev[1] > ev[hi]) hi = 1;
-        if (ev[2] < ev[lo]) lo = 2;
-        if (ev[2] > ev[hi]) hi = 2;
-        const int mid = lo == hi ? lo : 3 - lo - hi;
-        // selects instead of indexing with lo / mid / hi keep ev and Qm in registers
-        auto at = [](const double* v, int k) { return k == 0 ? v[0] : (k == 1 ? v[1] : v[2]); };
-        double nx = at(Qm, lo), ny = at(Qm + 3, lo), nz = at(Qm + 6, lo);
-        const double nl = sqrt(nx * nx + ny * ny + nz * nz);
-        if (nl > 0.0) {
-            nx /= nl;
-            ny /= nl;
-            nz /= nl;
-        }
-        out_nrm[3 * (int64_t)i + 0] = (float)nx;
-        out_nrm[3 * (int64_t)i + 1] = (float)ny;
-        out_nrm[3 * (int64_t)i + 2] = (float)nz;
-        out_pl[i] = (float)((at(ev, mid) - at(ev, lo)) / fmax(at(ev, hi), 1.0e-12));
+        pn_write(n, s1, s2, a, __float_as_int(P.w), out_nrm, out_pl);
     }
 }
 
@@ -560,8 +622,9 @@ int lw_normals(const float* xyz, int32_t xyz_stride, int64_t n, float radius, lw
     else
         k_pc_scatter<3><<<grid, 256, 0, s>>>(xyz, n, *pb, out_nrm, out_planarity);
     k_pc_normals<<<blocks_for(n, PN_CTA, 16 * sms), PN_CTA, 0, s>>>(a, *pb, out_nrm, out_planarity);
+    k_pc_normals_few<<<blocks_for(n, PN_CTA, 4 * sms), PN_CTA, 0, s>>>(a, *pb, out_nrm, out_planarity);
     LW_LAUNCHED("lw_normals");
-    count_launches(6);
+    count_launches(7);
     return LW_OK;
 }
 
