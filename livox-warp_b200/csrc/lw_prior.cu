@@ -318,7 +318,7 @@ struct PnSmem {
 // two take the same time, whatever the size: 1.0M / 0.2M points of a surface, few-to-a-cell way and shared way, us:
 // 1.2 points a cell 672 / 185 and 877 / 215, 2.0 662 / 181 and 732 / 191, 2.5 671 / 189 and 674 / 188, 3.0 682 / 198 and
 // 647 / 182, 5.2 656 / 212 and 534 / 179. (By the warp instead of for all, a mixture of the two took up to 1160.)
-__device__ __forceinline__ bool pn_few(const lw_pca_buf& pb) { return pb.tiles[0] > 0; }
+__device__ __forceinline__ bool pn_few(const lw_pca_buf& pb) { return __ldg(pb.tiles) > 0; }
 
 // Point i's normal and planarity from its n neighbours' sums.
 __device__ __forceinline__ void pn_write(int n, const long long (&s1)[3], const long long (&s2)[6], const PcaArgs& a, int i,
@@ -374,8 +374,7 @@ __device__ __forceinline__ void pn_write(int n, const long long (&s1)[3], const 
 __global__ void __launch_bounds__(PN_CTA, 3) k_pc_normals(PcaArgs a, lw_pca_buf pb, float* __restrict__ out_nrm,
                                                        float* __restrict__ out_pl) {
     __shared__ PnSmem sm;
-    if (pn_few(pb)) return;
-    const int m = *pb.stats;
+    const int n_pts = __ldg(pb.stats), m = pn_few(pb) ? 0 : n_pts;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned full = 0xFFFFFFFFu;
     const float4* __restrict__ pts = reinterpret_cast<const float4*>(pb.sorted);
@@ -460,8 +459,7 @@ __global__ void __launch_bounds__(PN_CTA, 3) k_pc_normals(PcaArgs a, lw_pca_buf 
 // in the shared way, whose warps look up their 32 cells one after another.
 __global__ void __launch_bounds__(PN_CTA, 4) k_pc_normals_few(PcaArgs a, lw_pca_buf pb, float* __restrict__ out_nrm,
                                                               float* __restrict__ out_pl) {
-    if (!pn_few(pb)) return;
-    const int m = *pb.stats;
+    const int n_pts = __ldg(pb.stats), m = pn_few(pb) ? n_pts : 0;
     const float4* __restrict__ pts = reinterpret_cast<const float4*>(pb.sorted);
     for (int q = blockIdx.x * PN_CTA + threadIdx.x; q < m; q += gridDim.x * PN_CTA) {
         const float4 P = pts[q];
