@@ -2,16 +2,17 @@
 // points, 512 -> 128 -> 6) on sm_100a. It has no counterpart in the reference, whose odometry predicts the next
 // pose with constant velocity (odom.py:591-592); that prediction stays the network's input frame and fallback.
 //
-// Forward: persistent CTAs of two groups of 128 threads, a point set per group at a time, eight 128-point tiles in turn. Layer 1 (K = 3) runs on the CUDA
-// cores; layers 2 and 3 are tcgen05.mma (kind::f16, bf16 operands from shared memory in the canonical K-major
-// layout without swizzle, float32 accumulators in TMEM). Layer 2 puts the points on M (D = H1 W2^T, one TMEM
-// lane per point), so each thread converts its own point's 128 channels back to bf16 for layer 3. Layer 3 puts
-// the channels on M (D = W3 H2^T, two M = 128 halves), so each thread holds one channel across the tile's points
+// Forward: persistent CTAs of two groups of 128 threads, a point set per group at a time, eight 128-point tiles in turn.
+// Layer 1 (K = 3) runs on the CUDA cores; layers 2 and 3 are tcgen05.mma (kind::f16, bf16 operands from shared memory
+// in the canonical K-major layout without swizzle, float32 accumulators in TMEM). Layer 2 puts the points on M (D = H1
+// W2^T, one TMEM lane per point), so each thread converts its own point's 128 channels back to bf16 for layer 3. Layer 3
+// puts the channels on M (D = W3 H2^T, two M = 128 halves), so each thread holds one channel across the tile's points
 // and the max-pool and its argmax are a per-thread scan of its TMEM lane -- no shuffles, no atomics.
 //
-// Backward: through the max only each channel's argmax point receives gradient, so it is sparse: one thread per
-// (set, channel) recomputes its point's layer-1 and layer-2 activations in float32 and writes the per-row factors
-// of the weight gradients; split-K reductions with a fixed order sum them (deterministic).
+// Backward: through the max only each channel's argmax point receives gradient, so it is sparse: a set's distinct argmax
+// points are gathered, their layer-1 and layer-2 activations recomputed in float32 once for all their channels, and the
+// weight gradients of layers 1 and 2 summed in registers over a CTA's sets; the CTAs' sums, and the layer-3 and head
+// gradients, are added in a fixed order (deterministic).
 #include <cuda_bf16.h>
 
 #include "lw_common.cuh"
@@ -21,7 +22,7 @@
 namespace lw {
 
 constexpr int NP = LW_NET_P;  // points per set
-constexpr int NET_T = 128;    // threads (and points) per forward CTA
+constexpr int NET_T = 128;    // threads (and points) per group of a forward CTA
 constexpr int C1 = 64, C2 = 128, C3 = 256, CH = 128, NOUT = 6;
 constexpr long long NET_SPINS = 1LL << 24;
 

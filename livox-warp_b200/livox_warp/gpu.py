@@ -422,8 +422,8 @@ class Pipeline:
                 s.wait_stream(last)
 
     def _carve_ws(self, rays: int):
-        """lw_carve_ws's workspace for at least `rays` rays, and where each ray's stop goes. It grows by doubling, and the smaller ones are kept: a
-        stream other than the one they were made on may still be using them."""
+        """lw_carve_ws's workspace for at least `rays` rays, and where each ray's stop goes. It grows by doubling, and the
+        smaller ones are kept: a stream other than the one they were made on may still be using them."""
         if rays > self._carve_rays:
             r = 1 << (rays - 1).bit_length()
             pairs, slots, d = 16 * r, min(4 * r, self.map_cap), self.device
