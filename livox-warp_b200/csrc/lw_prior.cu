@@ -374,6 +374,7 @@ __device__ __forceinline__ void pn_write(int n, const long long (&s1)[3], const 
 __global__ void __launch_bounds__(PN_CTA, 3) k_pc_normals(PcaArgs a, lw_pca_buf pb, float* __restrict__ out_nrm,
                                                        float* __restrict__ out_pl) {
     __shared__ PnSmem sm;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // k_pc_normals_few may come in beside the last CTAs
     const int n_pts = __ldg(pb.stats), m = pn_few(pb) ? 0 : n_pts;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned full = 0xFFFFFFFFu;
@@ -460,6 +461,8 @@ __global__ void __launch_bounds__(PN_CTA, 3) k_pc_normals(PcaArgs a, lw_pca_buf 
 __global__ void __launch_bounds__(PN_CTA, 4) k_pc_normals_few(PcaArgs a, lw_pca_buf pb, float* __restrict__ out_nrm,
                                                               float* __restrict__ out_pl) {
     const int n_pts = __ldg(pb.stats), m = pn_few(pb) ? n_pts : 0;
+    if (m == 0 && blockIdx.x > 0) return;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // one CTA is enough: the launch is not over before k_pc_normals is
     const float4* __restrict__ pts = reinterpret_cast<const float4*>(pb.sorted);
     for (int q = blockIdx.x * PN_CTA + threadIdx.x; q < m; q += gridDim.x * PN_CTA) {
         const float4 P = pts[q];
@@ -620,7 +623,17 @@ int lw_normals(const float* xyz, int32_t xyz_stride, int64_t n, float radius, lw
     else
         k_pc_scatter<3><<<grid, 256, 0, s>>>(xyz, n, *pb, out_nrm, out_planarity);
     k_pc_normals<<<blocks_for(n, PN_CTA, 16 * sms), PN_CTA, 0, s>>>(a, *pb, out_nrm, out_planarity);
-    k_pc_normals_few<<<blocks_for(n, PN_CTA, 4 * sms), PN_CTA, 0, s>>>(a, *pb, out_nrm, out_planarity);
+    // nothing k_pc_normals writes is read, so the launch need not wait for its end (it took 3 us of a small map's 200 so)
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks_for(n, PN_CTA, 4 * sms));
+    cfg.blockDim = dim3(PN_CTA);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    LW_CUDA(cudaLaunchKernelEx(&cfg, k_pc_normals_few, a, *pb, out_nrm, out_planarity));
     LW_LAUNCHED("lw_normals");
     count_launches(7);
     return LW_OK;
