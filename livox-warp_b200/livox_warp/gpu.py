@@ -214,7 +214,8 @@ class Pipeline:
         self._slot = torch.zeros(n, dtype=torch.int32, device=d)  # per-point scratch of the insert passes
         self._carve_rays, self._carve_t, self._carve_buf = 0, [], None  # lw_carve_ws's workspace
         self._carve_lock = threading.Lock()  # held while a carve is launched
-        self._carve_stream, self._carve_done = None, torch.cuda.Event()  # the last one's stream; its end (see _carve_wait)
+        # the last one's stream and its handle (None when foreign), and the end of a foreign one (see _carve_wait)
+        self._carve_last, self._carve_done = (None, None), torch.cuda.Event()
         self._carve_marks = torch.zeros(m, dtype=torch.int32, device=d)  # its own: an insertion may run beside a carve
         self._carve_ws(1 << 15)  # what a frame takes, made here so that no frame waits for an allocation
         self._tiles = torch.zeros(max(m, self.cap) // 1024 + 2, dtype=torch.int32, device=d)
@@ -394,32 +395,34 @@ class Pipeline:
         s = torch.cuda.current_stream()
         with self._carve_lock:
             ws, stop = self._carve_ws(rays)
-            # a capture neither waits (what it records runs later) nor is waited for
-            capturing = torch.cuda.is_current_stream_capturing()
-            if not capturing:
+            # on the stream of the carve before there is nothing to wait for; a capture neither waits (what it records
+            # runs later) nor is waited for
+            turn = self._carve_last[0] != s.cuda_stream and not torch.cuda.is_current_stream_capturing()
+            if turn:
                 self._carve_wait(s)
             _lib.call("lw_carve_ws", _lib.ptr(sx), row_stride(sx), _lib.ptr(sa), _lib.ptr(sf), _lib.ptr(n_dev), n,
                       _lib.ptr(self.poses), every, 1.0 / max(voxel, 1e-4), float(max_range), int(max_steps),
                       C_ref(self.map_struct), stop, ws, _lib.stream_ptr(s))
-            if not capturing:
-                if _foreign(s):
+            if turn:
+                foreign = _foreign(s)
+                self._carve_last = (None if foreign else s.cuda_stream, s)
+                if foreign:
                     self._carve_done.record(s)
-                self._carve_stream = s
 
     def _carve_wait(self, s):
-        """Let stream `s` wait for the carve before, unless that went to the same stream. A stream of the caller's own
-        making may be gone by now: of one the end of its carve is kept as an event, and nothing else. (An event for
-        every carve took 14 us of the host a call.)"""
-        last = self._carve_stream
+        """Let stream `s` wait for the carve before, which went to another. A stream of the caller's own making may be gone
+        by now: of one the end of its carve is kept as an event, and nothing else. (An event for every carve took 14 us of
+        the host a call.)"""
+        handle, last = self._carve_last
         if last is None:
             return
-        if _foreign(last):
+        if handle is None:
             s.wait_event(self._carve_done)
-        elif last.cuda_stream != s.cuda_stream:
-            with torch.cuda.stream(last):
-                capturing = torch.cuda.is_current_stream_capturing()
-            if not capturing:  # (torch.cuda.graph starts a capture on an idle device)
-                s.wait_stream(last)
+            return
+        with torch.cuda.stream(last):
+            capturing = torch.cuda.is_current_stream_capturing()
+        if not capturing:  # (torch.cuda.graph starts a capture on an idle device)
+            s.wait_stream(last)
 
     def _carve_ws(self, rays: int):
         """lw_carve_ws's workspace for at least `rays` rays, and where each ray's stop goes. It grows by doubling, and the
